@@ -4,6 +4,12 @@
 // N dimension; the reduction over K is order-free, so a lane's 8 consecutive channels serve as the fragment's k-slots and
 // the activations are loaded with the same addressing).  Tokens beyond M load nothing.  Warp partials meet in shared memory.
 //
+// A matrix with too few 16-row tiles for the chip has its contraction split over the CTAs of a thread-block cluster, whose sums meet
+// through distributed shared memory.  A decoding step is a chain of such products of 2 to 6 us each and is bound by the number of
+// launches in it, so the split needs no second launch (and no workspace), and up to four matrices that read the same activations share a launch.
+// Qwen3.5 0.8B, one row, 500 tokens of context: a step of 323 launches took 1275 us, one of
+// 209 launches 1022 us; the four products of a linear layer (6144, 2048, 16 and 16 rows of 1024) take 5.1 us in one launch.
+//
 // The reference sends these products to the library GEMM (cc/src/tyr.cpp:1003-1036).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -16,13 +22,25 @@ namespace tyr {
 
 constexpr int kSkWarps = 8;
 
+constexpr int kSkSegments = 4;
+constexpr int kSkMaxSplits = 8;  // a portable cluster
+
+// Matrices behind the first one that read the same activations: their 16-row tiles follow those of the first along gridDim.x.
+struct SkinnySegments {
+  int n;                                   // matrices in all, the first included
+  int tile0[kSkSegments];                  // first tile of each
+  const __nv_bfloat16* w[kSkSegments];
+  __nv_bfloat16* y[kSkSegments];
+  long long ldw[kSkSegments], ldy[kSkSegments];
+  int N[kSkSegments];
+};
+
 struct SkinnyArgs {
   const __nv_bfloat16* x;      // [M, K], row stride ldx
   const __nv_bfloat16* w;      // [N, K], row stride ldw
   const __nv_bfloat16* w2;     // gated form only: the second matrix [N, K]; y = silu(x w^T) * (x w2^T)
   const __nv_bfloat16* bias;   // [N] or null
   __nv_bfloat16* y;            // [M, N], row stride ldy
-  float* ws;                   // [M, N] fp32, zero on entry and exit; used when the reduction is split over gridDim.y CTAs
   long long ldx, ldw, ldy;
   int M, N, K;
   long long hx, hw, hy;        // per-head form: elements from head to head
@@ -46,11 +64,23 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 constexpr long long kSkPrefetchBytes = 32LL << 20;   // L2 prefetch issued by one launch before its input is ready
 
 template <int TILES, bool GATED>                   // token tiles of 8: M <= 8 * TILES; GATED: two matrices, SwiGLU epilogue
-__global__ void __launch_bounds__(kSkWarps * 32) skinny_gemm_kernel(SkinnyArgs a) {
+__global__ void __launch_bounds__(kSkWarps * 32) skinny_gemm_kernel(SkinnyArgs a, const __grid_constant__ SkinnySegments seg) {
   __shared__ float part[GATED ? 2 : 1][kSkWarps][TILES][16][8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int row0 = blockIdx.x * 16;
+  int tile = blockIdx.x;
+  if (!GATED && seg.n > 1) {
+    int s = 0;
+#pragma unroll
+    for (int i = 1; i < kSkSegments; ++i) s = (i < seg.n && tile >= seg.tile0[i]) ? i : s;
+    tile -= seg.tile0[s];
+    a.w = seg.w[s];
+    a.y = seg.y[s];
+    a.ldw = seg.ldw[s];
+    a.ldy = seg.ldy[s];
+    a.N = seg.N[s];
+  }
+  const int row0 = tile * 16;
   // The weights are constants: while the kernel that produces `x` still runs (this one may already be resident, see
   // launch_dependent), pull the head of every weight row of this CTA into the L2.  The whole grid asks for at most
   // kSkPrefetchBytes, so what it brings in is still there when the loop below reads it.
@@ -125,25 +155,52 @@ __global__ void __launch_bounds__(kSkWarps * 32) skinny_gemm_kernel(SkinnyArgs a
     }
   }
   __syncthreads();
+  const int splits = gridDim.y;
   for (int idx = tid; idx < TILES * 8 * 16; idx += kSkWarps * 32) {
     const int tok = idx >> 4, r = idx & 15;        // consecutive threads write consecutive output columns
     const int row = row0 + r;
-    if (tok < a.M && row < a.N) {
-      float s = 0.f;
+    float s = 0.f;
 #pragma unroll
-      for (int wp = 0; wp < kSkWarps; ++wp) s += part[0][wp][tok >> 3][r][tok & 7];
+    for (int wp = 0; wp < kSkWarps; ++wp) s += part[0][wp][tok >> 3][r][tok & 7];
+    if (!GATED && splits > 1) {
+      part[0][0][tok >> 3][r][tok & 7] = s;        // read by this thread only so far: now the CTA's sum
+      continue;
+    }
+    if (tok < a.M && row < a.N) {
       if (GATED) {
         float u = 0.f;
 #pragma unroll
         for (int wp = 0; wp < kSkWarps; ++wp) u += part[1][wp][tok >> 3][r][tok & 7];
         a.y[tok * a.ldy + row] = __float2bfloat16(s / (1.f + __expf(-s)) * u);
-      } else if (gridDim.y == 1) {
+      } else {
         if (a.bias) s += __bfloat162float(a.bias[row]);
         a.y[tok * a.ldy + row] = __float2bfloat16(sk_act(s, a, tok, row));
-      } else {
-        atomicAdd(a.ws + static_cast<long long>(tok) * a.N + row, s);
       }
     }
+  }
+  if (!GATED && splits > 1) {
+    // the CTAs of the cluster hold one share of the contraction each: the first sums them in their order
+    cluster_arrive();
+    cluster_wait();
+    if (blockIdx.y == 0) {
+      for (int idx = tid; idx < TILES * 8 * 16; idx += kSkWarps * 32) {
+        const int tok = idx >> 4, r = idx & 15, row = row0 + r;
+        if (tok >= a.M || row >= a.N) continue;
+        const uint32_t at = smem_u32(&part[0][0][tok >> 3][r][tok & 7]);
+        float v[kSkMaxSplits], s = 0.f;
+#pragma unroll
+        for (int i = 0; i < kSkMaxSplits; ++i) {
+          v[i] = 0.f;
+          if (i < splits) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[i]) : "r"(mapa_shared(at, i)) : "memory");
+        }
+#pragma unroll
+        for (int i = 0; i < kSkMaxSplits; ++i) s += v[i];
+        if (a.bias) s += __bfloat162float(a.bias[row]);
+        a.y[tok * a.ldy + row] = __float2bfloat16(sk_act(s, a, tok, row));
+      }
+    }
+    cluster_arrive();                              // no CTA leaves while its sums are being read
+    cluster_wait();
   }
 }
 
@@ -206,19 +263,6 @@ __global__ void __launch_bounds__(kSkWarps * 32) skinny_heads_kernel(SkinnyArgs 
     }
 }
 
-// Second pass of a split reduction: round the fp32 sums (+ bias) and leave the workspace zeroed for the next call.
-__global__ void __launch_bounds__(256) skinny_finish_kernel(SkinnyArgs a) {
-  pdl_entry();
-  const long long n = static_cast<long long>(a.M) * a.N;
-  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += static_cast<long long>(gridDim.x) * 256) {
-    const int tok = static_cast<int>(i / a.N), row = static_cast<int>(i - static_cast<long long>(tok) * a.N);
-    float s = a.ws[i];
-    a.ws[i] = 0.f;
-    if (a.bias) s += __bfloat162float(a.bias[row]);
-    a.y[tok * a.ldy + row] = __float2bfloat16(sk_act(s, a, tok, row));
-  }
-}
-
 }  // namespace tyr
 
 // The kernels above read the activations through the L1: the eight CTAs of an SM walk the same rows of x.  A kernel with a
@@ -252,55 +296,99 @@ static void skinny_prefer_l1() {
   skinny_set_carveout<4, true>();
 }
 
-// Number of CTAs the reduction should be split over for this shape (1 = no workspace needed): enough CTAs to cover the
-// SMs about three times, at least 1024 channels per split.
-extern "C" TYR_EXPORT int tyr_skinny_gemm_splits(int N, int K) {
-  const int row_ctas = (N + 15) / 16;
-  int splits = (3 * 148 + row_ctas - 1) / row_ctas;
-  const int max_by_k = K / 1024 > 0 ? K / 1024 : 1;
-  if (splits > max_by_k) splits = max_by_k;
-  if (splits > 8) splits = 8;
+// CTAs of a cluster that share the contraction of one 16-row tile: as many as stay resident at once beside the other tiles' (6, 4 or 3
+// on an SM for up to 8, 16 or 32 tokens), each with at least kSkSplitChannels channels.  One row, us at 1 / 2 / 3 / 4 / 8 CTAs: 1024 x 3584
+// 10.1 / 5.9 / 5.6 / 5.2 / 4.6, 4096 x 12288 36.8 / 23.4 / 20.3 / 26.4 / 25.5, 5120 x 17408 52.1 / 34.1 / 44.6 / 36.4 / 42.2 (past one wave of CTAs
+// it gets slower); 32 rows, two matrices of 1024 x 5120 27.2 / 15.9 / 13.5 / 20.9 / 28.2.
+constexpr int kSkSplitChannels = 512;
+static int skinny_splits(int row_ctas, int M, int K) {
+  int splits = 148 * (M <= 8 ? 6 : M <= 16 ? 4 : 3) / row_ctas;
+  if (splits > K / kSkSplitChannels) splits = K / kSkSplitChannels;
+  if (splits > tyr::kSkMaxSplits) splits = tyr::kSkMaxSplits;
   return splits < 1 ? 1 : splits;
 }
 
-static int skinny_launch(const void* x, const void* w, const void* bias, void* y, void* ws, long long ldx, long long ldw, long long ldy, int M,
-                         int N, int K, int act, float act_a, float act_b, void* stream, const void* aux = nullptr, long long ldaux = 0) {
+template <int TILES, bool GATED>
+static cudaError_t skinny_start(dim3 grid, cudaStream_t stream, const tyr::SkinnyArgs& a, const tyr::SkinnySegments& seg) {
   using namespace tyr;
-  if ((act != 0 && act != 6 && act != 9) || (act == 9) != (aux != nullptr)) return -4;
-  if (M < 1 || M > 32 || N < 1 || K < 32 || (K & 31)) return -1;
-  if ((ldx | ldw) & 7) return -2;                                    // 16-byte loads
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) return -3;
-  SkinnyArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, nullptr, (const __nv_bfloat16*)bias, (__nv_bfloat16*)y, (float*)ws, ldx, ldw, ldy, M, N, K,
-               0, 0, 0, act, act_a, act_b, (const __nv_bfloat16*)aux, ldaux};
-  const int splits = ws != nullptr ? tyr_skinny_gemm_splits(N, K) : 1;
-  const dim3 grid((N + 15) / 16, splits);
-  skinny_prefer_l1();
-  if (M <= 8) launch_dependent(skinny_gemm_kernel<1, false>, dim3(grid), dim3(kSkWarps * 32), 0, (cudaStream_t)stream, a);
-  else if (M <= 16) launch_dependent(skinny_gemm_kernel<2, false>, dim3(grid), dim3(kSkWarps * 32), 0, (cudaStream_t)stream, a);
-  else launch_dependent(skinny_gemm_kernel<4, false>, dim3(grid), dim3(kSkWarps * 32), 0, (cudaStream_t)stream, a);
-  if (splits > 1) {
-    long long blocks = (static_cast<long long>(M) * N + 255) / 256;
-    if (blocks > 592) blocks = 592;
-    launch_dependent(skinny_finish_kernel, dim3((int)blocks), dim3(256), 0, (cudaStream_t)stream, a);
-  }
-  return (int)cudaGetLastError();
+  if (grid.y == 1) return launch_dependent(skinny_gemm_kernel<TILES, GATED>, grid, dim3(kSkWarps * 32), 0, stream, a, seg);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kSkWarps * 32);
+  cfg.stream = stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = grid.y; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  cfg.attrs = at; cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, skinny_gemm_kernel<TILES, GATED>, a, seg);
 }
 
-extern "C" TYR_EXPORT int tyr_skinny_gemm_bf16(const void* x, const void* w, const void* bias, void* y, void* ws, long long ldx,
+static int skinny_launch(const tyr::SkinnyArgs& a, const tyr::SkinnySegments& seg, int row_ctas, int splits, void* stream) {
+  using namespace tyr;
+  if ((a.act != 0 && a.act != 6 && a.act != 9) || (a.act == 9) != (a.aux != nullptr)) return -4;
+  if (a.M < 1 || a.M > 32 || a.K < 32 || (a.K & 31) || splits < 0 || splits > kSkMaxSplits) return -1;
+  if (a.ldx & 7) return -2;                                          // 16-byte loads
+  if (reinterpret_cast<uintptr_t>(a.x) & 15) return -3;
+  for (int i = 0; i < seg.n; ++i) {
+    if (seg.N[i] < 1) return -1;
+    if (seg.ldw[i] & 7) return -2;
+    if (reinterpret_cast<uintptr_t>(seg.w[i]) & 15) return -3;
+  }
+  const dim3 grid(row_ctas, splits > 0 ? splits : skinny_splits(row_ctas, a.M, a.K));
+  const cudaStream_t st = (cudaStream_t)stream;
+  skinny_prefer_l1();
+  return (int)(a.M <= 8 ? skinny_start<1, false>(grid, st, a, seg) : a.M <= 16 ? skinny_start<2, false>(grid, st, a, seg) : skinny_start<4, false>(grid, st, a, seg));
+}
+
+static int skinny_single(const void* x, const void* w, const void* bias, void* y, long long ldx, long long ldw, long long ldy, int M, int N, int K,
+                         int act, float act_a, float act_b, void* stream, const void* aux = nullptr, long long ldaux = 0) {
+  using namespace tyr;
+  const SkinnyArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, nullptr, (const __nv_bfloat16*)bias, (__nv_bfloat16*)y, ldx, ldw, ldy, M, N, K,
+                     0, 0, 0, act, act_a, act_b, (const __nv_bfloat16*)aux, ldaux};
+  SkinnySegments seg{};
+  seg.n = 1; seg.w[0] = a.w; seg.y[0] = a.y; seg.ldw[0] = ldw; seg.ldy[0] = ldy; seg.N[0] = N;
+  return skinny_launch(a, seg, (N + 15) / 16, 0, stream);
+}
+
+// Up to four matrices W[i] [N[i], K] that read the same x: y[i] = x W[i]^T in one launch.  `splits`: CTAs that share a contraction (0: by size).
+extern "C" TYR_EXPORT int tyr_skinny_many_bf16(const void* x, long long ldx, int n, const void* const* w, void* const* y, const long long* ldw,
+                                               const long long* ldy, const int* N, int M, int K, int splits, void* stream) {
+  using namespace tyr;
+  if (n < 1 || n > kSkSegments) return -5;
+  SkinnySegments seg{};
+  seg.n = n;
+  long long tiles = 0;
+  for (int i = 0; i < n; ++i) {
+    seg.tile0[i] = (int)tiles;
+    seg.w[i] = (const __nv_bfloat16*)w[i];
+    seg.y[i] = (__nv_bfloat16*)y[i];
+    seg.ldw[i] = ldw[i];
+    seg.ldy[i] = ldy[i];
+    seg.N[i] = N[i];
+    tiles += (N[i] + 15LL) / 16;
+    if (tiles > 0x7fffffff) return -1;
+  }
+  const SkinnyArgs a{(const __nv_bfloat16*)x, seg.w[0], nullptr, nullptr, seg.y[0], ldx, ldw[0], ldy[0], M, N[0], K};
+  return skinny_launch(a, seg, (int)tiles, splits, stream);
+}
+
+extern "C" TYR_EXPORT int tyr_skinny_gemm_bf16(const void* x, const void* w, const void* bias, void* y, long long ldx,
                                                long long ldw, long long ldy, int M, int N, int K, void* stream) {
-  return skinny_launch(x, w, bias, y, ws, ldx, ldw, ldy, M, N, K, 0, 0.f, 0.f, stream);
+  return skinny_single(x, w, bias, y, ldx, ldw, ldy, M, N, K, 0, 0.f, 0.f, stream);
 }
 
 // The same with an activation in the epilogue (6: xIELU, factors act_a above zero and act_b below).
-extern "C" TYR_EXPORT int tyr_skinny_gemm_act_bf16(const void* x, const void* w, const void* bias, void* y, void* ws, long long ldx, long long ldw,
+extern "C" TYR_EXPORT int tyr_skinny_gemm_act_bf16(const void* x, const void* w, const void* bias, void* y, long long ldx, long long ldw,
                                                    long long ldy, int M, int N, int K, int act, float act_a, float act_b, void* stream) {
-  return skinny_launch(x, w, bias, y, ws, ldx, ldw, ldy, M, N, K, act, act_a, act_b, stream);
+  return skinny_single(x, w, bias, y, ldx, ldw, ldy, M, N, K, act, act_a, act_b, stream);
 }
 
 // y[M, N] = gelu(x W^T) * aux (tanh form); aux [M, N] with row stride ldaux.
-extern "C" TYR_EXPORT int tyr_skinny_gelu_mul_bf16(const void* x, const void* w, const void* aux, void* y, void* ws, long long ldx, long long ldw,
+extern "C" TYR_EXPORT int tyr_skinny_gelu_mul_bf16(const void* x, const void* w, const void* aux, void* y, long long ldx, long long ldw,
                                                    long long ldaux, long long ldy, int M, int N, int K, void* stream) {
-  return skinny_launch(x, w, nullptr, y, ws, ldx, ldw, ldy, M, N, K, 9, 0.f, 0.f, stream, aux, ldaux);
+  return skinny_single(x, w, nullptr, y, ldx, ldw, ldy, M, N, K, 9, 0.f, 0.f, stream, aux, ldaux);
 }
 
 // A product of its own for each head: y[m, h, :N] = x[m, h, :K] @ W[h]^T for `heads` heads, rows (ldx, ldy) and heads (hx, hw, hy) apart
@@ -311,7 +399,7 @@ extern "C" TYR_EXPORT int tyr_skinny_heads_bf16(const void* x, const void* w, vo
   if (M < 1 || M > 32 || N < 1 || K < 32 || (K & 31) || heads < 1 || heads > 65535) return -1;
   if ((ldx | ldw | hx | hw) & 7) return -2;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) return -3;
-  SkinnyArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, nullptr, nullptr, (__nv_bfloat16*)y, nullptr, ldx, ldw, ldy, M, N, K, hx, hw, hy, 0, 0.f, 0.f};
+  SkinnyArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, nullptr, nullptr, (__nv_bfloat16*)y, ldx, ldw, ldy, M, N, K, hx, hw, hy, 0, 0.f, 0.f};
   const dim3 grid((N + 16 * kSkWarps - 1) / (16 * kSkWarps), heads), block(kSkWarps * 32);
   const cudaStream_t st = (cudaStream_t)stream;
   return (int)(M <= 8 ? launch_dependent(skinny_heads_kernel<1>, grid, block, 0, st, a)
@@ -326,11 +414,11 @@ extern "C" TYR_EXPORT int tyr_skinny_swiglu_bf16(const void* x, const void* wg, 
   if (M < 1 || M > 32 || N < 1 || K < 32 || (K & 31)) return -1;
   if ((ldx | ldw) & 7) return -2;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wg) | reinterpret_cast<uintptr_t>(wu)) & 15) return -3;
-  SkinnyArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)wg, (const __nv_bfloat16*)wu, nullptr, (__nv_bfloat16*)y, nullptr, ldx, ldw, ldy, M, N, K};
+  SkinnyArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)wg, (const __nv_bfloat16*)wu, nullptr, (__nv_bfloat16*)y, ldx, ldw, ldy, M, N, K};
+  SkinnySegments seg{};
+  seg.n = 1;
   const dim3 grid((N + 15) / 16, 1);
+  const cudaStream_t st = (cudaStream_t)stream;
   skinny_prefer_l1();
-  if (M <= 8) launch_dependent(skinny_gemm_kernel<1, true>, dim3(grid), dim3(kSkWarps * 32), 0, (cudaStream_t)stream, a);
-  else if (M <= 16) launch_dependent(skinny_gemm_kernel<2, true>, dim3(grid), dim3(kSkWarps * 32), 0, (cudaStream_t)stream, a);
-  else launch_dependent(skinny_gemm_kernel<4, true>, dim3(grid), dim3(kSkWarps * 32), 0, (cudaStream_t)stream, a);
-  return (int)cudaGetLastError();
+  return (int)(M <= 8 ? skinny_start<1, true>(grid, st, a, seg) : M <= 16 ? skinny_start<2, true>(grid, st, a, seg) : skinny_start<4, true>(grid, st, a, seg));
 }

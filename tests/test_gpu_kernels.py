@@ -695,3 +695,17 @@ def test_skinny_swiglu_matches_reference(M, N, K):
     y = skinny_swiglu(x, wg, wu).float()
     ref = torch.nn.functional.silu(x.float() @ wg.float().T) * (x.float() @ wu.float().T)
     assert (y - ref).abs().max() < 2e-2 * max(1.0, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("M,Ns,K,splits", [(1, (40, 16, 7), 1024, 0), (5, (1024,), 3584, 0), (8, (6144, 2048, 16, 16), 1024, 0), (16, (130, 1), 4096, 0),
+                                           (17, (48, 48), 5120, 0), (32, (1024, 1024), 5120, 0), (3, (33, 64), 96, 3), (9, (15,), 32, 8)])
+def test_skinny_many_matches_reference(M, Ns, K, splits):
+    """Several matrices in one launch, and contractions shared by a cluster (also where some of its CTAs get no part).  Each sum of K bf16 products is
+    rounded to bf16 once: 2^-8 of the largest result covers it and the order of the sums."""
+    from tyr_b200.ops.skinny import skinny_many
+    g = torch.Generator().manual_seed(M + K)
+    x = torch.randn(M, K + 8, generator=g).to(torch.bfloat16).cuda()[:, 8:]
+    ws = [torch.randn(N, K + 16, generator=g).mul_(K ** -0.5).to(torch.bfloat16).cuda()[:, 8:8 + K] for N in Ns]
+    for y, w in zip(skinny_many(x, ws, splits), ws):
+        ref = x.double() @ w.double().T
+        assert y.shape == ref.shape and (y.double() - ref).abs().max() <= 2.0 ** -8 * ref.abs().max() + 1e-6

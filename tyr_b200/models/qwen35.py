@@ -21,7 +21,7 @@ from ..ops import moe as moe_ops
 from ..ops.attention import attention
 from ..ops.decode_attention import decode_attention, geometry_supported
 from ..ops.rope import rope_norm
-from .common import KVCache, LinearState, apply_rotary_partial, cached_attention, cos_sin_tables, head_norm, lin, norm_w, plain_inv_freq, swiglu_mlp
+from .common import KVCache, LinearState, apply_rotary_partial, cached_attention, cos_sin_tables, head_norm, lin, lin_many, norm_w, plain_inv_freq, swiglu_mlp
 from .generation import SamplingStrategy, generate_cached
 from .laguna import name_candidates
 from .session import HybridSession
@@ -283,7 +283,7 @@ def attention_core_decode(cfg: Qwen35Config, q_norm, k_norm, qg, k, v, cos_table
 
 
 def attention_forward(cfg: Qwen35Config, a: Attention, x, cos, sin, cache: Optional[KVCache], attn_mask=None):
-    o = attention_core(cfg, a.q_norm, a.k_norm, lin(x, a.q_proj), lin(x, a.k_proj), lin(x, a.v_proj), cos, sin, cache, attn_mask)
+    o = attention_core(cfg, a.q_norm, a.k_norm, *lin_many(x, (a.q_proj, a.k_proj, a.v_proj)), cos, sin, cache, attn_mask)
     return lin(o, a.o_proj)
 
 
@@ -339,7 +339,7 @@ def gated_delta_net_core(cfg: Qwen35Config, m, mixed, z, b, a, state: Optional[L
 def gated_delta_net_forward(cfg: Qwen35Config, m: GatedDeltaNet, x, state: Optional[LinearState] = None, attn_mask=None):
     if attn_mask is not None:
         x = x * attn_mask.to(x.dtype).unsqueeze(-1)
-    core = gated_delta_net_core(cfg, m, lin(x, m.in_proj_qkv), lin(x, m.in_proj_z), lin(x, m.in_proj_b), lin(x, m.in_proj_a), state)
+    core = gated_delta_net_core(cfg, m, *lin_many(x, (m.in_proj_qkv, m.in_proj_z, m.in_proj_b, m.in_proj_a)), state)
     return lin(core, m.out_proj)
 
 
@@ -440,8 +440,8 @@ class HybridCache(HybridSession):
         for i, l in enumerate(m.layers):
             if cfg.is_full(i):
                 a = l.mixer
-                o = attention_core_decode(cfg, a.q_norm, a.k_norm, lin(h1, a.q_proj), lin(h1, a.k_proj), lin(h1, a.v_proj), self.cos, self.sin,
-                                          self.pos_t, self.kv[i])
+                o = attention_core_decode(cfg, a.q_norm, a.k_norm, *lin_many(h1, (a.q_proj, a.k_proj, a.v_proj)), self.cos, self.sin, self.pos_t,
+                                          self.kv[i])
                 mixed = lin(o, a.o_proj)
             else:
                 mixed = gated_delta_net_forward(cfg, l.mixer, h1, self.lin[i])

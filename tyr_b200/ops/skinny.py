@@ -3,7 +3,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from typing import Optional
+from typing import List, Optional, Sequence
 
 import torch
 
@@ -11,16 +11,7 @@ from .._native import register_signatures
 from ._common import check, cur_stream, lib, ptr
 
 MAX_ROWS = 32
-_workspaces = {}
-
-
-def _workspace(device, M: int, N: int) -> torch.Tensor:
-    """fp32 [M * N] scratch of the split reduction; zero between calls (the finishing kernel re-zeroes what it read)."""
-    key = (device.index, M * N)
-    ws = _workspaces.get(key)
-    if ws is None:
-        ws = _workspaces[key] = torch.zeros(M * N, dtype=torch.float32, device=device)
-    return ws
+MAX_MATRICES = 4         # of one launch (skinny_many)
 
 
 @register_signatures
@@ -28,14 +19,13 @@ def _sigs(lib_):
     P, I, L = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
     fn = getattr(lib_, "tyr_skinny_gemm_bf16", None)
     if fn is not None:
-        fn.argtypes = [P, P, P, P, P, L, L, L, I, I, I, P]
+        fn.argtypes = [P, P, P, P, L, L, L, I, I, I, P]
         fn.restype = I
-        lib_.tyr_skinny_gemm_splits.argtypes = [I, I]
-        lib_.tyr_skinny_gemm_splits.restype = I
     F = ctypes.c_float
-    for name, args in (("tyr_skinny_gemm_act_bf16", [P, P, P, P, P, L, L, L, I, I, I, I, F, F, P]),
+    for name, args in (("tyr_skinny_gemm_act_bf16", [P, P, P, P, L, L, L, I, I, I, I, F, F, P]),
                        ("tyr_skinny_heads_bf16", [P, P, P, L, L, L, L, L, L, I, I, I, I, P]),
-                       ("tyr_skinny_gelu_mul_bf16", [P, P, P, P, P, L, L, L, L, I, I, I, P])):
+                       ("tyr_skinny_gelu_mul_bf16", [P, P, P, P, L, L, L, L, I, I, I, P]),
+                       ("tyr_skinny_many_bf16", [P, L, I, P, P, P, P, P, I, I, I, P])):
         fn = getattr(lib_, name, None)
         if fn is not None:
             fn.argtypes, fn.restype = args, I
@@ -71,9 +61,24 @@ def skinny_linear(x2: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor
     y = torch.empty((M, N), dtype=torch.bfloat16, device=x2.device) if out is None else out
     assert y.shape == (M, N) and y.dtype == torch.bfloat16 and y.stride(1) == 1
     b = None if bias is None else bias.to(torch.bfloat16).contiguous()
-    ws = _workspace(x2.device, M, N) if lib().tyr_skinny_gemm_splits(N, K) > 1 else None
-    check(lib().tyr_skinny_gemm_bf16(ptr(x2), ptr(w), ptr(b), ptr(y), ptr(ws), x2.stride(0), w.stride(0), y.stride(0), M, N, K, cur_stream(x2.device)), "skinny_gemm_bf16")
+    check(lib().tyr_skinny_gemm_bf16(ptr(x2), ptr(w), ptr(b), ptr(y), x2.stride(0), w.stride(0), y.stride(0), M, N, K, cur_stream(x2.device)), "skinny_gemm_bf16")
     return y
+
+
+def skinny_many(x2: torch.Tensor, ws: Sequence[torch.Tensor], splits: int = 0) -> List[torch.Tensor]:
+    """``[x2 w^T for w in ws]`` in one launch: x2 [M <= 32, K] bf16, up to four matrices [N_i, K] bf16 (rows may be strided).  ``splits``: CTAs
+    of a cluster that share a contraction (0: by size)."""
+    M, K = x2.shape
+    if not x2.is_cuda:
+        return [(x2.float() @ w.float().T).to(x2.dtype) for w in ws]
+    if not (all(w.shape[1] == K and w.dtype == torch.bfloat16 and w.stride(1) == 1 for w in ws) and x2.dtype == torch.bfloat16 and x2.stride(1) == 1):
+        raise ValueError("skinny_many takes bf16 rows and matrices over one contraction")
+    n = len(ws)
+    ys = [torch.empty((M, w.shape[0]), dtype=torch.bfloat16, device=x2.device) for w in ws]
+    P, L, I = ctypes.c_void_p * n, ctypes.c_longlong * n, ctypes.c_int * n
+    check(lib().tyr_skinny_many_bf16(ptr(x2), x2.stride(0), n, P(*[w.data_ptr() for w in ws]), P(*[y.data_ptr() for y in ys]), L(*[w.stride(0) for w in ws]),
+                                     L(*[y.stride(0) for y in ys]), I(*[w.shape[0] for w in ws]), M, K, splits, cur_stream(x2.device)), "skinny_many")
+    return ys
 
 
 _SWIGLU = os.environ.get("TYR_SKINNY_SWIGLU", "1") != "0"
@@ -102,8 +107,7 @@ def skinny_xielu(x2: torch.Tensor, w: torch.Tensor, a: float, b: float) -> torch
     M, K = x2.shape
     N = w.shape[0]
     y = torch.empty((M, N), dtype=torch.bfloat16, device=x2.device)
-    ws = _workspace(x2.device, M, N) if lib().tyr_skinny_gemm_splits(N, K) > 1 else None
-    check(lib().tyr_skinny_gemm_act_bf16(ptr(x2), ptr(w), None, ptr(y), ptr(ws), x2.stride(0), w.stride(0), N, M, N, K, 6, a, b, cur_stream(x2.device)),
+    check(lib().tyr_skinny_gemm_act_bf16(ptr(x2), ptr(w), None, ptr(y), x2.stride(0), w.stride(0), N, M, N, K, 6, a, b, cur_stream(x2.device)),
           "skinny_xielu")
     return y
 
@@ -114,8 +118,7 @@ def skinny_gelu_mul(x2: torch.Tensor, w: torch.Tensor, e: torch.Tensor) -> torch
     N = w.shape[0]
     assert e.shape == (M, N) and e.dtype == torch.bfloat16 and e.stride(1) == 1
     y = torch.empty((M, N), dtype=torch.bfloat16, device=x2.device)
-    ws = _workspace(x2.device, M, N) if lib().tyr_skinny_gemm_splits(N, K) > 1 else None
-    check(lib().tyr_skinny_gelu_mul_bf16(ptr(x2), ptr(w), ptr(e), ptr(y), ptr(ws), x2.stride(0), w.stride(0), e.stride(0), N, M, N, K, cur_stream(x2.device)),
+    check(lib().tyr_skinny_gelu_mul_bf16(ptr(x2), ptr(w), ptr(e), ptr(y), x2.stride(0), w.stride(0), e.stride(0), N, M, N, K, cur_stream(x2.device)),
           "skinny_gelu_mul")
     return y
 
