@@ -258,6 +258,42 @@ __global__ void __launch_bounds__(256) gated_norm_kernel(const float* __restrict
   }
 }
 
+// The same with SiLU on a read-out that the chunk scan left in bf16, the gain in bf16: half a warp per (row, head) up to 128 channels, else a
+// warp, 16 bytes a lane.  Bound by memory traffic; as library calls it was seven passes in fp32.
+__global__ void __launch_bounds__(256) gated_norm_rounded_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ z, long long ld_z,
+                                                                 const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, long long units,
+                                                                 int Hv, int dv, float eps) {
+  pdl_entry();
+  const int group = dv <= 128 ? 16 : 32, d = (threadIdx.x & (group - 1)) * 8;
+  const bool live = d < dv;
+  const long long per_block = 256 / group;
+  for (long long u = blockIdx.x * per_block + threadIdx.x / group; u < (units + per_block - 1) / per_block * per_block; u += gridDim.x * per_block) {
+    const bool ok = live && u < units;
+    float x[8] = {}, g[8] = {}, wv[8] = {};
+    if (ok) {
+      const uint4 a = *reinterpret_cast<const uint4*>(o + u * dv + d), b = *reinterpret_cast<const uint4*>(z + u / Hv * ld_z + u % Hv * dv + d),
+                  c = *reinterpret_cast<const uint4*>(w + d);
+      const uint32_t ua[4] = {a.x, a.y, a.z, a.w}, ub[4] = {b.x, b.y, b.z, b.w}, uc[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 fa = unpack_bf16x2(ua[j]), fb = unpack_bf16x2(ub[j]), fc = unpack_bf16x2(uc[j]);
+        x[2 * j] = fa.x; x[2 * j + 1] = fa.y;
+        g[2 * j] = fb.x; g[2 * j + 1] = fb.y;
+        wv[2 * j] = fc.x; wv[2 * j + 1] = fc.y;
+      }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += x[j] * x[j];
+    for (int m = group >> 1; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+    const float rstd = 1.f / sqrtf(ss / dv + eps);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = x[j] * rstd * wv[j] * dg_gate(g[j], 0);
+    if (ok)
+      *reinterpret_cast<uint4*>(y + u * dv + d) = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+  }
+}
+
 // The same for wide heads (all of a layer's channels normed together): one CTA per (row, head).
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) gated_norm_wide_kernel(const float* __restrict__ o, const T* __restrict__ z, long long ld_z,
@@ -418,4 +454,14 @@ extern "C" TYR_EXPORT int tyr_gated_norm(const float* o, const void* z, long lon
     return (int)launch_dependent(gated_norm_kernel<float>, grid, dim3(256), 0, st, o, (const float*)z, ld_z, w, (float*)y, ld_y, rows, Hv, dv, eps, act);
   return (int)launch_dependent(gated_norm_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, o, (const __nv_bfloat16*)z, ld_z, w, (__nv_bfloat16*)y, ld_y,
                                rows, Hv, dv, eps, act);
+}
+
+// y = o / rms(o) * w * silu(z) per head, all bf16: o and y [rows, Hv, dv] contiguous, z rows of stride ld_z; dv a multiple of 8 up to 256.
+extern "C" TYR_EXPORT int tyr_gated_norm_rounded(const void* o, const void* z, long long ld_z, const void* w, void* y, long long rows, int Hv, int dv,
+                                                 float eps, void* stream) {
+  if (rows <= 0 || Hv <= 0 || dv < 8 || dv > 256 || (dv & 7) || (ld_z & 7)) return -1;
+  if ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) return -2;
+  const long long units = rows * Hv, per_block = dv <= 128 ? 16 : 8, want = (units + per_block - 1) / per_block;
+  return (int)launch_dependent(gated_norm_rounded_kernel, dim3(static_cast<unsigned>(want < 148LL * 16 ? want : 148LL * 16)), dim3(256), 0, (cudaStream_t)stream,
+                               (const __nv_bfloat16*)o, (const __nv_bfloat16*)z, ld_z, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, units, Hv, dv, eps);
 }

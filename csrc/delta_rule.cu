@@ -1107,15 +1107,19 @@ __global__ void __launch_bounds__(256, 2) gdr_chunk_prepare_channel_kernel(GdrPr
 
 // Causal depthwise conv1d (kernel taps K <= 4, zero history) + bias + SiLU on channels-last activations:
 //   y[b, s, c] = silu(bias[c] + sum_j w[c, j] * x[b, s - (K - 1) + j, c]).
-// One thread per (32 tokens, 8 channels): its taps and a sliding window of K rows stay in registers, so every input row is
-// loaded once and a warp's accesses are 512 contiguous bytes.  The reference transposes to channels-first
+// A thread owns 8 channels (16 bytes) of CONV_TOK tokens and issues the loads of all their rows and of the K - 1 before them first; the
+// window is read again from cache by the thread of the next tokens.  Bound by memory traffic.  A sliding window of 32 tokens whose
+// loads waited for one another took 21.8 us for 333 tokens of 6144 channels; this form 11.7 us, the wait for the product in front of it included.  The thread of the last tokens also leaves the last K inputs of its channels in `window` ([B, C, K], zeros
+// before the start), where a decoding step goes on.  The reference transposes to channels-first
 // and calls the library's grouped convolution (Tyr/Model/Qwen35/Model.lean:642-700).
 namespace tyr {
-constexpr int CONV_TOK = 32;      // tokens per thread: the taps and the sliding window stay in registers
-template <int K>
-__global__ void __launch_bounds__(256) causal_conv1d_silu_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
-                                                                 const float* __restrict__ bias, __nv_bfloat16* __restrict__ y,
-                                                                 long long total, int S, int C, long long x_sb, long long x_ss) {
+constexpr int CONV_TOK = 8;
+template <int K, typename W>
+__global__ void __launch_bounds__(256) causal_conv1d_silu_kernel(const __nv_bfloat16* __restrict__ x, const W* __restrict__ w,
+                                                                 const W* __restrict__ bias, __nv_bfloat16* __restrict__ y,
+                                                                 __nv_bfloat16* __restrict__ window, long long total, int S, int C,
+                                                                 long long x_sb, long long x_ss) {
+  pdl_entry();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int c8 = C >> 3;
@@ -1124,76 +1128,84 @@ __global__ void __launch_bounds__(256) causal_conv1d_silu_kernel(const __nv_bflo
   const int nblk = (S + CONV_TOK - 1) / CONV_TOK;
   const int s0 = static_cast<int>(bt % nblk) * CONV_TOK;
   const long long b = bt / nblk;
+  const __nv_bfloat16* xb = x + b * x_sb + c;
+  uint4 rows[CONV_TOK + K - 1];                      // inputs s0 - (K - 1) .. s0 + CONV_TOK - 1
+#pragma unroll
+  for (int r = 0; r < CONV_TOK + K - 1; ++r) {
+    const int t = s0 - (K - 1) + r;
+    rows[r] = (t >= 0 && t < S) ? *reinterpret_cast<const uint4*>(xb + static_cast<long long>(t) * x_ss) : make_uint4(0u, 0u, 0u, 0u);
+  }
   float wt[8][K], bs[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
-    bs[e] = bias ? bias[c + e] : 0.f;
+    bs[e] = bias ? static_cast<float>(bias[c + e]) : 0.f;
 #pragma unroll
-    for (int j = 0; j < K; ++j) wt[e][j] = w[(c + e) * K + j];
+    for (int j = 0; j < K; ++j) wt[e][j] = static_cast<float>(w[(c + e) * K + j]);
   }
-  float win[K][8];                                   // win[j] = x[s - (K - 1) + j]
-  const __nv_bfloat16* xb = x + b * x_sb + c;
-  auto load_row = [&](int t, float (&dst)[8]) {
-    if (t < 0 || t >= S) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) dst[e] = 0.f;
-      return;
-    }
-    const uint4 u = *reinterpret_cast<const uint4*>(xb + static_cast<long long>(t) * x_ss);
-    const uint32_t uu[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = unpack_bf16x2(uu[e]);
-      dst[2 * e] = f.x;
-      dst[2 * e + 1] = f.y;
-    }
-  };
-#pragma unroll
-  for (int j = 0; j < K - 1; ++j) load_row(s0 - (K - 1) + j, win[j]);
-  for (int s = s0; s < min(S, s0 + CONV_TOK); ++s) {
-    load_row(s, win[K - 1]);
-    uint4 o;
-    uint32_t* oo = reinterpret_cast<uint32_t*>(&o);
+  for (int s = 0; s < CONV_TOK; ++s) {
+    if (s0 + s >= S) break;
     float acc[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      acc[e] = bs[e];
+    for (int e = 0; e < 8; ++e) acc[e] = bs[e];
 #pragma unroll
-      for (int j = 0; j < K; ++j) acc[e] += win[j][e] * wt[e][j];
+    for (int j = 0; j < K; ++j) {
+      const uint32_t uu[4] = {rows[s + j].x, rows[s + j].y, rows[s + j].z, rows[s + j].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = unpack_bf16x2(uu[e]);
+        acc[2 * e] += f.x * wt[2 * e][j];
+        acc[2 * e + 1] += f.y * wt[2 * e + 1][j];
+      }
     }
+    uint4 o;
+    uint32_t* oo = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float a0 = acc[2 * e], a1 = acc[2 * e + 1];
       oo[e] = pack_bf16x2(a0 / (1.f + __expf(-a0)), a1 / (1.f + __expf(-a1)));
     }
-    *reinterpret_cast<uint4*>(y + (b * S + s) * C + c) = o;
-#pragma unroll
-    for (int j = 0; j < K - 1; ++j)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) win[j][e] = win[j + 1][e];
+    *reinterpret_cast<uint4*>(y + (b * S + s0 + s) * C + c) = o;
   }
+  if (window != nullptr && s0 + CONV_TOK >= S) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const int t = S - K + j;
+      const uint4 u = t >= 0 ? *reinterpret_cast<const uint4*>(xb + static_cast<long long>(t) * x_ss) : make_uint4(0u, 0u, 0u, 0u);
+      const uint32_t uu[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        window[(b * C + c + e) * K + j] = __ushort_as_bfloat16(static_cast<unsigned short>(uu[e >> 1] >> ((e & 1) * 16)));
+    }
+  }
+}
+
+template <int K, typename W>
+static cudaError_t conv_launch(const void* x, const void* w, const void* bias, void* y, void* window, int B, int S, int C, long long x_sb,
+                               long long x_ss, cudaStream_t st) {
+  const long long total = static_cast<long long>(B) * ((S + CONV_TOK - 1) / CONV_TOK) * (C >> 3);
+  return launch_dependent(causal_conv1d_silu_kernel<K, W>, dim3(static_cast<unsigned>((total + 255) / 256)), dim3(256), 0, st, (const __nv_bfloat16*)x,
+                          (const W*)w, (const W*)bias, (__nv_bfloat16*)y, (__nv_bfloat16*)window, total, S, C, x_sb, x_ss);
 }
 }  // namespace tyr
 
-// x: bf16 [B, S, C] with (batch, token) element strides and contiguous channels; w: fp32 [C, K]; bias: fp32 [C] or null;
-// y: bf16 [B, S, C] contiguous.  C must be a multiple of 8.
-extern "C" TYR_EXPORT int tyr_causal_conv1d_silu(const void* x, const float* w, const float* bias, void* y, int B, int S, int C,
-                                                 int K, long long x_sb, long long x_ss, void* stream) {
+// x, y: bf16 [B, S, C] (x by batch and token strides); w [C, K] and bias [C] (nullable) in fp32, or bf16 with `w_bf16`; window: bf16 [B, C, K] (nullable).
+extern "C" TYR_EXPORT int tyr_causal_conv1d_silu(const void* x, const void* w, const void* bias, void* y, void* window, int B, int S, int C,
+                                                 int K, long long x_sb, long long x_ss, int w_bf16, void* stream) {
+  using namespace tyr;
   if (B <= 0 || S <= 0 || C <= 0 || (C & 7) || K <= 0 || K > 4 || (x_sb & 7) || (x_ss & 7)) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) return -2;
-  const long long total = static_cast<long long>(B) * ((S + tyr::CONV_TOK - 1) / tyr::CONV_TOK) * (C >> 3);
-  const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
-  auto* xx = reinterpret_cast<const __nv_bfloat16*>(x);
-  auto* yy = reinterpret_cast<__nv_bfloat16*>(y);
-  cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+#define TYR_CONV(k) \
+  case k: return (int)(w_bf16 ? conv_launch<k, __nv_bfloat16>(x, w, bias, y, window, B, S, C, x_sb, x_ss, st) : conv_launch<k, float>(x, w, bias, y, window, B, S, C, x_sb, x_ss, st))
   switch (K) {
-    case 1: tyr::causal_conv1d_silu_kernel<1><<<blocks, 256, 0, cs>>>(xx, w, bias, yy, total, S, C, x_sb, x_ss); break;
-    case 2: tyr::causal_conv1d_silu_kernel<2><<<blocks, 256, 0, cs>>>(xx, w, bias, yy, total, S, C, x_sb, x_ss); break;
-    case 3: tyr::causal_conv1d_silu_kernel<3><<<blocks, 256, 0, cs>>>(xx, w, bias, yy, total, S, C, x_sb, x_ss); break;
-    case 4: tyr::causal_conv1d_silu_kernel<4><<<blocks, 256, 0, cs>>>(xx, w, bias, yy, total, S, C, x_sb, x_ss); break;
-    default: return -3;
+    TYR_CONV(1);
+    TYR_CONV(2);
+    TYR_CONV(3);
+    TYR_CONV(4);
   }
-  return static_cast<int>(cudaGetLastError());
+#undef TYR_CONV
+  return -3;
 }
 
 // Chunk-local quantities of the gated delta rule (chunk 64, dk and dv multiples of 8 up to 128).  q, k: bf16 [B, S, Hk, dk] and

@@ -1,0 +1,141 @@
+// What lies between the projections and the mixer of a gated full-attention layer, over prompts:
+//   * attention_operands: per-head RMS norm (gain 1 + w) and partial rotation of queries and keys, and the rows of keys and values in the
+//     store, where attention reads them;
+//   * attention_gate:     the attention output times sigmoid of the gate that the query projection carries beside each head.
+//
+// Both are bound by memory traffic: every operand passes through once, 16 bytes a lane, one warp per (token, head).  As library calls
+// they were 27 passes over the same rows (contiguous copies, conversions, norms, concatenations, store writes).
+// Compiled without fast math.  A prompt of 333 tokens through Qwen3.5 0.8B took 1007 launches and 13.4 ms (6.3 ms of it on the GPU) and takes 414 and
+// 8.7 ms (4.6) with these and the fused passes of csrc/delta_rule.cu and csrc/delta_general.cu; 4 x 2048 tokens through 8 layers of the 27B widths 61.6 and 55.6 ms.
+#include "common.cuh"
+
+namespace tyr {
+
+__device__ __forceinline__ void pm_load8(const __nv_bfloat16* p, float (&f)[8]) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 v = unpack_bf16x2(w[i]);
+    f[2 * i] = v.x;
+    f[2 * i + 1] = v.y;
+  }
+}
+__device__ __forceinline__ void pm_store8(__nv_bfloat16* p, const float (&f)[8]) {
+  *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+}
+
+struct OperandArgs {
+  const __nv_bfloat16 *q, *k, *v;        // rows of B * S tokens, head h at column h * head_stride
+  long long q_row, k_row, v_row, q_head; // keys and values: heads D apart
+  const __nv_bfloat16 *qw, *kw;          // gains [D]
+  const float *cosT, *sinT;              // [S, half]: the tables' rows of these tokens
+  __nv_bfloat16* q_out;                  // [B, S, H, D]
+  __nv_bfloat16 *k_store, *v_store;      // [B, G, cap, D], written from slot `slot0` on
+  int B, S, H, G, D, half, cap, slot0;
+  float eps;
+};
+
+// Lane l keeps channels 8 l .. 8 l + 7 of a head (D <= 256), and the channels that rotate with them are half / 8 lanes away.
+__global__ void __launch_bounds__(256) attention_operands_kernel(OperandArgs a) {
+  pdl_entry();
+  const int lane = threadIdx.x & 31, heads = a.H + 2 * a.G, d = lane * 8, shift = a.half >> 3;
+  const bool live = d < a.D;
+  const long long total = static_cast<long long>(a.B) * a.S * heads;
+  for (long long i = blockIdx.x * 8LL + (threadIdx.x >> 5); i < total; i += gridDim.x * 8LL) {
+    const int h = static_cast<int>(i % heads);
+    const long long row = i / heads;
+    const int b = static_cast<int>(row / a.S), s = static_cast<int>(row % a.S);
+    const bool is_q = h < a.H, is_v = h >= a.H + a.G;
+    const int g = is_q ? h : (is_v ? h - a.H - a.G : h - a.H);
+    const __nv_bfloat16* src = is_q ? a.q + row * a.q_row + g * a.q_head : (is_v ? a.v + row * a.v_row : a.k + row * a.k_row) + static_cast<long long>(g) * a.D;
+    __nv_bfloat16* dst = is_q ? a.q_out + (row * a.H + g) * a.D
+                              : (is_v ? a.v_store : a.k_store) + ((static_cast<long long>(b) * a.G + g) * a.cap + a.slot0 + s) * a.D;
+    if (is_v) {
+      if (live) *reinterpret_cast<uint4*>(dst + d) = *reinterpret_cast<const uint4*>(src + d);
+      continue;
+    }
+    float x[8] = {}, w[8] = {};
+    if (live) {
+      pm_load8(src + d, x);
+      pm_load8((is_q ? a.qw : a.kw) + d, w);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += x[j] * x[j];
+    const float rstd = 1.f / sqrtf(warp_sum(ss) / a.D + a.eps);
+    const bool first = d < a.half, second = !first && d < 2 * a.half;
+    const int partner = first ? lane + shift : second ? lane - shift : lane;
+    const float* c = a.cosT + static_cast<long long>(s) * a.half + (first ? d : d - a.half);
+    const float* sn = a.sinT + static_cast<long long>(s) * a.half + (first ? d : d - a.half);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      x[j] = x[j] * rstd * (1.f + w[j]);
+      const float other = __shfl_sync(0xffffffffu, x[j], partner);
+      w[j] = first ? x[j] * c[j] - other * sn[j] : second ? x[j] * c[j] + other * sn[j] : x[j];
+    }
+    if (live) pm_store8(dst + d, w);
+  }
+}
+
+struct GateOutArgs {
+  const __nv_bfloat16 *o, *gate;
+  long long o_b, o_s, o_h, gate_row, gate_head;     // element strides of o [B, S, H, D] and gate [B * S, H, D]
+  __nv_bfloat16* y;                                 // [B * S, H * D]
+  long long rows;
+  int S, H, D;
+};
+
+__global__ void __launch_bounds__(256) attention_gate_kernel(GateOutArgs a) {
+  pdl_entry();
+  const int vecs = a.D >> 3;
+  const long long total = a.rows * a.H * vecs;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
+    const int d = static_cast<int>(i % vecs) * 8;
+    const long long t = i / vecs, row = t / a.H;
+    const int h = static_cast<int>(t % a.H);
+    float o[8], g[8];
+    pm_load8(a.o + row / a.S * a.o_b + row % a.S * a.o_s + h * a.o_h + d, o);
+    pm_load8(a.gate + row * a.gate_row + h * a.gate_head + d, g);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] *= 1.f / (1.f + expf(-g[j]));
+    pm_store8(a.y + t * a.D + d, o);
+  }
+}
+
+inline unsigned pm_grid(long long units, int per_block) {
+  const long long want = (units + per_block - 1) / per_block;
+  return static_cast<unsigned>(want < 148LL * 16 ? want : 148LL * 16);
+}
+
+}  // namespace tyr
+
+using namespace tyr;
+
+// strides: q row, k row, v row, q head (elements); dims: B, S, H, G, D, half, cap, slot0.  The head size is a multiple of 8 up to 256, the rotated
+// half a multiple of 8, all rows 16-byte aligned; slot0 + S <= cap.
+extern "C" TYR_EXPORT int tyr_attention_operands(const void* q, const void* k, const void* v, const long long* strides, const void* qw, const void* kw,
+                                                 const float* cosT, const float* sinT, void* q_out, void* k_store, void* v_store, const int* dims,
+                                                 float eps, void* stream) {
+  OperandArgs a{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, strides[0], strides[1], strides[2], strides[3],
+                (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, cosT, sinT, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_store, (__nv_bfloat16*)v_store,
+                dims[0], dims[1], dims[2], dims[3], dims[4], dims[5], dims[6], dims[7], eps};
+  if (a.B < 1 || a.S < 1 || a.H < 1 || a.G < 1 || a.D < 8 || a.D > 256 || (a.D & 7) || a.half < 8 || (a.half & 7) || 2 * a.half > a.D) return -1;
+  if (a.slot0 < 0 || a.slot0 + static_cast<long long>(a.S) > a.cap) return -2;
+  if ((a.q_row | a.k_row | a.v_row | a.q_head) & 7) return -3;
+  for (const void* p : {q, k, v, qw, kw, (const void*)q_out, (const void*)k_store, (const void*)v_store})
+    if (p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15)) return -4;
+  return (int)launch_dependent(attention_operands_kernel, dim3(pm_grid(1LL * a.B * a.S * (a.H + 2 * a.G), 8)), dim3(256), 0, (cudaStream_t)stream, a);
+}
+
+// y [rows, H * D] = o * sigmoid(gate); o [rows / S, S, H, D] by (batch, token, head) strides, gate [rows, H, D] by (row, head) strides.
+extern "C" TYR_EXPORT int tyr_attention_gate(const void* o, const void* gate, const long long* strides, void* y, long long rows, int S, int H, int D,
+                                             void* stream) {
+  if (rows < 1 || S < 1 || rows % S || H < 1 || D < 8 || (D & 7)) return -1;
+  for (int i = 0; i < 5; ++i)
+    if (strides[i] & 7) return -3;
+  for (const void* p : {o, gate, (const void*)y})
+    if (p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15)) return -4;
+  const GateOutArgs a{(const __nv_bfloat16*)o, (const __nv_bfloat16*)gate, strides[0], strides[1], strides[2], strides[3], strides[4], (__nv_bfloat16*)y, rows, S, H, D};
+  return (int)launch_dependent(attention_gate_kernel, dim3(pm_grid(rows * H * (D / 8), 256)), dim3(256), 0, (cudaStream_t)stream, a);
+}

@@ -194,3 +194,71 @@ def test_gpu_qwen35_dense_graph_decode_matches_full_forward():
         for t in range(130, 140):
             assert (c.step(ids[:, t]).float() - full[:, t]).abs().max().item() < 0.06 * scale, t
         assert c._graph.replays == 10 and int(c.pos_t) == 140
+
+
+# ---- prompts: the passes between projections and mixers ------------------------------------------------------------------------------------
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,S,H,G,D,half", [(1, 1, 2, 1, 64, 8), (2, 37, 8, 2, 256, 32), (3, 130, 4, 4, 128, 64), (1, 5, 3, 1, 40, 16)])
+def test_attention_operands_and_gate(B, S, H, G, D, half):
+    """Norm, rotation and store rows against fp64; each number is rounded to bf16 once (2^-8 relative, and 2^-8 of the larger of a rotated pair)."""
+    from tyr_b200.models.common import KVCache
+    from tyr_b200.ops import prompt_mix as pm
+    g = torch.Generator(device="cuda").manual_seed(S + D)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    wide = r(B, S, H * 2 * D + 2 * G * D)
+    q, k, v = wide[..., :H * 2 * D], wide[..., H * 2 * D:H * 2 * D + G * D], wide[..., H * 2 * D + G * D:]
+    qn, kn = r(D) * 0.1, r(D) * 0.1
+    ang = torch.rand(S, half, device="cuda", generator=g) * 6
+    cos, sin = ang.cos(), ang.sin()
+    store = KVCache.allocate(B, G, S + 3, D, "cuda", torch.bfloat16)
+    store.length = 2
+    assert pm.operands_supported(q, k, v, store, qn, kn, cos, D)
+    got = pm.attention_operands(q, 2 * D, k, v, qn, kn, cos, sin, 1e-6, H, G, D, store)
+
+    def want(t, w):
+        t = t.double()
+        t = t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True) + 1e-6) * (1 + w.double())
+        a, b, c, s = t[..., :half], t[..., half:2 * half], cos.double()[:, None], sin.double()[:, None]
+        return torch.cat([a * c - b * s, b * c + a * s, t[..., 2 * half:]], -1)
+    qg = q.unflatten(-1, (H, 2 * D))
+    for y, ref in ((got, want(qg[..., :D], qn)), (store.k[:, :, 2:S + 2].transpose(1, 2), want(k.unflatten(-1, (G, D)), kn))):
+        assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all()
+    assert store.length == S + 2 and torch.equal(store.v[:, :, 2:S + 2].transpose(1, 2), v.unflatten(-1, (G, D)))
+    assert not store.k[:, :, :2].any() and not store.k[:, :, S + 2:].any() and not store.v[:, :, S + 2:].any()
+    store.length = store.cap - S + 1
+    with pytest.raises(ValueError, match="overflow"):
+        pm.attention_operands(q, 2 * D, k, v, qn, kn, cos, sin, 1e-6, H, G, D, store)
+    o = r(B, H, S, D).transpose(1, 2)
+    y = pm.attention_gate(o, q[..., D:], 2 * D)
+    ref = (o.double() * torch.sigmoid(qg[..., D:].double())).flatten(2)
+    assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-6).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,S,C,K,bias", [(1, 1, 16, 4, True), (2, 3, 8, 4, False), (1, 8, 64, 3, True), (3, 41, 264, 4, True), (2, 16, 24, 1, False)])
+def test_causal_conv_and_window(B, S, C, K, bias):
+    from tyr_b200.ops import delta_rule as DR
+    g = torch.Generator(device="cuda").manual_seed(S + C)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, w, b = r(B, S, C + 8)[..., 8:], r(C, K), r(C) if bias else None
+    y, win = DR.causal_conv1d_window(x, w, b)
+    pad = torch.nn.functional.pad(x.double(), (0, 0, K - 1, 0))
+    z = sum(pad[:, j:j + S] * w.double()[:, j] for j in range(K)) + (0 if b is None else b.double())
+    ref = torch.nn.functional.silu(z)
+    assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all()
+    assert torch.equal(win, torch.nn.functional.pad(x, (0, 0, K, 0))[:, -K:].transpose(1, 2))
+    assert torch.equal(y, DR.causal_conv1d_silu(x, w.float(), None if b is None else b.float()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,S,Hv,dv", [(1, 1, 1, 8), (2, 19, 3, 128), (1, 5, 2, 72), (1, 40, 2, 256), (1, 3, 1, 136)])
+def test_gated_norm_of_a_rounded_readout(B, S, Hv, dv):
+    from tyr_b200.ops import delta_rule as DR
+    g = torch.Generator(device="cuda").manual_seed(S + dv)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    o, z, w = r(B, S, Hv, dv), r(B, S, Hv * dv + 8)[..., :Hv * dv], r(dv)
+    with torch.no_grad():
+        y = DR.gated_norm_rounded(o, z, w, 1e-6)
+    od = o.double()
+    ref = (od * torch.rsqrt(od.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()).flatten(2) * torch.nn.functional.silu(z.double())
+    assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-6).all()

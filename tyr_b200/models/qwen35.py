@@ -18,6 +18,7 @@ import torch.nn.functional as F
 from ..io import safetensors as st
 from ..ops import delta_rule as dr
 from ..ops import moe as moe_ops
+from ..ops import prompt_mix
 from ..ops.attention import attention
 from ..ops.decode_attention import decode_attention, geometry_supported
 from ..ops.rope import rope_norm
@@ -252,6 +253,12 @@ def attention_core(cfg: Qwen35Config, q_norm, k_norm, qg, k, v, cos, sin, cache:
     its local counts).  Returns [B, S, H*D]."""
     B, S, _ = qg.shape
     H, Hkv, D = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
+    if (attn_mask is None and cache is not None and cache.length == 0 and not torch.is_grad_enabled()
+            and prompt_mix.operands_supported(qg, k, v, cache, q_norm, k_norm, cos, D)):
+        # a fresh prompt: one pass makes the queries and the store's rows, which attention reads, and one gates its output
+        q = prompt_mix.attention_operands(qg, 2 * D, k, v, q_norm, k_norm, cos, sin, cfg.rms_norm_eps, H, Hkv, D, cache)
+        o = attention(q.transpose(1, 2), *cache.view(), causal=True)
+        return prompt_mix.attention_gate(o.transpose(1, 2), qg[..., D:], 2 * D)
     qg = qg.reshape(B, S, H, 2 * D)
     q, gate = qg[..., :D], qg[..., D:].reshape(B, S, H * D)
     k = k.reshape(B, S, Hkv, D)
@@ -306,8 +313,8 @@ def gated_delta_net_core(cfg: Qwen35Config, m, mixed, z, b, a, state: Optional[L
     if step and state.rec is not None and dr.gdn_decode_fused_supported(mixed, state.conv, state.rec, dk, dv):
         return dr.gdn_decode_fused(mixed, z, b, a, state.conv, m.conv1d_weight, m.conv1d_bias, m.dt_bias, m.a_log, m.norm_weight,
                                    cfg.rms_norm_eps, state.rec, Hk, Hv, dk, dv)
-    w = m.conv1d_weight.reshape(cd, K).to(mixed.dtype)
     if step:
+        w = m.conv1d_weight.reshape(cd, K).to(mixed.dtype)
         window = torch.cat([state.conv[:, :, 1:], mixed.transpose(1, 2)], dim=2)       # [B, cd, K]
         y = (window.float() * w.float()).sum(-1)
         if m.conv1d_bias is not None:
@@ -315,23 +322,29 @@ def gated_delta_net_core(cfg: Qwen35Config, m, mixed, z, b, a, state: Optional[L
         conv_out = F.silu(y).to(mixed.dtype).unsqueeze(1)                                 # [B, 1, cd]
         state.conv.copy_(window)                                                          # in place: the step is graph-replayable
     else:
-        xc = mixed.transpose(1, 2)
-        conv_out = dr.causal_conv1d_silu(mixed, m.conv1d_weight.reshape(cd, K), m.conv1d_bias)
+        w = m.conv1d_weight.reshape(cd, K)
         if state is not None:
-            state.conv = (xc[:, :, S - K:] if S >= K else F.pad(xc, (K - S, 0))).contiguous()
+            conv_out, state.conv = dr.causal_conv1d_window(mixed, w, m.conv1d_bias)
+        else:
+            conv_out = dr.causal_conv1d_silu(mixed, w, m.conv1d_bias)
     kd = cfg.linear_key_dim
     q = conv_out[..., :kd].reshape(B, S, Hk, dk)
     k = conv_out[..., kd:2 * kd].reshape(B, S, Hk, dk)
     v = conv_out[..., 2 * kd:].reshape(B, S, Hv, dv)
-    beta = torch.sigmoid(b.float())
-    g = -F.softplus(a.float() + m.dt_bias.float()) * torch.exp(m.a_log.float())
-    rep = Hv // Hk
+    if b.is_cuda and not torch.is_grad_enabled() and b.dtype == a.dtype and m.dt_bias.dtype == m.a_log.dtype == torch.float32:
+        g, beta = dr.delta_gates(b, a, m.dt_bias, m.a_log)
+    else:
+        beta = torch.sigmoid(b.float())
+        g = -F.softplus(a.float() + m.dt_bias.float()) * torch.exp(m.a_log.float())
     if step and state.rec is not None:
         core = dr.gdr_decode_step(q.contiguous(), k.contiguous(), v.contiguous(), g, beta, state.rec)
     else:
         core, rec = dr.chunk_gated_delta_rule(q, k, v, g, beta, state=state.rec if state is not None else None)    # keys stay grouped
         if state is not None:
             state.rec = rec.contiguous()
+    y = dr.gated_norm_rounded(core, z.reshape(B, S, Hv * dv), m.norm_weight, cfg.rms_norm_eps)
+    if y is not None:
+        return y
     core = rms_norm_gated(core.reshape(B * S * Hv, dv), z.reshape(B * S * Hv, dv), m.norm_weight, cfg.rms_norm_eps)
     return core.reshape(B, S, Hv * dv)
 
@@ -352,19 +365,31 @@ def moe_forward(cfg: Qwen35Config, m: SparseMoeBlock, x2: torch.Tensor) -> torch
     return moe_ops.moe_dense_forward(x2, ids, w, m.gate_up_proj, m.down_proj, counts=counts, add=shared)
 
 
-def layer_forward(cfg, i, layer: Layer, x, cos, sin, kv: Optional[KVCache], lin_state: Optional[LinearState], attn_mask=None):
+def _sublayers(cfg, i, layer: Layer, x, h1, cos, sin, kv: Optional[KVCache], lin_state: Optional[LinearState], attn_mask=None):
+    """One layer on the residual stream ``x`` and its norm ``h1``: (stream after the mixer, the feed-forward's output yet to be added)."""
     B, S, h = x.shape
-    h1 = rms(x, layer.input_layernorm, cfg.rms_norm_eps)
     if cfg.is_full(i):
         mixed = attention_forward(cfg, layer.mixer, h1, cos, sin, kv, attn_mask)
     else:
         mixed = gated_delta_net_forward(cfg, layer.mixer, h1, lin_state, attn_mask)
-    h2 = x + mixed
-    h3 = rms(h2, layer.post_attention_layernorm, cfg.rms_norm_eps)
+    h3, h2 = _add_norm(mixed, layer.post_attention_layernorm, cfg.rms_norm_eps, x)
     if isinstance(layer.ffn, MLP):
         f = swiglu_mlp(h3, layer.ffn.gate_proj, layer.ffn.up_proj, layer.ffn.down_proj)
     else:
         f = moe_forward(cfg, layer.ffn, h3.reshape(B * S, h)).reshape(B, S, h)
+    return h2, f
+
+
+def _add_norm(y, w, eps, x):
+    """(norm of ``x + y``, ``x + y``); one pass where no gradient is asked for."""
+    if torch.is_grad_enabled():
+        r = x + y
+        return rms(r, w, eps), r
+    return norm_w(y, w, eps, one_plus_w=True, residual=x, return_residual=True)
+
+
+def layer_forward(cfg, i, layer: Layer, x, cos, sin, kv: Optional[KVCache], lin_state: Optional[LinearState], attn_mask=None):
+    h2, f = _sublayers(cfg, i, layer, x, rms(x, layer.input_layernorm, cfg.rms_norm_eps), cos, sin, kv, lin_state, attn_mask)
     return h2 + f
 
 
@@ -403,10 +428,14 @@ class HybridCache(HybridSession):
         cfg, S = self.m.cfg, x.shape[1]
         self._check_room(S)
         cos, sin = self.cos[self.pos:self.pos + S], self.sin[self.pos:self.pos + S]
-        for i, l in enumerate(self.m.layers):
-            x = layer_forward(cfg, i, l, x, cos, sin, self.kv[i], self.lin[i])
+        layers = self.m.layers
+        h1 = rms(x, layers[0].input_layernorm, cfg.rms_norm_eps)
+        for i, l in enumerate(layers):
+            x, f = _sublayers(cfg, i, l, x, h1, cos, sin, self.kv[i], self.lin[i])
+            if i + 1 < len(layers):
+                h1, x = _add_norm(f, layers[i + 1].input_layernorm, cfg.rms_norm_eps, x)
         self._advance([S] * self.batch)
-        return x
+        return x + f
 
     def run(self, x: torch.Tensor) -> torch.Tensor:
         return self.head(self._norm(self.run_hidden(x)[:, -1]))

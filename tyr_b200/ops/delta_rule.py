@@ -52,7 +52,7 @@ def _sigs(lib_):
         fn.restype = ctypes.c_int
     fn = getattr(lib_, "tyr_causal_conv1d_silu", None)
     if fn is not None:
-        fn.argtypes = [P, P, P, P, I, I, I, I, L, L, P]
+        fn.argtypes = [P, P, P, P, P, I, I, I, I, L, L, I, P]
         fn.restype = ctypes.c_int
     F = ctypes.c_float
     for name, args in (("tyr_conv_silu", [P, P, P, I, I, I, I, L, L, I, P]),
@@ -60,6 +60,7 @@ def _sigs(lib_):
                        ("tyr_delta_gates", [P, P, L, L, P, P, P, P, L, I, I, P]),
                        ("tyr_gdr_recurrent", [P] * 8 + [ctypes.POINTER(L), I, I, I, I, I, I, I, P]),
                        ("tyr_gdr_recurrent_channel", [P] * 10 + [ctypes.POINTER(L), I, I, I, I, I, I, I, P]),
+                       ("tyr_gated_norm_rounded", [P, P, L, P, P, L, I, I, F, P]),
                        ("tyr_gated_norm", [P, P, L, P, P, L, L, I, I, F, I, I, P])):
         fn = getattr(lib_, name, None)
         if fn is not None:
@@ -137,6 +138,34 @@ def chunk_gated_delta_rule_fused(q, k, v, g, beta, state: Optional[torch.Tensor]
     return out, st_out
 
 
+def _conv_kernel_ok(x: torch.Tensor, K: int) -> bool:
+    return (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[2] % 8 == 0 and K <= 4 and x.stride(2) == 1 and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0
+            and x.data_ptr() % 16 == 0 and hasattr(lib(), "tyr_causal_conv1d_silu"))
+
+
+def _conv_kernel(x, weight, bias, window):
+    B, S, C = x.shape
+    K = weight.shape[-1]
+    y = torch.empty((B, S, C), dtype=x.dtype, device=x.device)
+    low = weight.dtype == torch.bfloat16 and (bias is None or bias.dtype == torch.bfloat16)      # taps in the activations' type are read as they are
+    w = (weight.reshape(C, K) if low else weight.reshape(C, K).float()).contiguous()
+    b = None if bias is None else (bias if low else bias.float()).contiguous()
+    check(lib().tyr_causal_conv1d_silu(ptr(x), ptr(w), ptr(b), ptr(y), ptr(window), B, S, C, K, x.stride(0), x.stride(1), 1 if low else 0, cur_stream(x.device)),
+          "causal_conv1d_silu")
+    return y
+
+
+def causal_conv1d_window(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
+    """:func:`causal_conv1d_silu` and the last K inputs of every channel [B, C, K] (zeros before the start), where a decoding step goes on."""
+    B, S, C = x.shape
+    K = weight.shape[-1]
+    if _conv_kernel_ok(x, K):
+        window = torch.empty((B, C, K), dtype=x.dtype, device=x.device)
+        return _conv_kernel(x, weight, bias, window), window
+    xc = x.transpose(1, 2)
+    return causal_conv1d_silu(x, weight, bias), (xc[:, :, S - K:] if S >= K else torch.nn.functional.pad(xc, (K - S, 0))).contiguous()
+
+
 def causal_conv1d_silu(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """x: [B, S, C] (channels last), weight: [C, K] -> silu(causal depthwise conv + bias) as [B, S, C], zero history."""
     B, S, C = x.shape
@@ -146,13 +175,8 @@ def causal_conv1d_silu(x: torch.Tensor, weight: torch.Tensor, bias: Optional[tor
         wf = weight.reshape(C, K).float().contiguous()
         check(lib().tyr_conv_silu(ptr(x), ptr(wf), ptr(y), B, S, C, K, x.stride(0), x.stride(1), _dt(x), cur_stream(x.device)), "conv_silu")
         return y
-    if (x.is_cuda and x.dtype == torch.bfloat16 and C % 8 == 0 and K <= 4 and x.stride(2) == 1 and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0
-            and x.data_ptr() % 16 == 0 and hasattr(lib(), "tyr_causal_conv1d_silu")):
-        y = torch.empty((B, S, C), dtype=x.dtype, device=x.device)
-        wf = weight.reshape(C, K).float().contiguous()
-        bf = None if bias is None else bias.float().contiguous()
-        check(lib().tyr_causal_conv1d_silu(ptr(x), ptr(wf), ptr(bf), ptr(y), B, S, C, K, x.stride(0), x.stride(1), cur_stream(x.device)), "causal_conv1d_silu")
-        return y
+    if _conv_kernel_ok(x, K):
+        return _conv_kernel(x, weight, bias, None)
     xc = x.transpose(1, 2)
     y = torch.nn.functional.conv1d(torch.nn.functional.pad(xc, (K - 1, 0)), weight.reshape(C, 1, K).to(xc.dtype), None if bias is None else bias.to(xc.dtype), groups=C)
     return torch.nn.functional.silu(y).transpose(1, 2)
@@ -348,6 +372,21 @@ def gated_norm(o: torch.Tensor, z: torch.Tensor, w: torch.Tensor, eps: float, ac
     assert y.dtype == z.dtype and y.shape == (B, S, Hv * dv)
     check(lib().tyr_gated_norm(ptr(o), ptr(z), row_stride(z), ptr(w), ptr(y), row_stride(y), B * S, Hv, dv, eps, {"silu": 0, "sigmoid": 1}[act], _dt(z),
                                cur_stream(z.device)), "gated_norm")
+    return y
+
+
+def gated_norm_rounded(o: torch.Tensor, z: torch.Tensor, w: torch.Tensor, eps: float) -> Optional[torch.Tensor]:
+    """:func:`gated_norm` (SiLU) of a bf16 read-out with a bf16 gain; None for what its kernel does not take."""
+    B, S, Hv, dv = o.shape
+    if not (o.is_cuda and o.dtype == z.dtype == w.dtype == torch.bfloat16 and o.is_contiguous() and w.is_contiguous() and dv % 8 == 0 and dv <= 256
+            and z.stride(2) == 1 and z.stride(1) % 8 == 0 and (B == 1 or S == 1 or z.stride(0) == S * z.stride(1)) and not torch.is_grad_enabled()
+            and all(t.data_ptr() % 16 == 0 for t in (o, z, w))):
+        return None
+    ld = z.stride(1) if S > 1 else z.stride(0)
+    if ld % 8:
+        return None
+    y = torch.empty((B, S, Hv * dv), dtype=z.dtype, device=z.device)
+    check(lib().tyr_gated_norm_rounded(ptr(o), ptr(z), ld, ptr(w), ptr(y), B * S, Hv, dv, eps, cur_stream(z.device)), "gated_norm_rounded")
     return y
 
 
