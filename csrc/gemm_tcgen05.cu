@@ -75,6 +75,13 @@ struct GemmParams {
   //  m_rot rotates the order of row tiles so that every rank starts with a different peer (mode 1)
   //  or with its own rows (mode 2).
   int tp_mode, tp_rank, tp_world, rows_per_rank, m_rot;
+  // > 0: the column tiles of several products that share A, one after the other: product s has seg_N[s] columns and the tiles from seg_tile[s]
+  // on, TmapPeers m[s] describes its B and m[4 + s] its C (bf16 out, no batch; a tile's batch index is its product).
+  int segs;
+  int seg_tile[5], seg_N[4];
+  // gated products whose gate and up rows are two matrices: B is the gate matrix, TmapPeers m[0] the up matrix, and a tile takes
+  // BN / 2 rows of each (N counts both, ragged widths allowed).
+  int split_b;
   void* peer_c[8];
   __nv_bfloat16* gather_buf;
   int* tile_ready;
@@ -180,7 +187,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
   const int worker = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
 
   const int tiles_m = (p.M + TILE_M - 1) / TILE_M;
-  const int tiles_n = (p.N + BN - 1) / BN;
+  const int tiles_n = p.segs > 0 ? p.seg_tile[p.segs] : (p.N + BN - 1) / BN;
   const int num_kb = (p.K + BK - 1) / BK;
   // set-up that reads nothing another kernel wrote: it may overlap the tail of the kernel before this one
   pdl_trigger();
@@ -284,7 +291,17 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
     }
     const int per_batch = tiles_m * tiles_n;
     bi = static_cast<int>(tile / per_batch);
-    const int r = static_cast<int>(tile % per_batch);
+    int r = static_cast<int>(tile % per_batch);
+    if (p.segs > 0) {
+      int nt = p.raster_m ? r / tiles_m : r % tiles_n;
+      const int mt = p.raster_m ? r % tiles_m : r / tiles_n;
+      bi = 0;
+#pragma unroll
+      for (int i = 1; i < 4; ++i) bi = (i < p.segs && nt >= p.seg_tile[i]) ? i : bi;
+      m0 = mt * TILE_M + static_cast<int>(cta_rank) * BM;
+      n0 = (nt - p.seg_tile[bi]) * BN;
+      return;
+    }
     // n fastest: concurrently resident tiles share A rows and keep B (weights) in L2.
     if (p.raster_m) {
       m0 = (r % tiles_m) * TILE_M;
@@ -339,6 +356,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
         int bi, m0, n0;
         decode_tile(tile, bi, m0, n0);
         const int a_src = p.tp_mode == 2 ? m0 / p.rows_per_rank : 0;
+        const CUtensorMap* tb = p.segs > 0 ? &tmP.m[bi] : &tmB;
+        const int z = p.segs > 0 ? 0 : bi;
         if (p.tp_mode == 2 && a_src != p.tp_rank) {
           // rows of a peer: wait until every gather warp has copied its part of this row tile
           const int* flag = p.tile_ready + m0 / BM;
@@ -372,7 +391,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
             const uint32_t bar = mapa_shared(smem_u32(&s.full[st]), 0);
             if (cta_rank == 0) mbar_expect_tx(&s.full[st], 2 * kStageBytes);
             if (!A_MN) {
-              tma_load_3d_pair(s.a[st], &tmA, bar, k0, m0, bi);
+              tma_load_3d_pair(s.a[st], &tmA, bar, k0, m0, z);
             } else {
 #pragma unroll
               for (int c = 0; c < BM / 64; ++c)
@@ -380,7 +399,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
             }
             const int nb = n0 + static_cast<int>(cta_rank) * BNL;
             if (!B_MN) {
-              tma_load_3d_pair(s.b[st], &tmB, bar, k0, nb, bi);
+              if (p.split_b) tma_load_3d_pair(s.b[st], cta_rank == 0 ? &tmB : &tmP.m[0], bar, k0, n0 / 2, 0);
+              else tma_load_3d_pair(s.b[st], tb, bar, k0, nb, z);
             } else {
 #pragma unroll
               for (int c = 0; c < BNL / 64; ++c)
@@ -395,14 +415,19 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
             else if (p.tp_mode == 2 && a_src == p.tp_rank)
               tma_load_3d(s.a[st], &tmP.m[a_src], &s.full[st], k0, m0 - a_src * p.rows_per_rank, bi);
             else
-              tma_load_3d(s.a[st], &tmA, &s.full[st], k0, m0, bi);
+              tma_load_3d(s.a[st], &tmA, &s.full[st], k0, m0, z);
           } else {
 #pragma unroll
             for (int c = 0; c < BM / 64; ++c)
               tma_load_3d(s.a[st] + c * (64 * BK * 2), &tmA, &s.full[st], m0 + c * 64, k0, bi);
           }
           if (!B_MN) {
-            tma_load_3d(s.b[st], &tmB, &s.full[st], k0, n0, bi);
+            if (p.split_b) {
+              tma_load_3d(s.b[st], &tmB, &s.full[st], k0, n0 / 2, 0);
+              tma_load_3d(s.b[st] + (BN / 2) * (BK * 2), &tmP.m[0], &s.full[st], k0, n0 / 2, 0);
+            } else {
+              tma_load_3d(s.b[st], tb, &s.full[st], k0, n0, z);
+            }
           } else {
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c)
@@ -534,6 +559,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       }
       tc_fence_after();
       int row = m0 + quarter * 32 + lane;
+      const int N = p.segs > 0 ? p.seg_N[bi] : p.N;
       const uint32_t t_row = tmem_base + buf * BN + (static_cast<uint32_t>(quarter * 32) << 16);
       bool row_ok = row < p.M;
       long long c_off, x_off;
@@ -574,7 +600,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           }
           }
           const int col = n0 / 2 + c * 32;
-          if (!row_ok || col >= p.N / 2) continue;
+          if (!row_ok || col >= N / 2) continue;
           __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + c_off + col;
           float v[32];
           if (p.act == 8) {
@@ -588,7 +614,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                                        : 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)));
             v[j] = a * (p.beta * __uint_as_float(ru[j]));
           }
-          if (col + 32 <= p.N / 2) {
+          if (col + 32 <= N / 2) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               uint4 u;
@@ -601,7 +627,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (col + j < p.N / 2) out[j] = __float2bfloat16(v[j]);
+              if (col + j < N / 2) out[j] = __float2bfloat16(v[j]);
           }
         }
         ++seg;
@@ -623,16 +649,16 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
         }
         const int col = n0 + c * 32;
         if (tma_out) {
-          if (col >= p.N) continue;            // a tile that ends inside the last valid chunk was flushed there
+          if (col >= N) continue;            // a tile that ends inside the last valid chunk was flushed there
           if (!(c & 1)) {                      // about to refill a staging tile: its previous store must have read it
             if (lane == 0) tma_store_wait_read<EPI_BUFS - 1>();
             __syncwarp();
           }
-        } else if (!row_ok || col >= p.N) {
+        } else if (!row_ok || col >= N) {
           continue;
         }
         float v[32];
-        const bool full = (col + 32 <= p.N);
+        const bool full = (col + 32 <= N);
         const bool use_aux = p.aux != nullptr && (p.beta != 0.f || p.act == 3 || p.act == 9) && row_ok;
         float ax[32];
         if (use_aux) {
@@ -648,7 +674,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
             }
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) ax[j] = (col + j < p.N) ? __bfloat162float(axp[j]) : 0.f;
+            for (int j = 0; j < 32; ++j) ax[j] = (col + j < N) ? __bfloat162float(axp[j]) : 0.f;
           }
         } else {
 #pragma unroll
@@ -673,18 +699,18 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
             const int chunk = (c & 1) * 4 + q;                       // 16-byte chunk of the 128-byte row
             *reinterpret_cast<uint4*>(st + ((chunk ^ (lane & 7)) << 4)) = u;
           }
-          if ((c & 1) || col + 32 >= p.N) {
+          if ((c & 1) || col + 32 >= N) {
             fence_proxy_async();
             __syncwarp();
             if (lane == 0 && m0 + quarter * 32 < p.M) {
               int y = m0 + quarter * 32;
-              const CUtensorMap* tm = &tmC;
+              const CUtensorMap* tm = p.segs > 0 ? &tmP.m[4 + bi] : &tmC;
               if (p.tp_mode == 1) {
                 const int owner = m0 / p.rows_per_rank;
                 tm = &tmP.m[owner];
                 y = p.tp_rank * p.rows_per_rank + (y - owner * p.rows_per_rank);
               }
-              tma_store_3d(tm, s.out_stage[epi][n_stores % EPI_BUFS], col - (c & 1) * 32, y, bi);
+              tma_store_3d(tm, s.out_stage[epi][n_stores % EPI_BUFS], col - (c & 1) * 32, y, p.segs > 0 ? 0 : bi);
               tma_store_commit();
             }
             ++n_stores;
@@ -704,7 +730,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           } else {
             #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (col + j < p.N) out[j] = __float2bfloat16(v[j]);
+              if (col + j < N) out[j] = __float2bfloat16(v[j]);
           }
         } else if (p.out_mode == 1) {
           float* out = reinterpret_cast<float*>(p.C) + c_off + col;
@@ -716,7 +742,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           } else {
             #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (col + j < p.N) out[j] = v[j];
+              if (col + j < N) out[j] = v[j];
           }
         } else {
           float* out = reinterpret_cast<float*>(p.C) + c_off + col;
@@ -729,7 +755,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           } else {
             #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (col + j < p.N) atomicAdd(out + j, v[j]);
+              if (col + j < N) atomicAdd(out + j, v[j]);
           }
         }
       }
@@ -812,6 +838,13 @@ struct TyrGemmArgs {
   void* stream;
   const int* group_offsets;         // grouped (MoE) mode, see GemmParams
   const int* group_tiles;
+  int tile_rows;                    // 128 or 256 (0 = choose)
+  int segs;                         // 2 .. 4: that many products of A (plain, bf16 out); B, C, N, ldb and ldc of each below
+  const void* B2;                   // gated products: the up matrix [N / 2, K] (B: the gate matrix, same stride); null: one interleaved matrix
+  const void* seg_B[4];
+  void* seg_C[4];
+  long long seg_ldb[4], seg_ldc[4];
+  int seg_N[4];
 };
 
 }  // extern "C"
@@ -846,6 +879,7 @@ static int launch_gemm(const TyrGemmArgs& a, const CUtensorMap& tmA, const CUten
                        const tyr::TmapPeers& tmP, const tyr::GemmParams& tp) {
   using namespace tyr;
   auto kern = gemm_bf16_tcgen05_kernel<BN, STAGES, A_MN, B_MN, PAIR>;
+  static_assert(sizeof(GemmSmem<PAIR ? BN / 2 : BN, STAGES, PAIR ? 8 : 4, PAIR ? 1 : 2>) + 1024 <= 232448, "shared memory of one SM");
   constexpr size_t smem = sizeof(GemmSmem<PAIR ? BN / 2 : BN, STAGES, PAIR ? 8 : 4, PAIR ? 1 : 2>) + 1024;
   constexpr unsigned kThreads = PAIR ? 320 : 256;
   static bool configured[kMaxGemmDevices] = {false};
@@ -880,12 +914,23 @@ static int launch_gemm(const TyrGemmArgs& a, const CUtensorMap& tmA, const CUten
   p.alpha = a.alpha; p.beta = a.beta; p.act = a.act; p.out_mode = a.out_mode; p.err = a.err;
   p.group_offsets = a.group_offsets;
   p.group_tiles = a.group_tiles;
+  p.segs = a.segs;
+  p.split_b = a.B2 != nullptr ? 1 : 0;
+  int seg_tiles = 0, seg_cols = 0;
+  for (int i = 0; i < a.segs; ++i) {
+    p.seg_tile[i] = seg_tiles;
+    p.seg_N[i] = a.seg_N[i];
+    seg_tiles += (a.seg_N[i] + BN - 1) / BN;
+    seg_cols += a.seg_N[i];
+  }
+  p.seg_tile[a.segs] = seg_tiles;
   p.tp_mode = tp.tp_mode; p.tp_rank = tp.tp_rank; p.tp_world = tp.tp_world;
   p.rows_per_rank = tp.rows_per_rank; p.m_rot = tp.m_rot;
   for (int i = 0; i < 8; ++i) p.peer_c[i] = tp.peer_c[i];
   p.gather_buf = tp.gather_buf; p.tile_ready = tp.tile_ready; p.lda = a.lda;
   constexpr int TILE_M = PAIR ? 2 * BM : BM;
   long long tiles = static_cast<long long>((a.M + TILE_M - 1) / TILE_M) * ((a.N + BN - 1) / BN) * a.batch;
+  if (a.segs > 0) tiles = static_cast<long long>((a.M + TILE_M - 1) / TILE_M) * seg_tiles;
   if (a.group_offsets != nullptr)   // host-side bound: every group may add one partial m-tile
     tiles = ((a.sA + BM - 1) / BM + (a.batch < a.sA ? a.batch : a.sA)) * ((a.N + BN - 1) / BN);
   // `grid` counts scheduler units: CTAs, or CTA pairs
@@ -896,7 +941,7 @@ static int launch_gemm(const TyrGemmArgs& a, const CUtensorMap& tmA, const CUten
     if (grid < 1) grid = 1;
   }
   if (a.out_mode != 2 && tiles < grid) grid = static_cast<int>(tiles);
-  p.raster_m = (a.group_offsets == nullptr && tp.tp_mode == 0 && a.M < a.N && g_raster_m) ? 1 : 0;
+  p.raster_m = (a.group_offsets == nullptr && tp.tp_mode == 0 && a.M < (a.segs > 0 ? seg_cols : a.N) && g_raster_m) ? 1 : 0;
   p.l2_prefetch = (a.group_offsets == nullptr && tp.tp_mode == 0) ? g_l2_prefetch : 0;
   p.sk_slabs = 0;
   if (a.out_mode == 2) {
@@ -966,6 +1011,33 @@ struct TyrTpArgs {
 };
 }
 
+// The output tile of a product whose tiles are handed out whole.  A tile of a pair's 256 x 256 is the only one that the tensor cores
+// bound; the smaller ones wait for L2 -> SM traffic (24 KB a k block and SM, about 125 GB/s), but drain sooner, and a product of few
+// tiles leaves fewer SMs idle with them.  Model in us per round of tiles, kb = k blocks of 64; fitted to products back to back in a graph,
+// weights from HBM (M x N x K: 256 x 256 / 256 x 128 / 128 x 128 / 128 x 64):
+//   333 x 1024 x 1024    11.5 /  8.8 /  8.5 /  7.9      256 x 9216 x 3072    23.7 / 18.8 / 18.9 / 28.3
+//   333 x 3072 x 12288   63.9 / 46.2 / 48.9 / 49.0      333 x 9216 x 3072    24.9 / 27.9 / 29.0 / 39.0
+//   750 x 1024 x 256      7.9 /  6.3 /  5.7 /  5.1      8000 x 3072 x 768    32.3 / 39.7 / 42.6 / 76.9
+static void choose_tile(const TyrGemmArgs& a, int* rows, int* bn) {
+  struct Tile { int rows, bn; double first0, first_kb, next0, next_kb; };
+  static const Tile tiles[] = {{256, 256, 7.0, 0.275, 0.8, 0.3}, {256, 128, 5.7, 0.2, 0.9, 0.195}, {128, 128, 4.9, 0.225, 1.0, 0.205}, {128, 64, 4.2, 0.23, 1.0, 0.2}};
+  const int sms = a.sm_count > 0 ? a.sm_count : device_sm_count();
+  const double kb = (a.K + 63) / 64;
+  double best = -1;
+  for (const Tile& t : tiles) {
+    long long cols = 0;
+    if (a.segs > 0)
+      for (int i = 0; i < a.segs; ++i) cols += (a.seg_N[i] + t.bn - 1) / t.bn;
+    else
+      cols = (a.N + t.bn - 1) / t.bn;
+    const long long n = (a.M + t.rows - 1LL) / t.rows * cols * a.batch;
+    const long long at_once = t.rows == 256 ? (sms > 1 ? sms / 2 : 1) : sms;
+    double cost = t.first0 + t.first_kb * kb + static_cast<double>((n + at_once - 1) / at_once - 1) * (t.next0 + t.next_kb * kb);
+    if (best >= 0) cost *= 1.1;        // within a tenth the 256 x 256 tile stays: with ties given away, a training step of depth 12 took 0.8 % longer
+    if (best < 0 || cost < best) { best = cost; *rows = t.rows; *bn = t.bn; }
+  }
+}
+
 static int gemm_impl(const TyrGemmArgs& a, const TyrTpArgs* tpa) {
   using namespace tyr;
   GemmParams tp{};
@@ -1002,15 +1074,27 @@ static int gemm_impl(const TyrGemmArgs& a, const TyrTpArgs* tpa) {
       return -10;
     }
   }
-  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.batch <= 0) return -1;
+  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.batch <= 0) return -1;       // with segs: B, C and N are those of the first product
   if ((reinterpret_cast<uintptr_t>(a.A) & 15) || (reinterpret_cast<uintptr_t>(a.B) & 15) ||
       (reinterpret_cast<uintptr_t>(a.C) & 15))
     return -2;
   if ((a.lda & 7) || (a.ldb & 7) || (a.group_offsets == nullptr && (a.sA & 7)) || (a.sB & 7)) return -3;
   if (a.out_mode == 0 ? (a.ldc & 7) : (a.ldc & 3)) return -4;
   if (a.aux && ((a.ldaux & 7) || (reinterpret_cast<uintptr_t>(a.aux) & 15))) return -5;
-  int bn = a.bn;
+  int bn = a.bn, rows = a.tile_rows;
+  const bool gated = a.act == 4 || a.act == 5 || a.act == 8;
+  if (a.segs != 0) {
+    if (a.segs < 2 || a.segs > 4 || tpa != nullptr || a.group_offsets != nullptr || a.a_mn || a.b_mn || a.batch != 1 || a.out_mode != 0 || gated || a.aux) return -15;
+    for (int i = 0; i < a.segs; ++i)
+      if (a.seg_N[i] <= 0 || (a.seg_ldb[i] & 7) || (a.seg_ldc[i] & 7) || (reinterpret_cast<uintptr_t>(a.seg_B[i]) & 15) || (reinterpret_cast<uintptr_t>(a.seg_C[i]) & 15)) return -15;
+  }
+  if (a.B2 != nullptr && (!gated || tpa != nullptr || a.group_offsets != nullptr || a.b_mn || a.batch != 1 || (a.N & 15) || (reinterpret_cast<uintptr_t>(a.B2) & 15))) return -16;
+  // tiles of other sizes: products whose tiles are handed out whole
+  const bool free_tile = tpa == nullptr && a.group_offsets == nullptr && a.out_mode != 2 && (!gated || a.B2 != nullptr);
+  if (!free_tile && (bn == 64 || rows == 128)) return -6;
+  if (bn == 0 && rows == 0 && free_tile && g_pair_enabled) choose_tile(a, &rows, &bn);
   if (bn == 0) bn = (a.N <= 128) ? 128 : 256;
+  if (rows == 0) rows = bn == 256 ? 256 : 128;
   CUtensorMap tmA, tmB;
   int r;
   if (a.group_offsets != nullptr) {
@@ -1023,15 +1107,27 @@ static int gemm_impl(const TyrGemmArgs& a, const TyrTpArgs* tpa) {
     r = make_tmap_bf16_3d(&tmA, a.A, a.M, a.K, a.batch, a.lda, a.sA, BK);
   if (r) return 3000 + r;
   // CTA pairs: plain products with a K-major A whose tiles are 256 columns wide
-  const bool pair = g_pair_enabled && tpa == nullptr && a.group_offsets == nullptr && bn == 256 &&
+  const bool pair = g_pair_enabled && tpa == nullptr && a.group_offsets == nullptr && rows == 256 &&
                     (a.out_mode != 2 || g_aligned_split);
+  if (!pair && rows == 256 && bn != 256) return -6;
+  const int box_b = pair || a.B2 != nullptr ? bn / 2 : bn;          // rows of one load of a K-major B
   if (!a.b_mn)
-    r = make_tmap_bf16_3d(&tmB, a.B, a.K, a.N, a.batch, a.ldb, a.sB, pair ? bn / 2 : bn);
+    r = make_tmap_bf16_3d(&tmB, a.B, a.K, a.B2 != nullptr ? a.N / 2 : a.N, a.batch, a.ldb, a.sB, box_b);
   else
     r = make_tmap_bf16_3d(&tmB, a.B, a.N, a.K, a.batch, a.ldb, a.sB, BK);
   if (r) return 4000 + r;
+  if (a.B2 != nullptr) {
+    r = make_tmap_bf16_3d(&tmP.m[0], a.B2, a.K, a.N / 2, 1, a.ldb, 0, box_b);
+    if (r) return 4000 + r;
+  }
+  for (int i = 0; i < a.segs; ++i) {
+    r = make_tmap_bf16_3d(&tmP.m[i], a.seg_B[i], a.K, a.seg_N[i], 1, a.seg_ldb[i], 0, box_b);
+    if (r) return 4000 + r;
+    r = make_tmap_bf16_3d(&tmP.m[4 + i], a.seg_C[i], a.seg_N[i], a.M, 1, a.seg_ldc[i], 0, 32);
+    if (r) return 6000 + r;
+  }
   CUtensorMap tmC{};
-  if (a.out_mode == 0 && a.group_offsets == nullptr && a.act != 4 && a.act != 5 && a.act != 8) {
+  if (a.out_mode == 0 && a.group_offsets == nullptr && !gated && a.segs == 0) {
     if (tpa != nullptr && tpa->mode == 1) {
       for (int i = 0; i < tpa->world; ++i) {
         r = make_tmap_bf16_3d(&tmP.m[i], tpa->peers[i], a.N, static_cast<uint64_t>(tpa->world) * tpa->rows_per_rank, 1,
@@ -1051,6 +1147,13 @@ static int gemm_impl(const TyrGemmArgs& a, const TyrTpArgs* tpa) {
     if (a.a_mn && a.b_mn) return launch_gemm<BNv, ST, true, true>(a, tmA, tmB, tmC, tmP, tp);     \
     return launch_gemm<BNv, ST, true, false>(a, tmA, tmB, tmC, tmP, tp);                      \
   } while (0)
+  if (pair && bn == 128) {
+    if (!a.a_mn && !a.b_mn) return launch_gemm<128, 7, false, false, true>(a, tmA, tmB, tmC, tmP, tp);
+    if (!a.a_mn && a.b_mn) return launch_gemm<128, 7, false, true, true>(a, tmA, tmB, tmC, tmP, tp);
+    if (a.a_mn && a.b_mn) return launch_gemm<128, 7, true, true, true>(a, tmA, tmB, tmC, tmP, tp);
+    return launch_gemm<128, 7, true, false, true>(a, tmA, tmB, tmC, tmP, tp);
+  }
+  if (pair && bn != 256) return -6;
   if (pair) {
     if (!a.a_mn && !a.b_mn) return launch_gemm<256, 6, false, false, true>(a, tmA, tmB, tmC, tmP, tp);
     if (!a.a_mn && a.b_mn) return launch_gemm<256, 6, false, true, true>(a, tmA, tmB, tmC, tmP, tp);
@@ -1059,6 +1162,7 @@ static int gemm_impl(const TyrGemmArgs& a, const TyrTpArgs* tpa) {
   }
   if (bn == 256) TYR_DISPATCH(256, 4);
   if (bn == 128) TYR_DISPATCH(128, 6);
+  if (bn == 64) TYR_DISPATCH(64, 7);
 #undef TYR_DISPATCH
   return -6;
 }

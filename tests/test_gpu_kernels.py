@@ -709,3 +709,54 @@ def test_skinny_many_matches_reference(M, Ns, K, splits):
     for y, w in zip(skinny_many(x, ws, splits), ws):
         ref = x.double() @ w.double().T
         assert y.shape == ref.shape and (y.double() - ref).abs().max() <= 2.0 ** -8 * ref.abs().max() + 1e-6
+
+
+TILES = [(256, 256), (256, 128), (128, 128), (128, 64)]
+
+
+@pytest.mark.parametrize("rows,bn", TILES)
+@pytest.mark.parametrize("a_layout,b_layout", [("K", "K"), ("K", "MN"), ("MN", "MN"), ("MN", "K")])
+@pytest.mark.parametrize("M,N,K,batch", [(8, 8, 8, 1), (136, 72, 200, 3), (264, 328, 64, 1), (520, 640, 1032, 1)])
+def test_gemm_tiles_match_reference(rows, bn, a_layout, b_layout, M, N, K, batch):
+    """Every output tile at ragged edges, plain and with a scaled addend, to bf16 and fp32.  Sums of bf16 products in fp32: 2^-8 of the largest
+    result covers the rounding to bf16, 1e-5 of it the order of fp32 sums."""
+    from tyr_b200.ops.gemm import gemm
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    a = r(batch, M, K) if a_layout == "K" else r(batch, K, M)
+    b = r(batch, N, K) if b_layout == "K" else r(batch, K, N)
+    aux = r(batch, M, N)
+    A, B = a.double() if a_layout == "K" else a.double().mT, b.double().mT if b_layout == "K" else b.double()
+    ref = A @ B
+    kw = dict(a_layout=a_layout, b_layout=b_layout, tile_rows=rows, bn=bn)
+    tol = ref.abs().max()
+    assert (gemm(a, b, **kw).double() - ref).abs().max() <= 2.0 ** -8 * tol
+    assert (gemm(a, b, out_dtype=torch.float32, **kw).double() - ref).abs().max() <= 1e-5 * tol
+    full = 0.5 * ref + 2.0 * aux.double()
+    assert (gemm(a, b, aux=aux, alpha=0.5, beta=2.0, **kw).double() - full).abs().max() <= 2.0 ** -8 * full.abs().max()
+
+
+@pytest.mark.parametrize("rows,bn", TILES + [(0, 0)])
+@pytest.mark.parametrize("M,Ns,K", [(3, (8, 16), 64), (333, (640, 8, 16, 48), 136), (300, (264, 72, 520), 1024)])
+def test_gemm_of_several_matrices(rows, bn, M, Ns, K):
+    from tyr_b200.ops.gemm import gemm_many
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, ws = r(M, K + 8)[:, 8:], [r(N, K) for N in Ns]
+    for y, w in zip(gemm_many(x, ws, tile_rows=rows, bn=bn), ws):
+        ref = x.double() @ w.double().T
+        assert y.shape == ref.shape and (y.double() - ref).abs().max() <= 2.0 ** -8 * ref.abs().max()
+
+
+@pytest.mark.parametrize("rows,bn", TILES + [(0, 0)])
+@pytest.mark.parametrize("M,N,K", [(5, 8, 64), (333, 200, 136), (300, 640, 1024)])
+def test_gated_gemm_of_two_matrices(rows, bn, M, N, K):
+    """Gate and up rows in their own matrices.  The fp32 sums differ from fp64 by 1e-5 of the largest, SiLU's exponential by 1e-6; the product is
+    rounded to bf16 once."""
+    from tyr_b200.ops.gemm import gemm
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, wg, wu = r(M, K), r(N, K) * K ** -0.5, r(N, K) * K ** -0.5
+    y = gemm(x, wg, up=wu, act="swiglu", tile_rows=rows, bn=bn)
+    ref = torch.nn.functional.silu(x.double() @ wg.double().T) * (x.double() @ wu.double().T)
+    assert y.shape == ref.shape and ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all()

@@ -192,7 +192,7 @@ def _swiglu(x, w1, w2):
 # ---- fused GPU path (bf16 inference on the hand-written kernels) ---------------------------------------------------
 # The same blocks with the element-wise glue folded into kernels: QK-norm + RoPE in one pass over the projection's output
 # (text and image rows written straight into one packed [B, S, 3, H, D] buffer, so nothing is concatenated), attention on
-# strided views of that buffer, SwiGLU in the epilogue of the gate/up product (weights re-ordered once per block), and the
+# strided views of that buffer, SwiGLU in the epilogue of the gate/up product, and the
 # single-stream block's [attention | MLP] operand of linear2 assembled in place.  At batch 4 the unfused sequence spent
 # 37 % of a denoising step in ATen element-wise and copy kernels.
 
@@ -201,19 +201,10 @@ def _fused_ok(cfg, x: torch.Tensor) -> bool:
             and cfg.mlp_hidden_dim % 128 == 0 and _flash.has_fwd() and flux_qk_post_supported(x, cfg.head_dim))
 
 
-def _gate_up_interleaved(owner, name: str, w1: torch.Tensor) -> torch.Tensor:
-    """``w1`` ([2*M, hidden], gate rows then up rows) in the gated epilogue's row order, cached on the block."""
-    key = (w1.data_ptr(), tuple(w1.shape), w1._version)
-    cached = getattr(owner, name, None)
-    if cached is None or cached[0] != key:
-        cached = (key, interleave_gate_up(w1))
-        setattr(owner, name, cached)
-    return cached[1]
-
-
-def _swiglu_fused(owner, name, x, w1, w2):
+def _swiglu_fused(x, w1, w2):
     B, S, h = x.shape
-    act = _gemm(x.reshape(B * S, h), _gate_up_interleaved(owner, name, w1), act="swiglu")
+    M = w1.shape[0] // 2
+    act = _gemm(x.reshape(B * S, h), w1[:M], up=w1[M:], act="swiglu")
     return lin(act.reshape(B, S, -1), w2)
 
 
@@ -234,9 +225,9 @@ def _double_block_fused(cfg, b: DoubleStreamBlock, img, txt, img_pe, txt_pe, mod
     attn = attn.view(B, St + Si, H * D)
     img = gate_residual(img, lin(attn[:, St:].contiguous(), b.img_attn.proj), mod_img[:, 2])
     txt = gate_residual(txt, lin(attn[:, :St].contiguous(), b.txt_attn.proj), mod_txt[:, 2])
-    img = gate_residual(img, _swiglu_fused(b, "_img_w1_il", layernorm_modulate(img, mod_img[:, 4], mod_img[:, 3], EPS),
+    img = gate_residual(img, _swiglu_fused(layernorm_modulate(img, mod_img[:, 4], mod_img[:, 3], EPS),
                                            b.img_mlp.w1, b.img_mlp.w2), mod_img[:, 5])
-    txt = gate_residual(txt, _swiglu_fused(b, "_txt_w1_il", layernorm_modulate(txt, mod_txt[:, 4], mod_txt[:, 3], EPS),
+    txt = gate_residual(txt, _swiglu_fused(layernorm_modulate(txt, mod_txt[:, 4], mod_txt[:, 3], EPS),
                                            b.txt_mlp.w1, b.txt_mlp.w2), mod_txt[:, 5])
     return img, txt
 
@@ -248,7 +239,7 @@ def _single_block_fused(cfg, b: SingleStreamBlock, x, pe, mod):
     qkv = _gemm(xm, b.linear1[:3 * H * D]).view(B, S, 3 * H * D)
     flux_qk_post(qkv, qkv, b.norm.query_norm, b.norm.key_norm, pe[0], pe[1], H, eps=EPS)      # in place; v untouched
     cat = torch.empty((B, S, H * D + M), dtype=x.dtype, device=x.device)                       # [attention | silu(gate) * up]
-    _gemm(xm, _gate_up_interleaved(b, "_mlp_w1_il", b.linear1[3 * H * D:]), act="swiglu",
+    _gemm(xm, b.linear1[3 * H * D:3 * H * D + M], up=b.linear1[3 * H * D + M:], act="swiglu",
           out=cat.view(B * S, H * D + M)[:, H * D:])
     x5 = qkv.view(B, S, 3, H, D)
     _flash.flash_fwd_bthd(x5[:, :, 0], x5[:, :, 1], x5[:, :, 2], causal=False, window=None, scale=None, need_lse=False,

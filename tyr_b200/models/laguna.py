@@ -21,7 +21,7 @@ from ..ops import decode_attention as da
 from ..ops.decode_attention import decode_attention
 from ..ops.rope import rope_norm
 from .common import (KVCache, apply_rotary_partial, cached_attention, cos_sin_tables, head_norm, lin, norm_w,
-                     plain_inv_freq, swiglu_mlp, yarn_inv_freq)
+                     plain_inv_freq, gated_mlp, swiglu_mlp, yarn_inv_freq)
 from .generation import SamplingStrategy, StreamCallback, generate_cached
 
 FULL, SLIDING = "full_attention", "sliding_attention"
@@ -377,7 +377,7 @@ def moe_forward(cfg: LagunaConfig, m: SparseMoeBlock, x2: torch.Tensor, use_fuse
     """``scale * sum_k w_k expert_k(x) + shared(x)`` over [tokens, hidden] (MoE.lean:267-356).  With ``ep`` the
     routed part runs expert-parallel: rows are pulled by the rank that owns the expert and the results pulled back."""
     ids, w, counts = route(cfg, m.router, x2)
-    shared = swiglu_mlp(x2, m.shared_gate_proj, m.shared_up_proj, m.shared_down_proj)
+    shared = gated_mlp(x2, m.shared_gate_proj, m.shared_up_proj, m.shared_down_proj)
     if ep is not None:
         from ..parallel.ep import local_expert_fn
         banks = m.experts if m.dense_experts is None else (
@@ -458,7 +458,7 @@ def layer_forward(cfg: LagunaConfig, i: int, layer: Layer, x: torch.Tensor, tabl
     h2 = x + attention_forward(cfg, i, layer.attn, h1, cos, sin, cache)
     h3 = norm_w(h2, layer.post_attention_layernorm, cfg.rms_norm_eps)
     if isinstance(layer.ffn, DenseMLP):
-        f = swiglu_mlp(h3, layer.ffn.gate_proj, layer.ffn.up_proj, layer.ffn.down_proj)
+        f = gated_mlp(h3, layer.ffn.gate_proj, layer.ffn.up_proj, layer.ffn.down_proj)
     else:
         f = moe_forward(cfg, layer.ffn, h3.reshape(B * S, h), use_fused, ep).reshape(B, S, h)
     return h2 + f

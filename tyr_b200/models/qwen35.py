@@ -22,7 +22,7 @@ from ..ops import prompt_mix
 from ..ops.attention import attention
 from ..ops.decode_attention import decode_attention, geometry_supported
 from ..ops.rope import rope_norm
-from .common import KVCache, LinearState, apply_rotary_partial, cached_attention, cos_sin_tables, head_norm, lin, lin_many, norm_w, plain_inv_freq, swiglu_mlp
+from .common import KVCache, LinearState, apply_rotary_partial, cached_attention, cos_sin_tables, gated_mlp, head_norm, lin, lin_many, norm_w, plain_inv_freq, swiglu_mlp
 from .generation import SamplingStrategy, generate_cached
 from .laguna import name_candidates
 from .session import HybridSession
@@ -360,7 +360,7 @@ def moe_forward(cfg: Qwen35Config, m: SparseMoeBlock, x2: torch.Tensor) -> torch
     """softmax router over all experts, top-k renormalised; gated shared expert added (Model.lean:162-292)."""
     logits = F.linear(x2, m.router.to(x2.dtype)).float()
     ids, w, counts = moe_ops.route(logits, cfg.num_experts_per_tok, softmax=True, renorm=True)
-    shared = swiglu_mlp(x2, m.shared_expert.gate_proj, m.shared_expert.up_proj, m.shared_expert.down_proj)
+    shared = gated_mlp(x2, m.shared_expert.gate_proj, m.shared_expert.up_proj, m.shared_expert.down_proj)
     shared = (torch.sigmoid(F.linear(x2, m.shared_expert_gate.to(x2.dtype)).float()) * shared.float()).to(x2.dtype)
     return moe_ops.moe_dense_forward(x2, ids, w, m.gate_up_proj, m.down_proj, counts=counts, add=shared)
 
@@ -374,7 +374,7 @@ def _sublayers(cfg, i, layer: Layer, x, h1, cos, sin, kv: Optional[KVCache], lin
         mixed = gated_delta_net_forward(cfg, layer.mixer, h1, lin_state, attn_mask)
     h3, h2 = _add_norm(mixed, layer.post_attention_layernorm, cfg.rms_norm_eps, x)
     if isinstance(layer.ffn, MLP):
-        f = swiglu_mlp(h3, layer.ffn.gate_proj, layer.ffn.up_proj, layer.ffn.down_proj)
+        f = gated_mlp(h3, layer.ffn.gate_proj, layer.ffn.up_proj, layer.ffn.down_proj)
     else:
         f = moe_forward(cfg, layer.ffn, h3.reshape(B * S, h)).reshape(B, S, h)
     return h2, f

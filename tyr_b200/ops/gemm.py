@@ -19,7 +19,7 @@ the epilogue math as separate kernels.
 from __future__ import annotations
 
 import ctypes
-from typing import Optional
+from typing import List, Optional, Sequence
 
 import torch
 
@@ -91,9 +91,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_layout: str = "K", b_layout: str
          out: Optional[torch.Tensor] = None, aux: Optional[torch.Tensor] = None,
          alpha: float = 1.0, beta: float = 0.0, act: Optional[str] = None,
          out_dtype: Optional[torch.dtype] = None, accumulate: bool = False,
-         bn: int = 0, sm_count: int = 0) -> torch.Tensor:
+         bn: int = 0, sm_count: int = 0, tile_rows: int = 0, up: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``up`` (gated products): the up matrix, ``b`` being the gate matrix in its own row order.  ``bn`` (64, 128, 256) and ``tile_rows`` (128, 256)
+    fix the output tile (0: by size)."""
     M, K, lda, batch_a, sA = _dims(a, a_layout, True)
     N, K2, ldb, batch_b, sB = _dims(b, b_layout, False)
+    if up is not None:
+        if act not in _GATED or up.shape != b.shape or up.stride() != b.stride() or b.dim() != 2 or b_layout != "K" or N % 8:
+            raise ValueError("gemm `up` goes with a gated activation and a K-major gate matrix of the same shape and strides")
+        N *= 2
     if K != K2:
         raise ValueError(f"gemm reduction mismatch: {tuple(a.shape)} ({a_layout}) vs {tuple(b.shape)} ({b_layout})")
     batch = max(batch_a, batch_b)
@@ -105,11 +111,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_layout: str = "K", b_layout: str
     if gated:
         # b holds, per block of 256 rows, 128 gate rows then the matching 128 up rows (`interleave_gate_up`); the result
         # is silu(alpha * gate) * (beta * up) (tanh-GELU for "geglu"), N / 2 columns wide
-        if N % 256 != 0 or b_layout != "K" or aux is not None or accumulate or batch != 1:
+        if (N % 256 != 0 and up is None) or b_layout != "K" or aux is not None or accumulate or batch != 1:
             raise ValueError("gated gemm needs K-major b with N % 256 == 0, no aux, no accumulation, no batch")
         if beta == 0.0:
             beta = 1.0
-        bn = 256
+        if up is None:
+            bn = 256
     n_out = N // 2 if gated else N
     shape = (M, n_out) if (a.dim() == 2 and b.dim() == 2) else (batch, M, n_out)
     if out_dtype is None:
@@ -119,6 +126,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_layout: str = "K", b_layout: str
             raise ValueError("accumulate=True needs an fp32 `out`")
         out_dtype = torch.float32
     if not a.is_cuda:
+        if up is not None:
+            gate_up = (a.float() if a_layout == "K" else a.float().transpose(-1, -2)) @ torch.cat([b, up]).float().T
+            g, u = gate_up[..., :n_out], gate_up[..., n_out:]
+            fn = torch.nn.functional.silu if act == "swiglu" else (lambda t: torch.nn.functional.gelu(t, approximate="tanh"))
+            res = (clamped_swiglu(g, u, alpha, beta) if act == "clamped_swiglu" else fn(alpha * g) * (beta * u)).to(out_dtype)
+            return res if out is None else out.copy_(res)
         res = _reference(a, b, a_layout, b_layout, aux, alpha, beta, act, out_dtype)
         if out is not None:
             if accumulate:
@@ -152,7 +165,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_layout: str = "K", b_layout: str
     args.out_mode = 2 if accumulate else (0 if out_dtype == torch.bfloat16 else 1)
     args.act = _ACT[act]
     args.alpha, args.beta = alpha, beta
-    args.bn, args.sm_count = bn, sm_count
+    args.bn, args.sm_count, args.tile_rows = bn, sm_count, tile_rows
+    if up is not None:
+        args.B2 = up.data_ptr()
     args.err = err_word(a.device).data_ptr()
     args.stream = cur_stream(a.device).value
     # batch==1 operands broadcast over the batch: the tensor map gets batch stride 0 only when
@@ -161,6 +176,31 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_layout: str = "K", b_layout: str
         raise ValueError("broadcast batched gemm is not supported; expand the operand")
     check(lib().tyr_gemm_bf16(ctypes.byref(args)), "tyr_gemm_bf16")
     return out
+
+
+MAX_MATRICES = 4         # of one launch (gemm_many)
+
+
+def gemm_many(a: torch.Tensor, bs: Sequence[torch.Tensor], *, bn: int = 0, tile_rows: int = 0) -> List[torch.Tensor]:
+    """``[a @ b^T for b in bs]`` in one launch: a [M, K] and two to four matrices [N_i, K] (rows may be strided), bf16."""
+    M, K = a.shape
+    if not a.is_cuda:
+        return [_reference(a, b, "K", "K", None, 1.0, 0.0, None, a.dtype) for b in bs]
+    if any(t.dtype != torch.bfloat16 or t.dim() != 2 or t.shape[1] != K or t.stride(1) != 1 for t in (a, *bs)):
+        raise TypeError("gemm_many takes bf16 rows and matrices over one contraction")
+    outs = [torch.empty((M, -(-b.shape[0] // 8) * 8), dtype=torch.bfloat16, device=a.device)[:, :b.shape[0]] for b in bs]
+    args = GemmArgs()
+    args.A, args.B, args.C = a.data_ptr(), bs[0].data_ptr(), outs[0].data_ptr()
+    args.M, args.N, args.K, args.batch = M, bs[0].shape[0], K, 1
+    args.lda, args.ldb, args.ldc = a.stride(0), bs[0].stride(0), outs[0].stride(0)
+    args.alpha = 1.0
+    args.bn, args.tile_rows, args.segs = bn, tile_rows, len(bs)
+    for i, (b, y) in enumerate(zip(bs, outs)):
+        args.seg_B[i], args.seg_C[i], args.seg_ldb[i], args.seg_ldc[i], args.seg_N[i] = b.data_ptr(), y.data_ptr(), b.stride(0), y.stride(0), b.shape[0]
+    args.err = err_word(a.device).data_ptr()
+    args.stream = cur_stream(a.device).value
+    check(lib().tyr_gemm_bf16(ctypes.byref(args)), "tyr_gemm_bf16(many)")
+    return outs
 
 
 class _LinearFn(torch.autograd.Function):
