@@ -441,9 +441,10 @@ __device__ __forceinline__ void mma_op(float (&c)[4], const Tf32Op<EXACT> (&a)[4
 __device__ __forceinline__ void store_pair(__nv_bfloat16* p, float x, float y) { *reinterpret_cast<uint32_t*>(p) = pack_bf16x2(x, y); }
 __device__ __forceinline__ void store_pair(float* p, float x, float y) { *reinterpret_cast<float2*>(p) = make_float2(x, y); }
 
-// `dv` columns of the state and the output; `u` has rows of dvp = dv rounded up to 64 columns.  `glast` holds the chunk's decay of the
+// A CTA owns 8 NT columns of one head's state and runs its chunks one after the other: bound by the chain of products of a chunk, so where heads are few
+// the columns are cut finer to occupy the chip (see the launch).  `dv` columns of the state and the output; `u` has rows of dvp = dv rounded up to 64 columns.  `glast` holds the chunk's decay of the
 // state: one number (gl_ld 1) or one per key channel (gl_ld GC_DK).
-template <bool EXACT, typename OutT>
+template <bool EXACT, typename OutT, int NT>
 __global__ void __launch_bounds__(256, 1)
 gdr_chunk_scan_kernel(const float* __restrict__ u, const float* __restrict__ w, const float* __restrict__ qg,
                       const float* __restrict__ kd, const float* __restrict__ intra, const float* __restrict__ glast, int gl_ld,
@@ -453,7 +454,8 @@ gdr_chunk_scan_kernel(const float* __restrict__ u, const float* __restrict__ w, 
   extern __shared__ __align__(16) uint8_t gdr_smem_raw[];
   GdrChunkSmem& sm = *reinterpret_cast<GdrChunkSmem*>(gdr_smem_raw);
   const int bh = blockIdx.y;
-  const int col0 = blockIdx.x * GC_DVS;
+  const int col0 = blockIdx.x * (8 * NT);
+  pdl_entry();
   const int grp = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const long long chunk_k = static_cast<long long>(GC_C) * GC_DK;      // floats per chunk of w / qg / kd
@@ -465,14 +467,14 @@ gdr_chunk_scan_kernel(const float* __restrict__ u, const float* __restrict__ w, 
   // output rows go straight to the [B, S, Hv, dv] layout of the layer (rows past the sequence end are dropped)
   OutT* o_p = out + (static_cast<long long>(bh / Hv) * seq * Hv + (bh % Hv)) * dv + col0;
 
-  // group 0: state rows [32 warp, 32 warp + 32) x 64 columns as two m-tiles x eight n-tiles of accumulators
-  float S[2][8][4];
+  // group 0: state rows [32 warp, 32 warp + 32) x 8 NT columns as two m-tiles x NT n-tiles of accumulators
+  float S[2][NT][4];
   if (grp == 0) {
     const float* si = state_in ? state_in + (static_cast<long long>(bh) * dk) * dv + col0 : nullptr;
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int h2 = 0; h2 < 2; ++h2) {
           const int r = warp * 32 + mt * 16 + g + h2 * 8, c = nt * 8 + 2 * t;
@@ -495,31 +497,37 @@ gdr_chunk_scan_kernel(const float* __restrict__ u, const float* __restrict__ w, 
     cp_async_wait<1>();            // w_i, qg_i landed (this thread's copies); the barrier publishes everyone's and S
     __syncthreads();
     // ---- group 0: X = w_i S, group 1: X = qg_i S; warp rows [16 warp, +16), K = dk
-    float X[8][4];
+    float X[NT][4];
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
+    for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
       for (int e = 0; e < 4; ++e) X[nt][e] = 0.f;
+    // u_i is needed after the first products only: its latency passes meanwhile
+    float2 uu[NT][2];
+    if (grp == 0) {
+      const float* ui = u_p + static_cast<long long>(i) * GC_C * dvp;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int h2 = 0; h2 < 2; ++h2) uu[nt][h2] = *reinterpret_cast<const float2*>(ui + static_cast<long long>(ar + h2 * 8) * dvp + nt * 8 + 2 * t);
+    }
     const float* A = grp == 0 ? sm.w : sm.q;
 #pragma unroll 2
     for (int kk = 0; kk < GC_DK / 8; ++kk) {
       const int kc = kk * 8 + t;
       const Op a[4] = {Op(A[ar * GC_LDW + kc]), Op(A[(ar + 8) * GC_LDW + kc]), Op(A[ar * GC_LDW + kc + 4]), Op(A[(ar + 8) * GC_LDW + kc + 4])};
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
+      for (int nt = 0; nt < NT; ++nt)
         mma_op<EXACT>(X[nt], a, Op(sm.s[kc * GC_LDS + nt * 8 + g]), Op(sm.s[(kc + 4) * GC_LDS + nt * 8 + g]));
     }
     // ---- v_new = u_i - X  -> shared memory (B operand of the next two products)
     if (grp == 0) {
-      const float* ui = u_p + static_cast<long long>(i) * GC_C * dvp;
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2) {
-          const int r = ar + h2 * 8, c = nt * 8 + 2 * t;
-          const float2 uu = *reinterpret_cast<const float2*>(ui + static_cast<long long>(r) * dvp + c);
-          *reinterpret_cast<float2*>(&sm.v[r * GC_LDS + c]) = make_float2(uu.x - X[nt][2 * h2], uu.y - X[nt][2 * h2 + 1]);
-        }
+        for (int h2 = 0; h2 < 2; ++h2)
+          *reinterpret_cast<float2*>(&sm.v[(ar + h2 * 8) * GC_LDS + nt * 8 + 2 * t]) =
+              make_float2(uu[nt][h2].x - X[nt][2 * h2], uu[nt][h2].y - X[nt][2 * h2 + 1]);
     }
     cp_async_wait<0>();            // kd_i, intra_i
     __syncthreads();               // v_new complete; every warp is done with w, qg and the old S in shared memory
@@ -536,7 +544,7 @@ gdr_chunk_scan_kernel(const float* __restrict__ u, const float* __restrict__ w, 
         const Op a[4] = {Op(sm.intra[ar * GC_LDI + kc]), Op(sm.intra[(ar + 8) * GC_LDI + kc]), Op(sm.intra[ar * GC_LDI + kc + 4]),
                          Op(sm.intra[(ar + 8) * GC_LDI + kc + 4])};
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
+        for (int nt = 0; nt < NT; ++nt)
           mma_op<EXACT>(X[nt], a, Op(sm.v[kc * GC_LDS + nt * 8 + g]), Op(sm.v[(kc + 4) * GC_LDS + nt * 8 + g]));
       }
 #pragma unroll
@@ -545,7 +553,7 @@ gdr_chunk_scan_kernel(const float* __restrict__ u, const float* __restrict__ w, 
         if (tok < seq) {
           OutT* oi = o_p + static_cast<long long>(tok) * Hv * dv;
 #pragma unroll
-          for (int nt = 0; nt < 8; ++nt)
+          for (int nt = 0; nt < NT; ++nt)
             if (col0 + nt * 8 < dv) store_pair(oi + nt * 8 + 2 * t, X[nt][2 * h2], X[nt][2 * h2 + 1]);
         }
       }
@@ -558,7 +566,7 @@ gdr_chunk_scan_kernel(const float* __restrict__ u, const float* __restrict__ w, 
         for (int h2 = 0; h2 < 2; ++h2) {
           const float e = gl[gl_ld == 1 ? 0 : warp * 32 + mt * 16 + g + h2 * 8];
 #pragma unroll
-          for (int nt = 0; nt < 8; ++nt) {
+          for (int nt = 0; nt < NT; ++nt) {
             S[mt][nt][2 * h2] *= e;
             S[mt][nt][2 * h2 + 1] *= e;
           }
@@ -570,7 +578,7 @@ gdr_chunk_scan_kernel(const float* __restrict__ u, const float* __restrict__ w, 
         const Op a0[4] = {Op(k0[0]), Op(k0[8]), Op(k4[0]), Op(k4[8])};
         const Op a1[4] = {Op(k0[16]), Op(k0[24]), Op(k4[16]), Op(k4[24])};
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
+        for (int nt = 0; nt < NT; ++nt) {
           const Op b0(sm.v[kc * GC_LDS + nt * 8 + g]), b1(sm.v[(kc + 4) * GC_LDS + nt * 8 + g]);
           mma_op<EXACT>(S[0][nt], a0, b0, b1);
           mma_op<EXACT>(S[1][nt], a1, b0, b1);
@@ -580,7 +588,7 @@ gdr_chunk_scan_kernel(const float* __restrict__ u, const float* __restrict__ w, 
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
           for (int h2 = 0; h2 < 2; ++h2)
             *reinterpret_cast<float2*>(&sm.s[(warp * 32 + mt * 16 + g + h2 * 8) * GC_LDS + nt * 8 + 2 * t]) =
@@ -593,7 +601,7 @@ gdr_chunk_scan_kernel(const float* __restrict__ u, const float* __restrict__ w, 
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int h2 = 0; h2 < 2; ++h2) {
           const int r = warp * 32 + mt * 16 + g + h2 * 8, c = nt * 8 + 2 * t;
@@ -607,28 +615,39 @@ gdr_chunk_scan_kernel(const float* __restrict__ u, const float* __restrict__ w, 
 // Chunked prefill: everything that is local to one chunk, in one launch per layer.
 //
 // One CTA per (chunk of 64 tokens, batch, value head), 256 threads:
-//   1. q, k rows -> fp32 shared memory, L2-normalised (q also scaled by dk^-1/2); gc = inclusive cumulative sum of g.
-//   2. k k^T and q k^T (64 x 64, K = 128) on tensor cores with the 3-term TF32 split (hi*hi + hi*lo + lo*hi, close to fp32:
-//      the first matrix feeds a triangular solve), then A = beta_i (k_i.k_j) exp(gc_i - gc_j) for j < i and
-//      intra = (q_i.k_j) exp(gc_i - gc_j) for j <= i.
+//   1. q, k, v rows -> shared memory as they are (bf16); the factors that give q and k unit length (q also dk^-1/2);
+//      gc = inclusive cumulative sum of g.
+//   2. k k^T and q k^T (64 x 64, K = 128) of the rows as they are: products of bf16 numbers are exact in the tensor cores' fp32 sums, and the
+//      lengths are taken out of the results, so one m16n8k16 product does what a 3-term TF32 split of normalised rows needed six m16n8k8 for.
+//      Then A = beta_i (k_i.k_j) exp(gc_i - gc_j) for j < i and intra = (q_i.k_j) exp(gc_i - gc_j) for j <= i.
 //   3. (I + A) X = [v beta | k beta exp(gc)] by forward substitution in fp32: one thread per right-hand-side column keeps
 //      its 64 unknowns in registers; the rows of A are broadcast from shared memory.  X = [u | w].
 //   4. qg = q exp(gc), kd = k exp(gc_last - gc), glast = exp(gc_last).
+// Bound by the substitution's 2016 dependent multiply-adds a thread and the 144 KB of fp32 that a CTA writes.  4 x 2048 tokens, 48 heads: 915 us with the split
+// products on fp32 rows, 608 us now.
 // The reference builds the same quantities as a graph of library ops over all chunks with a 63-step loop for the solve
 // (cc/src/tyr_qwen35.cpp:21-88).  Rows past the sequence end behave as g = 0, beta = 0, q = k = v = 0.  Key sizes below 128 are
 // padded with zero channels, which change neither norms nor products.
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int GP_LDA = GC_C + 4;
+constexpr int GP_LDK = GC_DK + 8;        // 272-byte rows: the fragments' 32-bit loads (8 rows x 4 words) fall on 32 banks
 
 struct GdrPrepSmem {
-  float k[GC_C * GC_LDW];
-  float q[GC_C * GC_LDW];
+  __nv_bfloat16 k[GC_C * GP_LDK];
+  __nv_bfloat16 q[GC_C * GP_LDK];
+  __nv_bfloat16 v[GC_C * 128];   // dv <= 128
   float a[GC_C * GP_LDA];
   float gc[GC_C];
   float beta[GC_C];
   float eg[GC_C];        // exp(gc_i)
-  __nv_bfloat16 v[GC_C * 128];   // the chunk's value rows (dv <= 128), staged with 16-byte loads
+  float qn[GC_C], kn[GC_C];      // 1 / |q_i| / sqrt(dk), 1 / |k_i|
 };
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
 
 struct GdrPrepArgs {
   const __nv_bfloat16 *q, *k, *v;
@@ -652,8 +671,10 @@ __global__ void __launch_bounds__(256, 2) gdr_chunk_prepare_kernel(GdrPrepArgs a
   const int b = bh / a.Hv, hv = bh % a.Hv, hk = hv / (a.Hv / a.Hk);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row0 = c * GC_C;
+  pdl_entry();
   const int len = a.lens ? min(a.lens[b], a.S) : a.S;
-  // ---- 1. stage q, k (fp32), g, beta
+  // ---- 1. stage q, k, v, g, beta
+#pragma unroll
   for (int i = tid; i < GC_C * (GC_DK / 8); i += 256) {
     const int r = i / (GC_DK / 8), d = (i % (GC_DK / 8)) * 8;
     const int tok = row0 + r;
@@ -662,13 +683,8 @@ __global__ void __launch_bounds__(256, 2) gdr_chunk_prepare_kernel(GdrPrepArgs a
       uq = *reinterpret_cast<const uint4*>(a.q + b * a.q_sb + static_cast<long long>(tok) * a.q_ss + hk * a.q_sh + d);
       uk = *reinterpret_cast<const uint4*>(a.k + b * a.k_sb + static_cast<long long>(tok) * a.k_ss + hk * a.k_sh + d);
     }
-    const uint32_t qq[4] = {uq.x, uq.y, uq.z, uq.w}, kk[4] = {uk.x, uk.y, uk.z, uk.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 fq = unpack_bf16x2(qq[e]), fk = unpack_bf16x2(kk[e]);
-      sm.q[r * GC_LDW + d + 2 * e] = fq.x; sm.q[r * GC_LDW + d + 2 * e + 1] = fq.y;
-      sm.k[r * GC_LDW + d + 2 * e] = fk.x; sm.k[r * GC_LDW + d + 2 * e + 1] = fk.y;
-    }
+    *reinterpret_cast<uint4*>(&sm.q[r * GP_LDK + d]) = uq;
+    *reinterpret_cast<uint4*>(&sm.k[r * GP_LDK + d]) = uk;
   }
   for (int i = tid; i < GC_C * (a.dvp / 8); i += 256) {
     const int r = i / (a.dvp / 8), d = (i % (a.dvp / 8)) * 8;
@@ -697,54 +713,48 @@ __global__ void __launch_bounds__(256, 2) gdr_chunk_prepare_kernel(GdrPrepArgs a
     sm.gc[2 * lane] = base + x0;
     sm.gc[2 * lane + 1] = base + x0 + x1;
   }
-  // L2 normalisation: 4 threads per row
+  // lengths: 4 threads per row, 32 channels each
   {
     const int r = tid >> 2, part = tid & 3;
     float sq = 0.f, sk = 0.f;
-    for (int d = part; d < GC_DK; d += 4) {            // bank (4 r + part + 4 i): the 32 lanes hit 32 banks
-      const float x = sm.q[r * GC_LDW + d], y = sm.k[r * GC_LDW + d];
-      sq += x * x; sk += y * y;
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+      const uint4 uq = *reinterpret_cast<const uint4*>(&sm.q[r * GP_LDK + part * 8 + d * 32]), uk = *reinterpret_cast<const uint4*>(&sm.k[r * GP_LDK + part * 8 + d * 32]);
+      const uint32_t qq[4] = {uq.x, uq.y, uq.z, uq.w}, kk[4] = {uk.x, uk.y, uk.z, uk.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 fq = unpack_bf16x2(qq[e]), fk = unpack_bf16x2(kk[e]);
+        sq += fq.x * fq.x + fq.y * fq.y;
+        sk += fk.x * fk.x + fk.y * fk.y;
+      }
     }
     sq += __shfl_xor_sync(0xffffffffu, sq, 1); sq += __shfl_xor_sync(0xffffffffu, sq, 2);
     sk += __shfl_xor_sync(0xffffffffu, sk, 1); sk += __shfl_xor_sync(0xffffffffu, sk, 2);
-    const float qn = rsqrtf(sq + 1e-6f) * rsqrtf(static_cast<float>(a.dk)), kn = rsqrtf(sk + 1e-6f);
-    for (int d = part; d < GC_DK; d += 4) {
-      sm.q[r * GC_LDW + d] *= qn;
-      sm.k[r * GC_LDW + d] *= kn;
+    if (part == 0) {
+      sm.qn[r] = rsqrtf(sq + 1e-6f) * rsqrtf(static_cast<float>(a.dk));
+      sm.kn[r] = rsqrtf(sk + 1e-6f);
     }
   }
   __syncthreads();
   if (tid < GC_C) sm.eg[tid] = __expf(sm.gc[tid]);
-  // ---- 2. warps 0-3: k k^T strips, warps 4-7: q k^T strips (16 rows each), 3-term TF32
+  // ---- 2. warps 0-3: k k^T strips, warps 4-7: q k^T strips (16 rows each)
   {
     const int g8 = lane >> 2, t = lane & 3;
     const bool is_q = warp >= 4;
-    const float* A = is_q ? sm.q : sm.k;
+    const __nv_bfloat16* A = is_q ? sm.q : sm.k;
     const int ar = (warp & 3) * 16 + g8;
     float acc[8][4];
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[nt][e] = 0.f;
-#pragma unroll 2
-    for (int kk = 0; kk < GC_DK / 8; ++kk) {
-      const int kc = kk * 8 + t;
-      const float af[4] = {A[ar * GC_LDW + kc], A[(ar + 8) * GC_LDW + kc], A[ar * GC_LDW + kc + 4], A[(ar + 8) * GC_LDW + kc + 4]};
-      uint32_t ah[4], al[4];
+    auto word = [&](const __nv_bfloat16* m, int r, int c2) { return *reinterpret_cast<const uint32_t*>(m + r * GP_LDK + c2); };
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        ah[e] = to_tf32(af[e]);
-        al[e] = to_tf32(af[e] - __uint_as_float(ah[e]));
-      }
+    for (int kk = 0; kk < GC_DK / 16; ++kk) {
+      const int kc = kk * 16 + 2 * t;
+      const uint32_t a0 = word(A, ar, kc), a1 = word(A, ar + 8, kc), a2 = word(A, ar, kc + 8), a3 = word(A, ar + 8, kc + 8);
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        const float b0f = sm.k[(nt * 8 + g8) * GC_LDW + kc], b1f = sm.k[(nt * 8 + g8) * GC_LDW + kc + 4];
-        const uint32_t b0h = to_tf32(b0f), b1h = to_tf32(b1f);
-        const uint32_t b0l = to_tf32(b0f - __uint_as_float(b0h)), b1l = to_tf32(b1f - __uint_as_float(b1h));
-        mma_tf32(acc[nt], al[0], al[1], al[2], al[3], b0h, b1h);
-        mma_tf32(acc[nt], ah[0], ah[1], ah[2], ah[3], b0l, b1l);
-        mma_tf32(acc[nt], ah[0], ah[1], ah[2], ah[3], b0h, b1h);
-      }
+      for (int nt = 0; nt < 8; ++nt) mma_bf16(acc[nt], a0, a1, a2, a3, word(sm.k, nt * 8 + g8, kc), word(sm.k, nt * 8 + g8, kc + 8));
     }
     __syncthreads();          // eg ready (written above by other threads)
     float* intra_o = a.intra + (static_cast<long long>(bh) * a.n + c) * GC_C * GC_C;
@@ -753,8 +763,8 @@ __global__ void __launch_bounds__(256, 2) gdr_chunk_prepare_kernel(GdrPrepArgs a
 #pragma unroll
       for (int h2 = 0; h2 < 2; ++h2) {
         const int i = ar + h2 * 8, j = nt * 8 + 2 * t;
-        const float gi = sm.gc[i];
-        float v0 = acc[nt][2 * h2] * __expf(gi - sm.gc[j]), v1 = acc[nt][2 * h2 + 1] * __expf(gi - sm.gc[j + 1]);
+        const float gi = sm.gc[i], ni = is_q ? sm.qn[i] : sm.kn[i];
+        float v0 = acc[nt][2 * h2] * (ni * sm.kn[j]) * __expf(gi - sm.gc[j]), v1 = acc[nt][2 * h2 + 1] * (ni * sm.kn[j + 1]) * __expf(gi - sm.gc[j + 1]);
         if (is_q) {
           v0 = j <= i ? v0 : 0.f;
           v1 = j + 1 <= i ? v1 : 0.f;
@@ -779,7 +789,7 @@ __global__ void __launch_bounds__(256, 2) gdr_chunk_prepare_kernel(GdrPrepArgs a
         for (int i = 0; i < GC_C; ++i) x[i] = __bfloat162float(sm.v[i * a.dvp + col]) * sm.beta[i];
       } else {
 #pragma unroll
-        for (int i = 0; i < GC_C; ++i) x[i] = sm.k[i * GC_LDW + (col - a.dvp)] * sm.beta[i] * sm.eg[i];
+        for (int i = 0; i < GC_C; ++i) x[i] = __bfloat162float(sm.k[i * GP_LDK + (col - a.dvp)]) * (sm.kn[i] * sm.beta[i] * sm.eg[i]);
       }
 #pragma unroll
       for (int i = 1; i < GC_C; ++i) {
@@ -808,11 +818,11 @@ __global__ void __launch_bounds__(256, 2) gdr_chunk_prepare_kernel(GdrPrepArgs a
     float* kd_o = a.kd + (static_cast<long long>(bh) * a.n + c) * GC_C * GC_DK;
     for (int i = tid; i < GC_C * (GC_DK / 4); i += 256) {
       const int r = i / (GC_DK / 4), d = (i % (GC_DK / 4)) * 4;
-      const float eq = sm.eg[r], ek = __expf(g_last - sm.gc[r]);
-      const float4 fq = *reinterpret_cast<const float4*>(&sm.q[r * GC_LDW + d]);
-      const float4 fk = *reinterpret_cast<const float4*>(&sm.k[r * GC_LDW + d]);
-      *reinterpret_cast<float4*>(qg_o + r * GC_DK + d) = make_float4(fq.x * eq, fq.y * eq, fq.z * eq, fq.w * eq);
-      *reinterpret_cast<float4*>(kd_o + r * GC_DK + d) = make_float4(fk.x * ek, fk.y * ek, fk.z * ek, fk.w * ek);
+      const float eq = sm.qn[r] * sm.eg[r], ek = sm.kn[r] * __expf(g_last - sm.gc[r]);
+      const uint2 uq = *reinterpret_cast<const uint2*>(&sm.q[r * GP_LDK + d]), uk = *reinterpret_cast<const uint2*>(&sm.k[r * GP_LDK + d]);
+      const float2 q0 = unpack_bf16x2(uq.x), q1 = unpack_bf16x2(uq.y), k0 = unpack_bf16x2(uk.x), k1 = unpack_bf16x2(uk.y);
+      *reinterpret_cast<float4*>(qg_o + r * GC_DK + d) = make_float4(q0.x * eq, q0.y * eq, q1.x * eq, q1.y * eq);
+      *reinterpret_cast<float4*>(kd_o + r * GC_DK + d) = make_float4(k0.x * ek, k0.y * ek, k1.x * ek, k1.y * ek);
     }
     if (tid == 0) a.glast[static_cast<long long>(bh) * a.n + c] = __expf(g_last);
   }
@@ -1240,8 +1250,7 @@ extern "C" TYR_EXPORT int tyr_gdr_chunk_prepare(const void* q, const void* k, co
     if (e != cudaSuccess) return 1000 + (int)e;
     configured = true;
   }
-  gdr_chunk_prepare_kernel<<<dim3(a.n, B * Hv), 256, smem, reinterpret_cast<cudaStream_t>(stream)>>>(a);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_dependent(gdr_chunk_prepare_kernel, dim3(a.n, B * Hv), dim3(256), smem, reinterpret_cast<cudaStream_t>(stream), a));
 }
 
 // Chunk-local quantities with a decay per key channel: a_raw bf16 [B * S, .] (channel hv * dk + d) and b_raw bf16 (channel hv) with row
@@ -1302,23 +1311,35 @@ extern "C" TYR_EXPORT int tyr_gdr_chunk_scan(const float* u, const float* w, con
   int cfg_dev = 0;
   if (cudaGetDevice(&cfg_dev) != cudaSuccess || cfg_dev < 0 || cfg_dev >= 64) cfg_dev = 0;
   bool& configured = configured_dev[cfg_dev];
+#define TYR_SCAN_ALL(X) X(8) X(4) X(2)
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gdr_chunk_scan_kernel<false, __nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gdr_chunk_scan_kernel<true, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaSuccess;
+#define TYR_SCAN_SET(nt)                                                                                                                          \
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(gdr_chunk_scan_kernel<false, __nv_bfloat16, nt>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(gdr_chunk_scan_kernel<true, float, nt>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    TYR_SCAN_ALL(TYR_SCAN_SET)
+#undef TYR_SCAN_SET
     if (e != cudaSuccess) return 1000 + (int)e;
     configured = true;
   }
-  const int slices = (dv + GC_DVS - 1) / GC_DVS, dvp = slices * GC_DVS;
-  const dim3 grid(slices, BH);
+  // 64 columns a CTA when that fills the chip (a chunk's w, q and k rows are then staged by two CTAs), else 32 or 16: 333 tokens of 16 heads
+  // took 34.5 us on 32 CTAs and take 20.4 on 128.
+  const int dvp = (dv + GC_DVS - 1) / GC_DVS * GC_DVS;
+  int nt = 8;
+  while (nt > 2 && static_cast<long long>((dv + 8 * nt - 1) / (8 * nt)) * BH < 148) nt >>= 1;
+  const dim3 grid((dv + 8 * nt - 1) / (8 * nt), BH);
   const int gl_ld = channel ? GC_DK : 1;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (exact)
-    gdr_chunk_scan_kernel<true, float><<<grid, 256, smem, st>>>(u, w, qg, kd, intra, glast, gl_ld, state_in, state_out, reinterpret_cast<float*>(out),
-                                                                n, dk, dv, dvp, S, Hv);
-  else
-    gdr_chunk_scan_kernel<false, __nv_bfloat16><<<grid, 256, smem, st>>>(u, w, qg, kd, intra, glast, gl_ld, state_in, state_out,
-                                                                         reinterpret_cast<__nv_bfloat16*>(out), n, dk, dv, dvp, S, Hv);
-  return static_cast<int>(cudaGetLastError());
+#define TYR_SCAN_RUN(w8)                                                                                                                          \
+  if (nt == w8)                                                                                                                                   \
+    return static_cast<int>(exact ? launch_dependent(gdr_chunk_scan_kernel<true, float, w8>, grid, dim3(256), smem, st, u, w, qg, kd, intra, glast, gl_ld, \
+                                                     state_in, state_out, reinterpret_cast<float*>(out), n, dk, dv, dvp, S, Hv)                    \
+                                  : launch_dependent(gdr_chunk_scan_kernel<false, __nv_bfloat16, w8>, grid, dim3(256), smem, st, u, w, qg, kd, intra, glast, \
+                                                     gl_ld, state_in, state_out, reinterpret_cast<__nv_bfloat16*>(out), n, dk, dv, dvp, S, Hv));
+  TYR_SCAN_ALL(TYR_SCAN_RUN)
+#undef TYR_SCAN_RUN
+#undef TYR_SCAN_ALL
+  return -3;
 }
 
 extern "C" TYR_EXPORT int tyr_gdr_decode_norm(const void* q, const void* k, const void* v, const float* g, const float* beta,
