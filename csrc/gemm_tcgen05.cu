@@ -40,7 +40,7 @@ struct GemmParams {
   long long ldc, ldaux, sC, sAux;
   float alpha, beta;
   int act;        // 0 none, 1 relu(x)^2, 2 relu, 3 acc * 2*sqrt(aux), 4 SwiGLU of column halves, 5 GELU(tanh)-gate of column halves,
-                  // 6 xIELU, 7 SiLU, 8 clamped SwiGLU of column halves (limit alpha, slope beta), 9 tanh-GELU times aux
+                  // 6 xIELU, 7 SiLU, 8 clamped SwiGLU of column halves (limit alpha, slope beta), 9 tanh-GELU times aux, 10 aux + gate * acc
   int out_mode;   // 0 bf16 store, 1 fp32 store, 2 fp32 atomic add (stream-K)
   // out_mode 2 only.  > 0: the first (tiles / grid) * grid tiles are reduced whole, one per CTA and round, and every
   // remaining tile is cut into sk_slabs equal k ranges that are dealt round-robin, slab by slab.  All CTAs then sweep the
@@ -82,6 +82,9 @@ struct GemmParams {
   // gated products whose gate and up rows are two matrices: B is the gate matrix, TmapPeers m[0] the up matrix, and a tile takes
   // BN / 2 rows of each (N counts both, ragged widths allowed).
   int split_b;
+  const __nv_bfloat16* gate;      // act 10: a gate per column for every gate_rows rows, sets ld_gate elements apart
+  long long ld_gate;
+  int gate_rows;
   void* peer_c[8];
   __nv_bfloat16* gather_buf;
   int* tile_ready;
@@ -121,10 +124,12 @@ __device__ __forceinline__ float apply_act(float v, int act) {
 //   ACT 3: v = alpha * acc * 2 * sqrt(aux)     (gradient of y = relu(z)^2 given aux = y)
 //   ACT 7: alpha * silu(acc) (+ ...)
 //   ACT 9: gelu(acc) * aux
+//   ACT 10: aux + gate * acc (`gt`: the chunk's gates)
 //   ACT 6: xIELU of acc: alpha z^2 + z / 2 above zero, beta (e^z - 1 - z) + z / 2 below (no aux)
 template <int ACT>
 __device__ __forceinline__ void epi_chunk(const uint32_t (&r)[32], const float (&ax)[32], bool use_aux, float alpha,
                                           float beta, float (&v)[32]) {
+  static_assert(ACT != 10, "takes a gate per column: see the epilogue");
   if constexpr (ACT == 3) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = alpha * __uint_as_float(r[j]) * 2.f * sqrtf(fmaxf(ax[j], 0.f));
@@ -659,7 +664,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
         }
         float v[32];
         const bool full = (col + 32 <= N);
-        const bool use_aux = p.aux != nullptr && (p.beta != 0.f || p.act == 3 || p.act == 9) && row_ok;
+        const bool use_aux = p.aux != nullptr && (p.beta != 0.f || p.act == 3 || p.act == 9 || p.act == 10) && row_ok;
         float ax[32];
         if (use_aux) {
           const __nv_bfloat16* axp = p.aux + x_off + col;
@@ -686,6 +691,22 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
         else if (p.act == 7) epi_chunk<7>(r, ax, use_aux, p.alpha, p.beta, v);
         else if (p.act == 9) epi_chunk<9>(r, ax, use_aux, p.alpha, p.beta, v);
         else if (p.act == 6) epi_chunk<6>(r, ax, use_aux, p.alpha, p.beta, v);
+        else if (p.act == 10) {
+          // the lanes of a warp (rows) mostly share their gates: the loads are broadcasts
+          const __nv_bfloat16* gp = p.gate + (row_ok ? row / p.gate_rows : 0) * p.ld_gate + col;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            uint4 u = make_uint4(0u, 0u, 0u, 0u);
+            if (col + q * 8 < N) u = *reinterpret_cast<const uint4*>(gp + q * 8);        // N is a multiple of 8
+            const uint32_t uu[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 g2 = unpack_bf16x2(uu[e]);
+              v[q * 8 + 2 * e] = fmaf(g2.x, __uint_as_float(r[q * 8 + 2 * e]), ax[q * 8 + 2 * e]);
+              v[q * 8 + 2 * e + 1] = fmaf(g2.y, __uint_as_float(r[q * 8 + 2 * e + 1]), ax[q * 8 + 2 * e + 1]);
+            }
+          }
+        }
         else epi_chunk<3>(r, ax, use_aux, p.alpha, p.beta, v);
         if (tma_out) {
           uint8_t* st = s.out_stage[epi][n_stores % EPI_BUFS] + lane * 128;
@@ -845,6 +866,9 @@ struct TyrGemmArgs {
   void* seg_C[4];
   long long seg_ldb[4], seg_ldc[4];
   int seg_N[4];
+  const void* gate;                 // act 10: bf16 [ceil(M / gate_rows), N], rows ld_gate apart
+  long long ld_gate;
+  int gate_rows;
 };
 
 }  // extern "C"
@@ -915,6 +939,9 @@ static int launch_gemm(const TyrGemmArgs& a, const CUtensorMap& tmA, const CUten
   p.group_offsets = a.group_offsets;
   p.group_tiles = a.group_tiles;
   p.segs = a.segs;
+  p.gate = reinterpret_cast<const __nv_bfloat16*>(a.gate);
+  p.ld_gate = a.ld_gate;
+  p.gate_rows = a.gate_rows;
   p.split_b = a.B2 != nullptr ? 1 : 0;
   int seg_tiles = 0, seg_cols = 0;
   for (int i = 0; i < a.segs; ++i) {
@@ -1088,6 +1115,9 @@ static int gemm_impl(const TyrGemmArgs& a, const TyrTpArgs* tpa) {
     for (int i = 0; i < a.segs; ++i)
       if (a.seg_N[i] <= 0 || (a.seg_ldb[i] & 7) || (a.seg_ldc[i] & 7) || (reinterpret_cast<uintptr_t>(a.seg_B[i]) & 15) || (reinterpret_cast<uintptr_t>(a.seg_C[i]) & 15)) return -15;
   }
+  if (a.act == 10 && (a.aux == nullptr || a.gate == nullptr || a.gate_rows <= 0 || (a.ld_gate & 7) || (reinterpret_cast<uintptr_t>(a.gate) & 15) || (a.N & 7) ||
+                      a.batch != 1 || a.out_mode == 2 || a.group_offsets != nullptr || tpa != nullptr))
+    return -17;
   if (a.B2 != nullptr && (!gated || tpa != nullptr || a.group_offsets != nullptr || a.b_mn || a.batch != 1 || (a.N & 15) || (reinterpret_cast<uintptr_t>(a.B2) & 15))) return -16;
   // tiles of other sizes: products whose tiles are handed out whole
   const bool free_tile = tpa == nullptr && a.group_offsets == nullptr && a.out_mode != 2 && (!gated || a.B2 != nullptr);

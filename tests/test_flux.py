@@ -194,3 +194,21 @@ def _to_cuda(m):
             return [conv(v) for v in o]
         return o
     return conv(m)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,St,Si,axes", [(1, 77, 256, (16, 16, 16, 16)), (2, 5, 0, (1, 2, 3, 10)), (3, 0, 33, (8, 8, 24, 24))])
+def test_rope_tables_and_timestep_embedding(B, St, Si, axes):
+    """Against fp64 angles: fp32 angles of up to 300 rad and one exponential are off by 300 * 2^-22."""
+    from tyr_b200.ops import modulate as mod
+    g = torch.Generator().manual_seed(St + Si)
+    txt, img = torch.randint(0, 300, (B, St, 4), generator=g).cuda(), torch.randint(0, 300, (B, Si, 4), generator=g).cuda()
+    assert mod.flux_rope_tables_supported(txt, img, axes)
+    cos, sin = mod.flux_rope_tables(txt, img, axes, 2000)
+    ids = torch.cat([txt, img], 1).double()
+    ang = torch.cat([ids[..., a, None] * 2000.0 ** -(torch.arange(n, device="cuda", dtype=torch.float64) / n) for a, n in enumerate(axes)], -1)
+    assert (cos.double() - ang.cos()).abs().max() < 1e-4 and (sin.double() - ang.sin()).abs().max() < 1e-4
+    t = torch.rand(B, generator=g).cuda()
+    e = FX.timestep_embedding(t, 2 * sum(axes) + 1).bfloat16()
+    got = mod.timestep_embedding_bf16(t, 2 * sum(axes) + 1, 10000.0, 1000.0)
+    assert (got.float() - e.float()).abs().max() <= 2.0 ** -7 and not got[:, -1].any()

@@ -760,3 +760,17 @@ def test_gated_gemm_of_two_matrices(rows, bn, M, N, K):
     y = gemm(x, wg, up=wu, act="swiglu", tile_rows=rows, bn=bn)
     ref = torch.nn.functional.silu(x.double() @ wg.double().T) * (x.double() @ wu.double().T)
     assert y.shape == ref.shape and ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all()
+
+
+@pytest.mark.parametrize("rows,bn", TILES + [(0, 0)])
+@pytest.mark.parametrize("sets,per,N,K", [(1, 7, 8, 64), (3, 111, 200, 136), (2, 256, 520, 1024)])
+def test_gemm_with_gated_addend(rows, bn, sets, per, N, K):
+    """aux + gate * (a b^T), rounded to bf16 once (2^-8 of the result), the fp32 sum before it off by 1e-5 of the largest."""
+    from tyr_b200.ops.gemm import gemm
+    g = torch.Generator(device="cuda").manual_seed(per + N)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    a, b, aux, gate = r(sets * per, K), r(N, K), r(sets * per, N), r(sets, 2 * N)[:, N:]
+    y = gemm(a, b, act="gated_add", aux=aux, gate=gate, tile_rows=rows, bn=bn)
+    acc = a.double() @ b.double().T
+    ref = aux.double() + gate.double().repeat_interleave(per, 0) * acc
+    assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * acc.abs().max() * gate.abs().max().double()).all()

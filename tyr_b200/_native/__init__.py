@@ -140,6 +140,7 @@ class GemmArgs(ctypes.Structure):
         ("err", c_void_p), ("stream", c_void_p), ("group_offsets", c_void_p), ("group_tiles", c_void_p),
         ("tile_rows", c_int), ("segs", c_int), ("B2", c_void_p),
         ("seg_B", c_void_p * 4), ("seg_C", c_void_p * 4), ("seg_ldb", c_ll * 4), ("seg_ldc", c_ll * 4), ("seg_N", c_int * 4),
+        ("gate", c_void_p), ("ld_gate", c_ll), ("gate_rows", c_int),
     ]
 
 

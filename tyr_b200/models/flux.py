@@ -17,10 +17,11 @@ import torch.nn.functional as F
 from ..io import safetensors as st
 from ..ops.attention import attention
 from ..ops import flash as _flash
-from ..ops.gemm import gemm as _gemm, interleave_gate_up
-from ..ops.modulate import flux_qk_post, flux_qk_post_supported, gate_residual, layernorm_modulate
+from ..ops.gemm import gemm as _gemm
+from ..ops.modulate import (flux_qk_post, flux_qk_post_supported, flux_rope_tables, flux_rope_tables_supported, gate_residual, layernorm_modulate,
+                            timestep_embedding_bf16)
 from ..ops.norm import rms_norm_weighted
-from .common import lin
+from .common import TCGEN05_MIN_ROWS, lin, lin_many
 
 
 @dataclass
@@ -201,11 +202,22 @@ def _fused_ok(cfg, x: torch.Tensor) -> bool:
             and cfg.mlp_hidden_dim % 128 == 0 and _flash.has_fwd() and flux_qk_post_supported(x, cfg.head_dim))
 
 
-def _swiglu_fused(x, w1, w2):
+def _swiglu_fused(x, w1):
     B, S, h = x.shape
     M = w1.shape[0] // 2
-    act = _gemm(x.reshape(B * S, h), w1[:M], up=w1[M:], act="swiglu")
-    return lin(act.reshape(B, S, -1), w2)
+    return _gemm(x.reshape(B * S, h), w1[:M], up=w1[M:], act="swiglu").reshape(B, S, -1)
+
+
+def _lin_gated_add(x, w, resid, gate):
+    """``resid + gate[:, None] * lin(x, w)``, in the product's epilogue where the tensor-core product applies (a 1024 x 1024 picture's pass: 30.6 -> 30.0 ms
+    with the pass over three tensors behind 40 products gone)."""
+    B, S, h = resid.shape
+    x2 = x.reshape(B * S, -1)
+    if not (B * S >= TCGEN05_MIN_ROWS and x2.is_contiguous() and resid.is_contiguous() and w.is_contiguous() and gate.stride(1) == 1 and gate.data_ptr() % 16 == 0
+            and (B == 1 or gate.stride(0) % 8 == 0) and h % 8 == 0 and w.shape[1] % 8 == 0 and x.dtype == w.dtype == resid.dtype == gate.dtype == torch.bfloat16
+            and x2.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and resid.data_ptr() % 16 == 0):
+        return gate_residual(resid, lin(x, w), gate)
+    return _gemm(x2, w, act="gated_add", aux=resid.view(B * S, h), gate=gate).view(B, S, h)
 
 
 def _double_block_fused(cfg, b: DoubleStreamBlock, img, txt, img_pe, txt_pe, mod_img, mod_txt):
@@ -223,12 +235,10 @@ def _double_block_fused(cfg, b: DoubleStreamBlock, img, txt, img_pe, txt_pe, mod
     attn, _ = _flash.flash_fwd_bthd(x5[:, :, 0], x5[:, :, 1], x5[:, :, 2], causal=False, window=None, scale=None,
                                     need_lse=False)
     attn = attn.view(B, St + Si, H * D)
-    img = gate_residual(img, lin(attn[:, St:].contiguous(), b.img_attn.proj), mod_img[:, 2])
-    txt = gate_residual(txt, lin(attn[:, :St].contiguous(), b.txt_attn.proj), mod_txt[:, 2])
-    img = gate_residual(img, _swiglu_fused(layernorm_modulate(img, mod_img[:, 4], mod_img[:, 3], EPS),
-                                           b.img_mlp.w1, b.img_mlp.w2), mod_img[:, 5])
-    txt = gate_residual(txt, _swiglu_fused(layernorm_modulate(txt, mod_txt[:, 4], mod_txt[:, 3], EPS),
-                                           b.txt_mlp.w1, b.txt_mlp.w2), mod_txt[:, 5])
+    img = _lin_gated_add(attn[:, St:].contiguous(), b.img_attn.proj, img, mod_img[:, 2])
+    txt = _lin_gated_add(attn[:, :St].contiguous(), b.txt_attn.proj, txt, mod_txt[:, 2])
+    img = _lin_gated_add(_swiglu_fused(layernorm_modulate(img, mod_img[:, 4], mod_img[:, 3], EPS), b.img_mlp.w1), b.img_mlp.w2, img, mod_img[:, 5])
+    txt = _lin_gated_add(_swiglu_fused(layernorm_modulate(txt, mod_txt[:, 4], mod_txt[:, 3], EPS), b.txt_mlp.w1), b.txt_mlp.w2, txt, mod_txt[:, 5])
     return img, txt
 
 
@@ -244,7 +254,7 @@ def _single_block_fused(cfg, b: SingleStreamBlock, x, pe, mod):
     x5 = qkv.view(B, S, 3, H, D)
     _flash.flash_fwd_bthd(x5[:, :, 0], x5[:, :, 1], x5[:, :, 2], causal=False, window=None, scale=None, need_lse=False,
                           out=cat.view(B, S, -1)[:, :, :H * D].unflatten(-1, (H, D)))
-    return gate_residual(x, lin(cat, b.linear2), mod[:, 2])
+    return _lin_gated_add(cat, b.linear2, x, mod[:, 2])
 
 
 def double_block_forward(cfg, b: DoubleStreamBlock, img, txt, img_pe, txt_pe, mod_img, mod_txt):
@@ -277,22 +287,30 @@ def forward(m: FluxModel, img, txt, timesteps, img_ids, txt_ids) -> torch.Tensor
     """img [B, Si, in_channels], txt [B, St, context], timesteps [B] -> predicted velocity [B, Si, in_channels]."""
     cfg = m.cfg
     h = cfg.hidden_size
-    vec = lin(F.silu(lin(timestep_embedding(timesteps, cfg.time_dim).to(m.dtype), m.time_in_layer)), m.time_out_layer)
-    mod_img = modulation(vec, m.double_stream_modulation_img, 6)
-    mod_txt = modulation(vec, m.double_stream_modulation_txt, 6)
-    mod_single = modulation(vec, m.single_stream_modulation, 3)
+    fused = _fused_ok(cfg, img)
+    if fused and timesteps.is_cuda and timesteps.dtype == torch.float32 and timesteps.dim() == 1:
+        emb = timestep_embedding_bf16(timesteps, cfg.time_dim, 10000.0, 1000.0)
+    else:
+        emb = timestep_embedding(timesteps, cfg.time_dim).to(m.dtype)
+    vec = F.silu(lin(F.silu(lin(emb, m.time_in_layer)), m.time_out_layer))
+    mod_img, mod_txt, mod_single, mod2 = lin_many(vec, (m.double_stream_modulation_img, m.double_stream_modulation_txt, m.single_stream_modulation,
+                                                        m.final_modulation))
+    mod_img, mod_txt, mod_single = (t.reshape(t.shape[0], -1, h) for t in (mod_img, mod_txt, mod_single))
     img = lin(img, m.img_in)
     txt = lin(txt, m.txt_in)
-    img_pe = rope_embed(img_ids, cfg.half_axes_dims, cfg.theta)
-    txt_pe = rope_embed(txt_ids, cfg.half_axes_dims, cfg.theta)
+    if fused and flux_rope_tables_supported(txt_ids, img_ids, cfg.half_axes_dims) and txt_ids.shape[:2] == txt.shape[:2] and img_ids.shape[:2] == img.shape[:2]:
+        pe = flux_rope_tables(txt_ids, img_ids, cfg.half_axes_dims, cfg.theta)
+        txt_pe, img_pe = tuple(t[:, :txt.shape[1]] for t in pe), tuple(t[:, txt.shape[1]:] for t in pe)
+    else:
+        img_pe = rope_embed(img_ids, cfg.half_axes_dims, cfg.theta)
+        txt_pe = rope_embed(txt_ids, cfg.half_axes_dims, cfg.theta)
+        pe = (torch.cat([txt_pe[0], img_pe[0]], 1), torch.cat([txt_pe[1], img_pe[1]], 1))
     for b in m.double_blocks:
         img, txt = double_block_forward(cfg, b, img, txt, img_pe, txt_pe, mod_img, mod_txt)
     x = torch.cat([txt, img], dim=1)
-    pe = (torch.cat([txt_pe[0], img_pe[0]], 1), torch.cat([txt_pe[1], img_pe[1]], 1))
     for b in m.single_blocks:
         x = single_block_forward(cfg, b, x, pe, mod_single)
     img_out = x[:, txt.shape[1]:].contiguous()
-    mod2 = lin(F.silu(vec), m.final_modulation)
     shift, scale = mod2[:, :h], mod2[:, h:]
     return lin(layernorm_modulate(img_out, scale, shift, EPS), m.final_linear)
 

@@ -9,7 +9,8 @@ Operand layouts (no transposes are ever materialised):
 * ``b_layout='MN'`` : ``b`` has shape ``[..., K, N]``
 
 ``out = alpha * act(A @ B) + beta * aux`` (``act='relu2_grad'``: ``alpha * (A @ B) * 2*sqrt(aux)``; ``act='xielu'``: xIELU of A @ B with
-factors ``alpha`` above zero and ``beta`` below, no ``aux``; ``act='gelu_mul'``: tanh-GELU of A @ B times ``aux``; the gated
+factors ``alpha`` above zero and ``beta`` below, no ``aux``; ``act='gelu_mul'``: tanh-GELU of A @ B times ``aux``;
+``act='gated_add'``: ``aux + gate[row // (M / sets)] * (A @ B)`` with ``gate`` [sets, N]; the gated
 ``act='clamped_swiglu'`` has limit ``alpha`` and slope ``beta``); ``out_dtype`` bf16 or fp32; ``accumulate=True`` adds
 into an existing fp32 ``out`` with an even stream-K split (used for weight gradients).
 
@@ -26,7 +27,7 @@ import torch
 from .._native import GemmArgs
 from ._common import check, cur_stream, err_word, lib
 
-_ACT = {None: 0, "none": 0, "relu2": 1, "relu": 2, "relu2_grad": 3, "swiglu": 4, "geglu": 5, "xielu": 6, "silu": 7, "clamped_swiglu": 8, "gelu_mul": 9}
+_ACT = {None: 0, "none": 0, "relu2": 1, "relu": 2, "relu2_grad": 3, "swiglu": 4, "geglu": 5, "xielu": 6, "silu": 7, "clamped_swiglu": 8, "gelu_mul": 9, "gated_add": 10}
 _GATED = ("swiglu", "geglu", "clamped_swiglu")
 
 
@@ -91,7 +92,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_layout: str = "K", b_layout: str
          out: Optional[torch.Tensor] = None, aux: Optional[torch.Tensor] = None,
          alpha: float = 1.0, beta: float = 0.0, act: Optional[str] = None,
          out_dtype: Optional[torch.dtype] = None, accumulate: bool = False,
-         bn: int = 0, sm_count: int = 0, tile_rows: int = 0, up: Optional[torch.Tensor] = None) -> torch.Tensor:
+         bn: int = 0, sm_count: int = 0, tile_rows: int = 0, up: Optional[torch.Tensor] = None,
+         gate: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``up`` (gated products): the up matrix, ``b`` being the gate matrix in its own row order.  ``bn`` (64, 128, 256) and ``tile_rows`` (128, 256)
     fix the output tile (0: by size)."""
     M, K, lda, batch_a, sA = _dims(a, a_layout, True)
@@ -106,6 +108,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_layout: str = "K", b_layout: str
     if batch_a not in (1, batch) or batch_b not in (1, batch):
         raise ValueError("gemm batch mismatch")
     gated = act in _GATED
+    if act == "gated_add" and (aux is None or gate is None or gate.dim() != 2 or gate.shape[1] != N or M % gate.shape[0] or gate.stride(1) != 1 or N % 8
+                               or a.dim() != 2 or accumulate or out_dtype == torch.float32):
+        raise ValueError("gated_add takes its addend as aux [M, N] and gates [sets, N] with N % 8 == 0 and M a multiple of the sets")
     if act == "gelu_mul" and aux is None:
         raise ValueError("gelu_mul takes its factor as aux")
     if gated:
@@ -132,7 +137,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_layout: str = "K", b_layout: str
             fn = torch.nn.functional.silu if act == "swiglu" else (lambda t: torch.nn.functional.gelu(t, approximate="tanh"))
             res = (clamped_swiglu(g, u, alpha, beta) if act == "clamped_swiglu" else fn(alpha * g) * (beta * u)).to(out_dtype)
             return res if out is None else out.copy_(res)
-        res = _reference(a, b, a_layout, b_layout, aux, alpha, beta, act, out_dtype)
+        if act == "gated_add":
+            acc = _reference(a, b, a_layout, b_layout, None, 1.0, 0.0, None, torch.float32)
+            res = (aux.float() + gate.float().repeat_interleave(M // gate.shape[0], 0) * acc).to(out_dtype)
+        else:
+            res = _reference(a, b, a_layout, b_layout, aux, alpha, beta, act, out_dtype)
         if out is not None:
             if accumulate:
                 out.add_(res.reshape(out.shape))
@@ -168,6 +177,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_layout: str = "K", b_layout: str
     args.bn, args.sm_count, args.tile_rows = bn, sm_count, tile_rows
     if up is not None:
         args.B2 = up.data_ptr()
+    if act == "gated_add":
+        if gate.dtype != torch.bfloat16:
+            raise TypeError("gated_add takes bf16 gates")
+        args.gate, args.ld_gate, args.gate_rows = gate.data_ptr(), gate.stride(0) if gate.shape[0] > 1 else 0, M // gate.shape[0]
     args.err = err_word(a.device).data_ptr()
     args.stream = cur_stream(a.device).value
     # batch==1 operands broadcast over the batch: the tensor map gets batch stride 0 only when
