@@ -42,6 +42,7 @@
 namespace tyr {
 
 constexpr int F4_BM = 128;
+constexpr int F4_STRIP = 32;   // rows of one load of activations
 constexpr int F4_BN = 128;
 constexpr int F4_BKB = 128;            // bytes of K per stage = 256 e2m1 elements = four MMAs of K = 64
 constexpr int F4_STAGES = 5;
@@ -213,8 +214,11 @@ fp4_gather_quantize_kernel(const __nv_bfloat16* __restrict__ x, const int* __res
 // offsets / scatter / zero-fill / gather launches of the sorted layout.
 constexpr int F4_SCATTER_WARPS = 4;
 
+// With group_tiles the rows go to the sorted layout instead: pair_pos[pair] is the pair's expert-major position, offsets and group_tiles [E + 1] the
+// experts' first positions and row tiles.  4000 tokens of 3072 channels to 10 experts each: 31 us; quantising every pair's row for itself took 146.
 __global__ void __launch_bounds__(F4_SCATTER_WARPS * 32)
 fp4_scatter_quantize_fixed_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ ids, int* __restrict__ cursors,
+                                  const int* __restrict__ pair_pos, const int* __restrict__ offsets, const int* __restrict__ group_tiles,
                                   uint8_t* __restrict__ packed, uint8_t* __restrict__ sf, float* __restrict__ row_scale,
                                   int* __restrict__ pair_ppos, int T, int k, int h, int E, int* err) {
   extern __shared__ __align__(16) uint8_t sq_smem[];
@@ -265,17 +269,23 @@ fp4_scatter_quantize_fixed_kernel(const __nv_bfloat16* __restrict__ x, const int
       if (lane == 0) pair_ppos[pair] = -1;
       continue;
     }
-    int slot = 0;
-    if (lane == 0) slot = atomicAdd(cursors + e, 1);
-    slot = __shfl_sync(0xffffffffu, slot, 0);
-    if (slot >= F4_BM) {                           // cannot happen while T <= 128; recorded, the row is dropped
-      if (lane == 0) { report_error(err, ERR_BOUNDS, 1500); pair_ppos[pair] = -1; }
-      continue;
+    int prow;
+    if (group_tiles != nullptr) {
+      prow = F4_BM * group_tiles[e] + pair_pos[pair] - offsets[e];
+    } else {
+      int slot = 0;
+      if (lane == 0) slot = atomicAdd(cursors + e, 1);
+      slot = __shfl_sync(0xffffffffu, slot, 0);
+      if (slot >= F4_BM) {                           // cannot happen while T <= 128; recorded, the row is dropped
+        if (lane == 0) { report_error(err, ERR_BOUNDS, 1500); pair_ppos[pair] = -1; }
+        continue;
+      }
+      prow = e * F4_BM + slot;
     }
-    const int prow = e * F4_BM + slot;
     uint8_t* dst = packed + static_cast<long long>(prow) * (h >> 1);
     for (int c = lane * 16; c < (h >> 1); c += 512) *reinterpret_cast<uint4*>(dst + c) = *reinterpret_cast<const uint4*>(q + c);
-    for (int kb = lane; kb < (h >> 4); kb += 32) sf[sf_offset(prow, kb, ktiles)] = qs[kb];
+    for (int kb = lane * 4; kb < (h >> 4); kb += 128)             // four neighbouring blocks are neighbours in the scale order (h is a multiple of 256)
+      *reinterpret_cast<uint32_t*>(sf + sf_offset(prow, kb, ktiles)) = *reinterpret_cast<const uint32_t*>(qs + kb);
     if (lane == 0) {
       row_scale[prow] = g;
       pair_ppos[pair] = prow;
@@ -398,6 +408,9 @@ fp4_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, Fp4Params p) {
       for (long long tile = tile0; tile < tiles && ok; tile += stride) {
         int e, mt, nt, lt;
         decode(tile, e, mt, nt, lt);
+        // Only the strips of 32 rows that hold rows of the expert are fetched; what lies in the others' shared memory reaches no stored result.  An SM
+        // takes in about 125 GB/s, and with 8 of 128 rows used the padding was 12 of a stage's 36 KB.
+        const int strips = min(4, (s.gr[e + 1] - s.gr[e] - lt * F4_BM + F4_STRIP - 1) / F4_STRIP);
         const uint8_t* sfa = p.sfa + static_cast<long long>(mt) * ktiles * 512;
         const uint8_t* sfb = p.sfb + (static_cast<long long>(e) * tiles_n + nt) * ktiles * 512;
         // the weight tile of a stage is one contiguous 16 KB image (rows already swizzled): a plain bulk copy, and DRAM sees
@@ -407,8 +420,9 @@ fp4_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, Fp4Params p) {
           const int st = it % F4_STAGES;
           const uint32_t ph = (it / F4_STAGES) & 1;
           if (!mbar_wait(&s.empty[st], ph ^ 1, p.err, 1100 + st)) { ok = false; break; }
-          mbar_expect_tx(&s.full[st], kStageBytes);
-          tma_load_2d(s.a[st], &tmA, &s.full[st], ks * F4_BKB, mt * F4_BM);
+          mbar_expect_tx(&s.full[st], kStageBytes - (4 - strips) * (F4_STRIP * F4_BKB));
+          for (int i = 0; i < strips; ++i)
+            tma_load_2d(s.a[st] + i * (F4_STRIP * F4_BKB), &tmA, &s.full[st], ks * F4_BKB, mt * F4_BM + i * F4_STRIP);
           bulk_load(s.b[st], wt + static_cast<long long>(ks) * (F4_BN * F4_BKB), F4_BN * F4_BKB, &s.full[st]);
           bulk_load(s.sfa[st], sfa + static_cast<long long>(ks) * F4_SF_STAGE, F4_SF_STAGE, &s.full[st]);
           bulk_load(s.sfb[st], sfb + static_cast<long long>(ks) * F4_SF_STAGE, F4_SF_STAGE, &s.full[st]);
@@ -558,13 +572,13 @@ static EncodeTiledFn f4_encode_fn() {
   });
   return fn;
 }
-// bytes [rows, kbytes] row-major, box 128 bytes x 128 rows, 128-byte swizzle
+// bytes [rows, kbytes] row-major, box 128 bytes x F4_STRIP rows, 128-byte swizzle
 static int make_tmap_u8(CUtensorMap* tm, const void* base, uint64_t kbytes, uint64_t rows) {
   EncodeTiledFn fn = f4_encode_fn();
   if (!fn) return -1;
   cuuint64_t dims[2] = {kbytes, rows};
   cuuint64_t strides[1] = {kbytes};
-  cuuint32_t box[2] = {128, 128};
+  cuuint32_t box[2] = {128, F4_STRIP};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -595,17 +609,30 @@ TYR_EXPORT int tyr_fp4_gather_quantize(const void* x, const int* pair_order, con
 
 // Quantise + scatter into the fixed-slot layout (T <= 128 tokens; see fp4_scatter_quantize_fixed_kernel).  `cursors` [E]
 // int32 zero on entry; packed [128 E, h / 2]; sf 128 E / 128 * (h / 64) * 512 bytes; row_scale [128 E]; pair_ppos [T k].
-TYR_EXPORT int tyr_fp4_scatter_quantize_fixed(const void* x, const int* ids, int* cursors, void* packed, void* sf, float* row_scale,
-                                              int* pair_ppos, int T, int k, int h, int E, int* err, void* stream) {
-  if (T <= 0 || T > F4_BM || h <= 0 || (h & 255) || k <= 0 || E <= 0) return -1;
+static int scatter_quantize(const void* x, const int* ids, int* cursors, const int* pair_pos, const int* offsets, const int* group_tiles, void* packed,
+                            void* sf, float* row_scale, int* pair_ppos, int T, int k, int h, int E, int* err, void* stream) {
+  if (T <= 0 || h <= 0 || (h & 255) || k <= 0 || E <= 0) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(packed)) & 15) return -2;
   const size_t per_warp = (static_cast<size_t>(h >> 1) + (h >> 4) + 15) & ~static_cast<size_t>(15);
   const size_t smem = per_warp * F4_SCATTER_WARPS;
   if (smem > 48 * 1024) return -3;
   return static_cast<int>(launch_dependent(
       fp4_scatter_quantize_fixed_kernel, dim3((T + F4_SCATTER_WARPS - 1) / F4_SCATTER_WARPS), dim3(F4_SCATTER_WARPS * 32), smem,
-      reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const __nv_bfloat16*>(x), ids, cursors,
+      reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const __nv_bfloat16*>(x), ids, cursors, pair_pos, offsets, group_tiles,
       reinterpret_cast<uint8_t*>(packed), reinterpret_cast<uint8_t*>(sf), row_scale, pair_ppos, T, k, h, E, err));
+}
+
+TYR_EXPORT int tyr_fp4_scatter_quantize_fixed(const void* x, const int* ids, int* cursors, void* packed, void* sf, float* row_scale,
+                                              int* pair_ppos, int T, int k, int h, int E, int* err, void* stream) {
+  if (T > F4_BM) return -1;
+  return scatter_quantize(x, ids, cursors, nullptr, nullptr, nullptr, packed, sf, row_scale, pair_ppos, T, k, h, E, err, stream);
+}
+
+// Quantise + scatter into the sorted layout: any number of tokens, positions from tyr_moe_layout.
+TYR_EXPORT int tyr_fp4_scatter_quantize(const void* x, const int* ids, const int* pair_pos, const int* offsets, const int* group_tiles, void* packed,
+                                        void* sf, float* row_scale, int* pair_ppos, int T, int k, int h, int E, int* err, void* stream) {
+  if (pair_pos == nullptr || offsets == nullptr || group_tiles == nullptr) return -5;
+  return scatter_quantize(x, ids, nullptr, pair_pos, offsets, group_tiles, packed, sf, row_scale, pair_ppos, T, k, h, E, err, stream);
 }
 
 struct TyrFp4GemmArgs {

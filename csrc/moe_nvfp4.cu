@@ -116,6 +116,11 @@ struct RouteArgs {
   float softcap, scale;
   int groups, keep;      // groups > 1: E / groups neighbouring experts form a group; only the `keep` groups with the best expert compete
   int ld;                // columns of a row of logits: E, or more where other projections of the token follow the router's
+  // Products with the terms of a split router matrix: a logit is the sum of `parts` numbers part_stride apart and, with `low`, of two columns of
+  // low [T, 2 E] that are E apart.
+  int parts;
+  long long part_stride;
+  const float* low;
 };
 
 // One warp routes one token from its row of logits.  The row may have been written by other CTAs of the same launch, so it is
@@ -131,6 +136,12 @@ __device__ __forceinline__ void route_token_n(const RouteArgs& a, const float* r
   for (int j = 0; j < kMaxPer; ++j) {
     const int e = lane + 32 * j;
     float l = (j < per && e < a.E) ? __ldcg(row + e) : -INFINITY;
+    if (a.low != nullptr && j < per && e < a.E) {
+      const float* lo = a.low + static_cast<long long>(tok) * 2 * a.E + e;
+      float s = __ldcg(lo) + __ldcg(lo + a.E);
+      for (int p = 1; p < a.parts; ++p) s += __ldcg(row + p * a.part_stride + e);
+      l += s;
+    }
     if (a.softcap > 0.f && l != -INFINITY) l = a.softcap * tanhf(l / a.softcap);
     score[j] = l;
     mx = fmaxf(mx, l);
@@ -222,7 +233,29 @@ __device__ __forceinline__ void route_token(const RouteArgs& a, const float* row
   else route_token_n<16>(a, row, tok, lane);       // E <= 512
 }
 
+__global__ void __launch_bounds__(256) split_bf16x3_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ out, long long n) {
+  pdl_entry();
+  for (long long i = (blockIdx.x * 256LL + threadIdx.x) * 4; i < n; i += gridDim.x * 1024LL) {
+    const float4 v = *reinterpret_cast<const float4*>(w + i);
+    const float f[4] = {v.x, v.y, v.z, v.w};
+    float t[3][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float hi = __bfloat162float(__float2bfloat16(f[j]));
+      const bool finite = fabsf(hi) < INFINITY;
+      const float r = finite ? f[j] - hi : 0.f, mid = __bfloat162float(__float2bfloat16(r));
+      t[0][j] = hi;
+      t[1][j] = mid;
+      t[2][j] = r - mid;
+    }
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+      *reinterpret_cast<uint2*>(out + p * n + i) = make_uint2(pack_bf16x2(t[p][0], t[p][1]), pack_bf16x2(t[p][2], t[p][3]));
+  }
+}
+
 __global__ void __launch_bounds__(256) moe_route_kernel(RouteArgs a) {
+  pdl_entry();
   const int lane = threadIdx.x & 31;
   const int tok = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (tok >= a.T) return;
@@ -349,6 +382,67 @@ __global__ void moe_scatter_kernel(const int* ids, const int* offsets, int* curs
   }
 }
 
+// The layout of a decode-sized batch in one launch: block 0 counts, sums and places all pairs (at most kSmallPairs; offsets, tiles, active as in
+// moe_offsets_kernel; order and pos of pairs that are not routed are 0), the other blocks clear `zero`.  In place of two clears and
+// two launches of a few us each.
+constexpr int kSmallPairs = 4096;
+__global__ void __launch_bounds__(1024) moe_layout_small_kernel(const int* __restrict__ ids, int* __restrict__ offsets, int* __restrict__ tiles,
+                                                                int* __restrict__ active, int* __restrict__ pair_order, int* __restrict__ pair_pos,
+                                                                int pairs, int E, float4* __restrict__ zero, long long n_zero) {
+  pdl_entry();
+  for (long long i = (blockIdx.x - 1LL) * blockDim.x + threadIdx.x; blockIdx.x > 0 && i < n_zero; i += (gridDim.x - 1LL) * blockDim.x)
+    zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (blockIdx.x > 0) return;
+  __shared__ int count[1024], first[1024];
+  __shared__ int warp_sum3[3][32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  if (t < E) count[t] = 0;
+  __syncthreads();
+  for (int p = t; p < pairs; p += blockDim.x) {
+    const int e = ids[p];
+    pair_order[p] = 0;
+    if (e >= 0 && e < E) atomicAdd(count + e, 1);
+    else (void)TYR_INDEX_OK(e, E + 1, 11);
+  }
+  __syncthreads();
+  const int c = t < E ? count[t] : 0;
+  int v[3] = {c, (c + 127) >> 7, c > 0 ? 1 : 0};
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const int u = __shfl_up_sync(0xffffffffu, v[q], o);
+      if (lane >= o) v[q] += u;
+    }
+  if (lane == 31)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) warp_sum3[q][warp] = v[q];
+  __syncthreads();
+  for (int w = 0; w < warp; ++w)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) v[q] += warp_sum3[q][w];
+  if (t < E) {
+    offsets[t + 1] = v[0];
+    tiles[t + 1] = v[1];
+    if (c > 0) active[v[2] - 1] = t;
+    if (t == E - 1) active[E] = v[2];
+    first[t] = v[0] - c;
+    count[t] = 0;
+  }
+  if (t == 0) offsets[0] = tiles[0] = 0;
+  __syncthreads();
+  for (int p = t; p < pairs; p += blockDim.x) {
+    const int e = ids[p];
+    if (e < 0 || e >= E) {
+      pair_pos[p] = 0;
+      continue;
+    }
+    const int pos = first[e] + atomicAdd(count + e, 1);
+    pair_order[pos] = p;
+    pair_pos[p] = pos;
+  }
+}
+
 // counts[e] += number of pairs routed to expert e; ids outside [0, E) are not counted (counts zero on entry)
 __global__ void moe_count_kernel(const int* ids, int* counts, int pairs, int E) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < pairs; p += gridDim.x * blockDim.x) {
@@ -470,15 +564,27 @@ moe_combine_kernel(const __nv_bfloat16* y, const int* pair_pos, const float* wei
        i < static_cast<long long>(T) * vec; i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int tok = static_cast<int>(i / vec), c = static_cast<int>(i % vec);
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int s = 0; s < k; ++s) {
-      const int pair = tok * k + s;
-      const float w = weights[pair];
-      const int pp = pair_pos[pair];
-      if (pp < 0) continue;                        // a pair that was not routed to an expert of this bank
-      uint4 u = reinterpret_cast<const uint4*>(y + static_cast<long long>(pp) * h)[c];
-      float2 a0 = unpack_bf16x2(u.x), a1 = unpack_bf16x2(u.y), a2 = unpack_bf16x2(u.z), a3 = unpack_bf16x2(u.w);
-      acc[0] += w * a0.x; acc[1] += w * a0.y; acc[2] += w * a1.x; acc[3] += w * a1.y;
-      acc[4] += w * a2.x; acc[5] += w * a2.y; acc[6] += w * a3.x; acc[7] += w * a3.y;
+    constexpr int U = 4;                             // rows in flight: one by one each waited for its place and then for itself
+    for (int s0 = 0; s0 < k; s0 += U) {
+      float w[U];
+      int pp[U];
+      uint4 u[U];
+#pragma unroll
+      for (int j = 0; j < U; ++j) {
+        const bool in = s0 + j < k;
+        pp[j] = in ? pair_pos[tok * k + s0 + j] : -1;      // -1: a pair that was not routed to an expert of this bank
+        w[j] = in ? weights[tok * k + s0 + j] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < U; ++j)
+        if (pp[j] >= 0) u[j] = reinterpret_cast<const uint4*>(y + static_cast<long long>(pp[j]) * h)[c];
+#pragma unroll
+      for (int j = 0; j < U; ++j) {
+        if (pp[j] < 0) continue;
+        const float2 a0 = unpack_bf16x2(u[j].x), a1 = unpack_bf16x2(u[j].y), a2 = unpack_bf16x2(u[j].z), a3 = unpack_bf16x2(u[j].w);
+        acc[0] += w[j] * a0.x; acc[1] += w[j] * a0.y; acc[2] += w[j] * a1.x; acc[3] += w[j] * a1.y;
+        acc[4] += w[j] * a2.x; acc[5] += w[j] * a2.y; acc[6] += w[j] * a3.x; acc[7] += w[j] * a3.y;
+      }
     }
     if (add) {
       uint4 u = reinterpret_cast<const uint4*>(add + static_cast<long long>(tok) * h)[c];
@@ -756,13 +862,18 @@ extern "C" TYR_EXPORT int tyr_nvfp4_dequant(const void* packed, const void* scal
 
 extern "C" TYR_EXPORT int tyr_moe_route(const float* logits, const float* bias, int* ids, float* weights, int* counts,
                                         int T, int E, int k, int softmax, int renorm, float softcap, float scale,
-                                        int groups, int keep, int ld, void* stream) {
-  if (ld < E) return -5;
+                                        int groups, int keep, int ld, int parts, long long part_stride, const float* low, void* stream) {
+  if (ld < E || parts < 1 || (parts > 1 && low == nullptr)) return -5;
   if (T <= 0 || E <= 0 || E > 512 || k <= 0 || k > 32 || k > E) return -1;
   if (groups > 1 && (groups > 32 || E % groups || keep <= 0 || keep > groups || k > keep * (E / groups))) return -4;
-  RouteArgs a{logits, bias, ids, weights, counts, T, E, k, softmax, renorm, softcap, scale, groups, keep, ld};
-  moe_route_kernel<<<(T + 7) / 8, 256, 0, (cudaStream_t)stream>>>(a);
-  return (int)cudaGetLastError();
+  RouteArgs a{logits, bias, ids, weights, counts, T, E, k, softmax, renorm, softcap, scale, groups, keep, ld, parts, part_stride, low};
+  return (int)launch_dependent(moe_route_kernel, dim3((T + 7) / 8), dim3(256), 0, (cudaStream_t)stream, a);
+}
+
+// w fp32 [n] -> bf16 [3][n], whose sum is w to 24 bits (the first term alone where it is not finite).
+extern "C" TYR_EXPORT int tyr_split_bf16x3(const float* w, void* out, long long n, void* stream) {
+  if (n <= 0 || (n & 3) || (reinterpret_cast<uintptr_t>(w) & 15) || (reinterpret_cast<uintptr_t>(out) & 7)) return -1;
+  return (int)launch_dependent(split_bf16x3_kernel, dim3(blocks_for(n / 4)), dim3(256), 0, (cudaStream_t)stream, w, (__nv_bfloat16*)out, n);
 }
 
 // Router GEMV + routing in one launch: x bf16 [T, h] (h a multiple of 8), router weight fp32 [ld, h] whose first E rows route (the
@@ -782,7 +893,7 @@ extern "C" TYR_EXPORT int tyr_moe_route_fused(const void* x, const float* router
     cudaFuncSetAttribute(moe_route_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     configured = smem;
   }
-  RouteArgs a{nullptr, bias, ids, weights, counts, T, E, k, softmax, renorm, softcap, scale, groups, keep, ld};
+  RouteArgs a{nullptr, bias, ids, weights, counts, T, E, k, softmax, renorm, softcap, scale, groups, keep, ld, 1, 0, nullptr};
   dim3 grid((T + kRouteTok - 1) / kRouteTok, (ld + kRouteExp - 1) / kRouteExp);
   return (int)launch_dependent(moe_route_fused_kernel, grid, dim3(256), smem, (cudaStream_t)stream, a, (const __nv_bfloat16*)x,
                                router_w, logits, tickets, h);
@@ -798,6 +909,17 @@ extern "C" TYR_EXPORT int tyr_moe_layout(const int* ids, const int* counts, int*
   moe_scatter_kernel<<<blocks_for(pairs), 256, 0, (cudaStream_t)stream>>>(ids, offsets, cursors, pair_order,
                                                                          pair_pos, pairs, E);
   return (int)cudaGetLastError();
+}
+
+// The same from the ids alone for at most 4096 pairs; `zero`: n_zero floats (a multiple of 4, 16-byte aligned, nullable) that the launch clears.
+extern "C" TYR_EXPORT int tyr_moe_layout_small(const int* ids, int* offsets, int* tiles, int* active, int* pair_order, int* pair_pos, int pairs, int E,
+                                               float* zero, long long n_zero, void* stream) {
+  if (pairs <= 0 || pairs > kSmallPairs || E <= 0 || E > 1024 || n_zero < 0 || (n_zero & 3) || (reinterpret_cast<uintptr_t>(zero) & 15)) return -1;
+  const long long clear = zero != nullptr ? (n_zero / 4 + 4095) / 4096 : 0;
+  int threads = 32;
+  while (threads < E || (threads < pairs && threads < 1024)) threads <<= 1;
+  return (int)launch_dependent(moe_layout_small_kernel, dim3(1 + (unsigned)(clear < 147 ? clear : 147)), dim3(threads), 0, (cudaStream_t)stream, ids, offsets,
+                               tiles, active, pair_order, pair_pos, pairs, E, reinterpret_cast<float4*>(zero), zero != nullptr ? n_zero / 4 : 0);
 }
 
 extern "C" TYR_EXPORT int tyr_moe_count(const int* ids, int* counts, int pairs, int E, void* stream) {

@@ -198,3 +198,60 @@ def test_gpu_grouped_gemm_empty_and_ragged_groups():
     assert torch.allclose(y.float().cpu(), ref.float(), atol=0.05, rtol=0.02)
 
 
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,k,E", [(1, 1, 1), (1, 10, 256), (7, 3, 33), (512, 8, 1024), (64, 32, 500)])
+def test_gpu_layout_of_a_decode_batch_in_one_launch(T, k, E):
+    g = torch.Generator().manual_seed(T + E)
+    ids = torch.stack([torch.randperm(E + 1, generator=g)[:k] for _ in range(T)]).int()      # E marks a pair that is not routed
+    zero = torch.ones(4 * 1031, device="cuda")
+    off, order, pos, tiles, active = (t.cpu() for t in moe.layout_small(ids.cuda(), E, zero))
+    flat = ids.reshape(-1).long()
+    live = flat < E
+    counts = torch.bincount(flat[live], minlength=E)
+    assert torch.equal(off[1:].long(), counts.cumsum(0)) and off[0] == 0 and torch.equal(tiles[1:].long(), ((counts + 127) // 128).cumsum(0)) and tiles[0] == 0
+    n = int((counts > 0).sum())
+    assert active[E] == n and torch.equal(active[:n].long(), torch.nonzero(counts).reshape(-1)) and not zero.any()
+    at = pos.long()[live]
+    assert torch.equal(order.long()[at], torch.nonzero(live).reshape(-1)) and torch.equal(torch.sort(at)[0], torch.arange(int(live.sum())))
+    assert ((at >= off.long()[flat[live]]) & (at < off.long()[flat[live] + 1])).all() and not pos[~live].any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,E,h", [(257, 8, 64), (300, 68, 1000), (513, 512, 3072)])
+def test_gpu_router_logits_in_three_terms(T, E, h):
+    """No further from 64 bits than the fp32 product; weights that are not finite give what they gave."""
+    g = torch.Generator().manual_seed(T + E)
+    x, w = torch.randn(T, h, generator=g).bfloat16().cuda(), torch.randn(E, h, generator=g).mul_(h ** -0.5).cuda()
+    with torch.no_grad():
+        assert moe.split_logits_supported(x, w)
+        total = lambda t: t[0].sum(0) + t[1].unflatten(1, (2, E)).sum(1)
+        got = moe.split_logits(x, w)
+        ref = x.double() @ w.double().T
+        err = lambda y: float((y.double() - ref).norm() / ref.norm())
+        single = x.float() @ w.T
+        assert err(total(got)) <= 1.2 * err(single) + 2.0 ** -24
+        a, b = moe.route(got[0], 5, low=got[1], renorm=True), moe.route(single, 5, renorm=True)
+        same = (a[0] == b[0]).all(1)
+        assert same.float().mean() > 0.98 and (a[1] - b[1])[same].abs().max() < 1e-5
+        w[1, 3] = float("inf")
+        assert torch.equal(total(moe.split_logits(x, w))[:, 1].isfinite(), (x.float() @ w.T)[:, 1].isfinite())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,k,E,h", [(1, 1, 3, 256), (130, 4, 9, 512), (300, 2, 40, 768)])
+def test_gpu_scatter_quantize_equals_gather_quantize(T, k, E, h):
+    """Every routed row at its place: the same codes, scales and factors."""
+    from tyr_b200.ops import fp4
+    g = torch.Generator().manual_seed(T + E)
+    x = torch.randn(T, h, generator=g).bfloat16().cuda()
+    ids = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(T)]).int().cuda()
+    off, order, pos, tiles = moe.layout(ids, moe.count_experts(ids, E), want_tiles=True)
+    padded = ((T * k + 127 * E + 127) // 128) * 128
+    a = fp4.gather_quantize(x, order, ids.reshape(-1), off, tiles, k, padded, T * k)
+    b = fp4.scatter_quantize(x, ids, pos, off, tiles, padded)
+    rows = a[3].long()
+    assert torch.equal(rows, b[3].long())
+    sf = lambda t: fp4.unswizzle_scales(t, padded, h // 16)[rows]
+    assert torch.equal(a[0][rows], b[0][rows]) and torch.equal(sf(a[1]), sf(b[1])) and torch.equal(a[2][rows], b[2][rows])

@@ -52,6 +52,14 @@ def _sigs(lib_):
         fn.restype = I
 
 
+@register_signatures
+def _scatter_sigs(lib_):
+    P, I = ctypes.c_void_p, ctypes.c_int
+    fn = getattr(lib_, "tyr_fp4_scatter_quantize", None)
+    if fn is not None:
+        fn.argtypes, fn.restype = [P] * 9 + [I] * 4 + [P, P], I
+
+
 def available() -> bool:
     return hasattr(lib(), "tyr_fp4_grouped_gemm")
 
@@ -226,9 +234,23 @@ def grouped_gemm_fp4(a_packed, a_sf, a_row_scale, w_packed, w_sf, w_global, tile
     return out if mode == 0 else (out, out_sf)
 
 
+def scatter_quantize(x: torch.Tensor, ids: torch.Tensor, pos: torch.Tensor, offsets: torch.Tensor, tiles: torch.Tensor, padded_rows: int):
+    """:func:`gather_quantize` of the sorted layout the other way round: every token is quantised once and its row written to each of its pairs'
+    places.  ids int32 [T, k], ``pos`` their expert-major positions -> the same four results."""
+    T, h = x.shape
+    k, E, dev = ids.shape[1], offsets.numel() - 1, x.device
+    packed = torch.empty((padded_rows, h // 2), dtype=torch.uint8, device=dev)
+    sf = torch.empty(padded_rows * (h // 16), dtype=torch.uint8, device=dev)
+    rs = torch.empty(padded_rows, dtype=torch.float32, device=dev)
+    ppos = torch.empty(T * k, dtype=torch.int32, device=dev)
+    check(lib().tyr_fp4_scatter_quantize(ptr(x.contiguous()), ptr(ids), ptr(pos), ptr(offsets), ptr(tiles), ptr(packed), ptr(sf), ptr(rs), ptr(ppos), T, k, h, E,
+                                         ptr(err_word(dev)), cur_stream(dev)), "fp4_scatter_quantize")
+    return packed, sf, rs, ppos
+
+
 def moe_fp4_tc_forward(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, ex, offsets, order, tiles,
-                       add: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """x [T, h] bf16, ids int32 [T, k], weights fp32 [T, k]; ``offsets`` / ``order`` / ``tiles`` from ``ops.moe.layout``.
+                       add: Optional[torch.Tensor] = None, pos: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """x [T, h] bf16, ids int32 [T, k], weights fp32 [T, k]; ``offsets`` / ``order`` / ``tiles`` from ``ops.moe.layout``, and its ``pos`` where there is one.
     Everything stays on the device: the row count of the padded layout is bounded on the host by T * k + 127 * E."""
     from . import moe as M
     T, h = x.shape
@@ -239,7 +261,8 @@ def moe_fp4_tc_forward(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor
     padded = ((pairs + 127 * min(E, pairs) + 127) // 128) * 128
     st = cur_stream(x.device)
     ids32 = ids.to(torch.int32).contiguous()
-    xq, xsf, xrs, ppos = gather_quantize(x, order, ids32.reshape(-1), offsets, tiles, k, padded, pairs)
+    xq, xsf, xrs, ppos = (gather_quantize(x, order, ids32.reshape(-1), offsets, tiles, k, padded, pairs) if pos is None else
+                          scatter_quantize(x, ids32, pos, offsets, tiles, padded))
     hq, hsf = grouped_gemm_fp4(xq, xsf, xrs, w4.gu_packed, w4.gu_sf, w4.gate_global, tiles, offsets,
                                2 * mi, h, mode=1, w_global2=w4.up_global)
     y = grouped_gemm_fp4(hq, hsf, None, w4.dn_packed, w4.dn_sf, w4.dn_global, tiles, offsets, h, mi, mode=0)
