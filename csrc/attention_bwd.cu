@@ -57,6 +57,7 @@ struct BwdParams {
   __nv_bfloat16* dQ;
   long long dk_sb, dk_st, dk_sh, dv_sb, dv_st, dv_sh, dq_sb, dq_st, dq_sh;
   int* err;
+  TileOrder order;
 };
 
 constexpr int BW_QST = 3;    // stages of the Q ring (dK/dV kernel) and of the K ring (dQ kernel)
@@ -115,9 +116,10 @@ flash_bwd_d128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   }
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int j = blockIdx.x;
-  const int kvh = blockIdx.y;
-  const int batch = blockIdx.z;
+  int j, bh;                                     // early key blocks are seen by the most queries: start them first
+  tile_of_block(p.order, blockIdx.x, j, bh);
+  const int kvh = bh % p.Hkv;
+  const int batch = bh / p.Hkv;
   const int G = p.Hq / p.Hkv;
   int ilo, ihi;
   q_range(p, j, ilo, ihi);
@@ -492,9 +494,11 @@ flash_bwd_dq_d128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   }
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int i = gridDim.x - 1 - blockIdx.x;      // late query blocks see the most keys: start them first
-  const int head = blockIdx.y;
-  const int batch = blockIdx.z;
+  int rank, bh;                                  // late query blocks see the most keys: start them first
+  tile_of_block(p.order, blockIdx.x, rank, bh);
+  const int i = p.order.tiles - 1 - rank;
+  const int head = bh % p.Hq;
+  const int batch = bh / p.Hq;
   const int kvh = head / (p.Hq / p.Hkv);
   int jlo, jhi;
   k_range(p, i * BW_T, jlo, jhi);
@@ -848,9 +852,11 @@ extern "C" TYR_EXPORT int tyr_flash_bwd(const void* dout, const void* q, const v
   p.dQ = (__nv_bfloat16*)dq;
   p.dq_sb = sdq[0]; p.dq_st = sdq[1]; p.dq_sh = sdq[2];
   p.err = err;
-  dim3 grid((Tk + BW_T - 1) / BW_T, Hkv, B);
-  launch_dependent(flash_bwd_d128_kernel, dim3(grid), dim3(640), smem, cs, tq, tk, tv, tdo, p);
-  launch_dependent(flash_bwd_dq_d128_kernel, dim3((Tq + BW_T - 1) / BW_T, Hq, B), dim3(576), smem_dq, cs, tq, tk, tv, tdo, p);
+  const bool uneven = causal && window == 0;
+  p.order = tile_order((Tk + BW_T - 1) / BW_T, B * Hkv, uneven, 512LL * Tq * Hq / Hkv);
+  launch_dependent(flash_bwd_d128_kernel, dim3(static_cast<unsigned>(p.order.tiles) * p.order.heads), dim3(640), smem, cs, tq, tk, tv, tdo, p);
+  p.order = tile_order((Tq + BW_T - 1) / BW_T, B * Hq, uneven, 512LL * Tk * Hkv / Hq);
+  launch_dependent(flash_bwd_dq_d128_kernel, dim3(static_cast<unsigned>(p.order.tiles) * p.order.heads), dim3(576), smem_dq, cs, tq, tk, tv, tdo, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + (int)e;
 }

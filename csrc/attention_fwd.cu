@@ -60,6 +60,7 @@ struct AttnParams {
   long long o_row_stride, o_batch_stride, o_head_stride;
   float* lse;         // [B, Hq, Tq]
   int* err;
+  TileOrder order;
   // distance penalty forms only
   const float *r1, *r2;   // [Hq]
   int k_steps;        // 16-channel steps of Q K^T
@@ -183,9 +184,11 @@ flash_fwd_d128_kernel(const __grid_constant__ CUtensorMap tmQ,
   const int lane = threadIdx.x & 31;
 
   // heavy (late) query tiles first: causal work grows with the row index
-  const int pair = gridDim.x - 1 - blockIdx.x;
-  const int head = blockIdx.y;
-  const int batch = blockIdx.z;
+  int rank, bh;
+  tile_of_block(p.order, blockIdx.x, rank, bh);
+  const int pair = p.order.tiles - 1 - rank;
+  const int head = bh % p.Hq;
+  const int batch = bh / p.Hq;
   const int kv_head = head / (p.Hq / p.Hkv);
   const int row0 = pair * 2 * ATT_BM;
 
@@ -684,8 +687,10 @@ static int flash_fwd_launch(const void* q, const void* k, const void* v, void* o
   p.O = (__nv_bfloat16*)o; p.o_batch_stride = st[9]; p.o_row_stride = st[10]; p.o_head_stride = st[11];
   p.lse = lse; p.err = err;
   p.r1 = r1; p.r2 = r2; p.k_steps = (dk + 15) / 16; p.dv = dv;
-  dim3 grid((Tq + 2 * ATT_BM - 1) / (2 * ATT_BM), Hq, B);
-  launch_dependent(kernel, dim3(grid), dim3(640), smem, (cudaStream_t)stream, tq, tk, tv, p);
+  const long long tiles = (Tq + 2 * ATT_BM - 1) / (2 * ATT_BM), heads = static_cast<long long>(B) * Hq;
+  if (tiles * heads > 0x7fffffff) return -5;
+  p.order = tile_order(static_cast<int>(tiles), static_cast<int>(heads), causal && window == 0, 512LL * Tk * Hkv / Hq);
+  launch_dependent(kernel, dim3(static_cast<unsigned>(tiles * heads)), dim3(640), smem, (cudaStream_t)stream, tq, tk, tv, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + (int)e;
 }

@@ -158,6 +158,7 @@ def _declare_kernels(lib):
     _sig(lib, "tyr_bind_device", [c_int])
     _sig(lib, "tyr_newton_schulz_scratch_bytes", [c_int, c_int, c_int], c_ll)
     _sig(lib, "tyr_newton_schulz_bf16", [P, P, c_ll, c_int, c_int, c_int, c_int, c_float, c_float, c_float, P, P])
+    _sig(lib, "tyr_newton_schulz_bf16_moved", [P, P, c_ll, c_int, c_int, c_int, c_int, c_float, c_float, c_float, P, P])
     _sig(lib, "tyr_lincomb_rmsnorm_fwd", [P, P, P, P, P, c_int, c_int, c_int, P, P, c_float, P])
     _sig(lib, "tyr_lincomb_rmsnorm_bwd",
          [ctypes.POINTER(P), ctypes.POINTER(P), P, P, P, P, P, c_int, c_int, c_int, c_float, P])

@@ -68,6 +68,31 @@ def _tall_step(g: torch.Tensor, a: float, b: float, c: float) -> torch.Tensor:
 _scratch = {}
 
 
+def _chain_scratch(x, need: int) -> torch.Tensor:
+    key = (x.device.index, need)
+    buf = _scratch.get(key)
+    if buf is None:
+        buf = torch.empty(need, dtype=torch.uint8, device=x.device)
+        _scratch.clear()
+        _scratch[key] = buf
+    return buf
+
+
+def newton_schulz_moved(x: torch.Tensor, num_iters: int) -> torch.Tensor:
+    """:func:`newton_schulz_` of a contiguous stacked batch whose storage the iterations may use: the result is x's storage or a fresh buffer, and x is not
+    kept."""
+    if not (_use_native(x) and x.dtype == torch.bfloat16 and x.dim() == 3 and x.is_contiguous()):
+        return newton_schulz_(x, num_iters)
+    from ._common import check, cur_stream, err_word, lib, ptr
+    B, R, C = x.shape
+    need = lib().tyr_newton_schulz_scratch_bytes(B, R, C)
+    buf = torch.empty(need, dtype=torch.uint8, device=x.device)
+    check(lib().tyr_newton_schulz_bf16_moved(ptr(x), ptr(buf), need, B, R, C, num_iters, *MUON_COEFFS, ptr(err_word(x.device)), cur_stream(x.device)),
+          "newton_schulz_moved")
+    S = min(R, C)
+    return buf[4 * B * S * S:4 * B * S * S + 2 * B * R * C].view(torch.bfloat16).view(B, R, C) if num_iters % 2 else x
+
+
 def _native_chain(x: torch.Tensor, num_iters: int) -> torch.Tensor:
     """All iterations through one native call (csrc/gemm_tcgen05.cu: tyr_newton_schulz_bf16);
     the scratch buffer is cached per (device, size)."""
@@ -76,12 +101,7 @@ def _native_chain(x: torch.Tensor, num_iters: int) -> torch.Tensor:
     B, R, C = xb.shape
     out = xb.contiguous().clone()
     need = lib().tyr_newton_schulz_scratch_bytes(B, R, C)
-    key = (x.device.index, need)
-    buf = _scratch.get(key)
-    if buf is None:
-        buf = torch.empty(need, dtype=torch.uint8, device=x.device)
-        _scratch.clear()
-        _scratch[key] = buf
+    buf = _chain_scratch(x, need)
     a, b, c = MUON_COEFFS
     check(lib().tyr_newton_schulz_bf16(ptr(out), ptr(buf), need, B, R, C, num_iters, a, b, c,
                                        ptr(err_word(x.device)), cur_stream(x.device)), "newton_schulz")

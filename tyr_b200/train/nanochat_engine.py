@@ -152,7 +152,7 @@ class MuonGroup:
         self.sumsq.zero_()
         ok.muon_momentum_(self.grad, self.momentum, self.u, self.sumsq, momentum, grad_scale)
         ok.scale_by_inv_norm_(self.u, self.sumsq, 1e-7)
-        o = polar.newton_schulz_(self.u, num_iters)
+        o = polar.newton_schulz_moved(self.u, num_iters)
         eff_lr = lr * aspect_ratio_scale(self.master.shape)
         ok.muon_apply_(self.master, o.contiguous(), eff_lr, weight_decay,
                        self.work if self.work.dtype == torch.bfloat16 else None)
