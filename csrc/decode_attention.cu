@@ -162,23 +162,66 @@ __device__ __forceinline__ void decode_combine(const DecodeAttnArgs& a, int b, i
   __syncthreads();
   if (*ticket != a.splits - 1) return;
   __threadfence();
-  for (int i = tid; i < G * DV; i += kDecWarps * 32) {
-    const int g = i / DV, d = i - g * DV;
+  // The slices' weights first, a warp per head, then the sums with the loads of several channels and slices in flight.  One channel after the other,
+  // each with its own passes over the slices, was most of the kernel where few CTAs merge much: one row of
+  // 8 heads of 256 over 564 keys in 9 slices took 26.2 us and takes 13.4, 32 slices 67.6 and 16.6.
+  __shared__ float s_f[GM][32], s_M[GM], s_L[GM];                 // at most 32 slices
+  const int warp = tid >> 5, lane = tid & 31;
+  for (int g = warp; g < G; g += kDecWarps) {
     const long long row = static_cast<long long>(b) * a.Hq + hq0 + g;
-    float M = -INFINITY;
-    if (a.back != nullptr && d >= a.back_half) continue;
-    for (int sp = 0; sp < a.splits; ++sp) M = fmaxf(M, __ldcg(&a.part_ml[(row * a.splits + sp) * 2]));
-    float L = 0.f, A = 0.f, A2 = 0.f;
-    if (M > -INFINITY) {
+    const bool in = lane < a.splits;
+    const float m = in ? __ldcg(&a.part_ml[(row * a.splits + lane) * 2]) : -INFINITY;
+    const float M = warp_max(m);
+    const float f = in && m > -INFINITY ? exp2f(m - M) : 0.f;
+    const float L = warp_sum(f != 0.f ? __ldcg(&a.part_ml[(row * a.splits + lane) * 2 + 1]) * f : 0.f);
+    s_f[g][lane] = f;
+    if (lane == 0) {
+      s_M[g] = M;
+      s_L[g] = L;
+    }
+  }
+  __syncthreads();
+  const float* part = a.part_acc + (static_cast<long long>(b) * a.Hq + hq0) * a.splits * DV;
+  if (a.back != nullptr) {
+    for (int i = tid; i < G * DV; i += kDecWarps * 32) {
+      const int g = i / DV, d = i % DV;
+      if (d >= a.back_half) continue;
+      const float* acc = part + static_cast<long long>(g) * a.splits * DV + d;
+      float A = 0.f, A2 = 0.f;
+#pragma unroll 4
       for (int sp = 0; sp < a.splits; ++sp) {
-        const float f = exp2f(__ldcg(&a.part_ml[(row * a.splits + sp) * 2]) - M);
-        L += __ldcg(&a.part_ml[(row * a.splits + sp) * 2 + 1]) * f;
-        A += __ldcg(&a.part_acc[(row * a.splits + sp) * DV + d]) * f;
-        if (a.back != nullptr) A2 += __ldcg(&a.part_acc[(row * a.splits + sp) * DV + d + a.back_half]) * f;
+        A += __ldcg(acc + sp * DV) * s_f[g][sp];
+        A2 += __ldcg(acc + sp * DV + a.back_half) * s_f[g][sp];
+      }
+      decode_write_turned(a, b, hq0 + g, d, a.pos[b * a.pos_stride], s_M[g], s_L[g], A, A2);
+    }
+  } else {
+    constexpr int U = 4;                         // channels of a thread at a time; no branch between the loads
+    for (int i0 = tid; i0 < G * DV; i0 += U * kDecWarps * 32) {
+      float A[U];
+      const float* acc[U];
+      const float* f[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = min(i0 + u * kDecWarps * 32, G * DV - 1), g = i / DV;
+        A[u] = 0.f;
+        acc[u] = part + static_cast<long long>(g) * a.splits * DV + i % DV;
+        f[u] = s_f[g];
+      }
+#pragma unroll 4
+      for (int sp = 0; sp < a.splits; ++sp) {
+        float v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = __ldcg(acc[u] + sp * DV);
+#pragma unroll
+        for (int u = 0; u < U; ++u) A[u] += v[u] * f[u][sp];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + u * kDecWarps * 32;
+        if (i < G * DV) decode_write(a, b, hq0 + i / DV, i % DV, s_M[i / DV], s_L[i / DV], A[u]);
       }
     }
-    if (a.back != nullptr) decode_write_turned(a, b, hq0 + g, d, a.pos[b * a.pos_stride], M, L, A, A2);
-    else decode_write(a, b, hq0 + g, d, M, L, A);
   }
   if (tid == 0) a.counters[b * a.Hkv + hkv] = 0;
 }

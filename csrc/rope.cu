@@ -396,13 +396,16 @@ struct RopeNormArgs {
   const int* pos;              // [rows] (nullable)
   long long row_stride;        // elements between rows of x
   long long y_row_stride;      // elements between rows of y
+  long long head_stride;       // elements between heads of x
   int rows, T, H, D, rot;
   float eps;
   int one_plus_w;
 };
+struct RopeNormPair { RopeNormArgs of[2]; };    // gridDim.y of them in one launch (queries and keys)
 
-__global__ void __launch_bounds__(256) rope_norm_kernel(RopeNormArgs a) {
+__global__ void __launch_bounds__(256) rope_norm_kernel(const __grid_constant__ RopeNormPair pair) {
   pdl_entry();
+  const RopeNormArgs& a = pair.of[blockIdx.y];
   const int lane = threadIdx.x & 31;
   const long long unit0 = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const long long units = static_cast<long long>(a.rows) * a.H;
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(256) rope_norm_kernel(RopeNormArgs a) {
   for (long long u = unit0; u < units; u += stride) {
     const long long row = u / a.H;
     const int head = static_cast<int>(u % a.H);
-    const __nv_bfloat16* x = a.x + row * a.row_stride + static_cast<long long>(head) * a.D;
+    const __nv_bfloat16* x = a.x + row * a.row_stride + head * a.head_stride;
     __nv_bfloat16* y = a.y + row * a.y_row_stride + static_cast<long long>(head) * a.D;
     float rstd = 1.f;
     if (a.w) {
@@ -497,8 +500,20 @@ extern "C" TYR_EXPORT int tyr_rope_norm(const void* x, void* y, const void* w, c
                                         int one_plus_w, void* stream) {
   if (rot > D || (rot & 1)) return -1;
   RopeNormArgs a{(const __nv_bfloat16*)x, (__nv_bfloat16*)y, (const __nv_bfloat16*)w, cosT, sinT,
-                 pos, row_stride, y_row_stride, rows, T, H, D, rot, eps, one_plus_w};
-  return (int)launch_dependent(rope_norm_kernel, dim3(grid_for_units(1LL * rows * H, 8)), dim3(256), 0, (cudaStream_t)stream, a);
+                 pos, row_stride, y_row_stride, D, rows, T, H, D, rot, eps, one_plus_w};
+  return (int)launch_dependent(rope_norm_kernel, dim3(grid_for_units(1LL * rows * H, 8)), dim3(256), 0, (cudaStream_t)stream, RopeNormPair{{a, a}});
+}
+
+// Queries and keys of the same rows in one launch.  strides: row and head strides of q, of k; both outputs are contiguous.
+extern "C" TYR_EXPORT int tyr_rope_norm_qk(const void* q, const void* k, void* q_out, void* k_out, const void* qw, const void* kw, const float* cosT,
+                                           const float* sinT, const int* pos, const long long* strides, int rows, int T, int H, int G, int D, int rot,
+                                           float eps, int one_plus_w, void* stream) {
+  if (rot > D || (rot & 1) || rows < 1 || H < 1 || G < 1) return -1;
+  const RopeNormPair pair{{{(const __nv_bfloat16*)q, (__nv_bfloat16*)q_out, (const __nv_bfloat16*)qw, cosT, sinT, pos, strides[0], 1LL * H * D, strides[1],
+                            rows, T, H, D, rot, eps, one_plus_w},
+                           {(const __nv_bfloat16*)k, (__nv_bfloat16*)k_out, (const __nv_bfloat16*)kw, cosT, sinT, pos, strides[2], 1LL * G * D, strides[3],
+                            rows, T, G, D, rot, eps, one_plus_w}}};
+  return (int)launch_dependent(rope_norm_kernel, dim3(grid_for_units(1LL * rows * (H > G ? H : G), 8), 2), dim3(256), 0, (cudaStream_t)stream, pair);
 }
 
 TYR_DEFINE_BOUNDS_STATUS(rope)

@@ -48,6 +48,13 @@ struct SkinnyArgs {
   float act_a, act_b;
   const __nv_bfloat16* aux;    // [M, N], row stride ldaux
   long long ldaux;
+  // NORM form: the activations are the RMS norm of x + resid (both [M, K], rows ldx and ldr apart; resid nullable) with gain norm_w (or 1 + norm_w);
+  // the sum goes to resid_out [M, K] (nullable).
+  const __nv_bfloat16 *resid, *norm_w;
+  __nv_bfloat16* resid_out;
+  long long ldr;
+  float eps;
+  int one_plus_w;
 };
 
 __device__ __forceinline__ float sk_act(float z, const SkinnyArgs& a, int tok, int row) {
@@ -63,9 +70,71 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 
 constexpr long long kSkPrefetchBytes = 32LL << 20;   // L2 prefetch issued by one launch before its input is ready
 
-template <int TILES, bool GATED>                   // token tiles of 8: M <= 8 * TILES; GATED: two matrices, SwiGLU epilogue
+// The norm in front of the products, taken again by every CTA: a launch of its own costs a decoding step about 2.5 us, reading the rows from the L2
+// and one more reduction about 1.  A row belongs to 8 / (M rounded up to a power of two) warps; the sum is rounded to bf16 before the norm, like
+// the norm kernel's.  -> xs [M][K + 8]
+__device__ __forceinline__ void sk_norm_rows(const SkinnyArgs& a, __nv_bfloat16* xs, float* s_part) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int per = a.M <= 1 ? 8 : a.M <= 2 ? 4 : a.M <= 4 ? 2 : 1;       // warps of a row
+  const int row = warp / per, part = warp % per, nvec = a.K >> 3;
+  const bool live = row < a.M;
+  const bool first = blockIdx.x == 0 && blockIdx.y == 0 && a.resid_out != nullptr;
+  auto unpack = [](uint4 u, float (&f)[8]) {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 p = unpack_bf16x2(w[j]);
+      f[2 * j] = p.x;
+      f[2 * j + 1] = p.y;
+    }
+  };
+  auto pack = [](const float (&f)[8]) {
+    return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+  };
+  float ss = 0.f;
+  if (live)
+#pragma unroll 4
+    for (int v = part * 32 + lane; v < nvec; v += per * 32) {
+      uint4 u = *reinterpret_cast<const uint4*>(a.x + row * a.ldx + v * 8);
+      float f[8];
+      unpack(u, f);
+      if (a.resid != nullptr) {
+        float r[8];
+        unpack(*reinterpret_cast<const uint4*>(a.resid + row * a.ldr + v * 8), r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] += r[j];
+        u = pack(f);
+        unpack(u, f);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+      *reinterpret_cast<uint4*>(xs + row * (a.K + 8) + v * 8) = u;
+      if (first) *reinterpret_cast<uint4*>(a.resid_out + static_cast<long long>(row) * a.K + v * 8) = u;
+    }
+  ss = warp_sum(ss);
+  if (lane == 0) s_part[warp] = ss;
+  __syncthreads();
+  if (live) {
+    float t = 0.f;
+    for (int i = 0; i < per; ++i) t += s_part[row * per + i];
+    const float rstd = rsqrtf(t / a.K + a.eps);
+#pragma unroll 4
+    for (int v = part * 32 + lane; v < nvec; v += per * 32) {
+      float f[8], w[8];
+      unpack(*reinterpret_cast<const uint4*>(xs + row * (a.K + 8) + v * 8), f);
+      unpack(__ldg(reinterpret_cast<const uint4*>(a.norm_w + v * 8)), w);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * (a.one_plus_w ? w[j] + 1.f : w[j]);
+      *reinterpret_cast<uint4*>(xs + row * (a.K + 8) + v * 8) = pack(f);
+    }
+  }
+  __syncthreads();
+}
+
+template <int TILES, bool GATED, bool NORM>        // token tiles of 8: M <= 8 * TILES; GATED: two matrices, SwiGLU epilogue
 __global__ void __launch_bounds__(kSkWarps * 32) skinny_gemm_kernel(SkinnyArgs a, const __grid_constant__ SkinnySegments seg) {
   __shared__ float part[GATED ? 2 : 1][kSkWarps][TILES][16][8];
+  extern __shared__ __align__(16) __nv_bfloat16 sk_rows[];         // NORM: [M][K + 8]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
   int tile = blockIdx.x;
@@ -96,6 +165,10 @@ __global__ void __launch_bounds__(kSkWarps * 32) skinny_gemm_kernel(SkinnyArgs a
       bulk_prefetch_l2((tid < 16 ? a.w : a.w2) + static_cast<long long>(r) * a.ldw + 32LL * c0, static_cast<uint32_t>(per_row));
   }
   pdl_wait();
+  if constexpr (NORM) {
+    __shared__ float s_part[kSkWarps];
+    sk_norm_rows(a, sk_rows, s_part);
+  }
   int r_lo = row0 + g, r_hi = row0 + g + 8;
   r_lo = r_lo < a.N ? r_lo : a.N - 1;            // clamped rows are not written
   r_hi = r_hi < a.N ? r_hi : a.N - 1;
@@ -109,7 +182,7 @@ __global__ void __launch_bounds__(kSkWarps * 32) skinny_gemm_kernel(SkinnyArgs a
   for (int i = 0; i < TILES; ++i) {
     const int tok = 8 * i + g;
     live[i] = tok < a.M;
-    xr[i] = a.x + (live[i] ? tok : 0) * a.ldx + 8 * t;
+    xr[i] = NORM ? sk_rows + (live[i] ? tok : 0) * (a.K + 8) + 8 * t : a.x + (live[i] ? tok : 0) * a.ldx + 8 * t;
   }
   float acc[TILES][4], acc2[TILES][4];
 #pragma unroll
@@ -132,7 +205,8 @@ __global__ void __launch_bounds__(kSkWarps * 32) skinny_gemm_kernel(SkinnyArgs a
     }
 #pragma unroll
     for (int i = 0; i < TILES; ++i) {
-      const uint4 xv = live[i] ? __ldg(reinterpret_cast<const uint4*>(xr[i] + 32 * c)) : make_uint4(0u, 0u, 0u, 0u);
+      const uint4* xp = reinterpret_cast<const uint4*>(xr[i] + 32 * c);
+      const uint4 xv = live[i] ? (NORM ? *xp : __ldg(xp)) : make_uint4(0u, 0u, 0u, 0u);
       mma_16816(acc[i], lo.x, hi.x, lo.y, hi.y, xv.x, xv.y);
       mma_16816(acc[i], lo.z, hi.z, lo.w, hi.w, xv.z, xv.w);
       if (GATED) {
@@ -273,12 +347,12 @@ template <int TILES, bool GATED>
 static void skinny_set_carveout() {
   const int per_cta = (GATED ? 2 : 1) * tyr::kSkWarps * TILES * 16 * 8 * 4 + 1024;
   int ctas = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, tyr::skinny_gemm_kernel<TILES, GATED>, tyr::kSkWarps * 32, 0) != cudaSuccess ||
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, tyr::skinny_gemm_kernel<TILES, GATED, false>, tyr::kSkWarps * 32, 0) != cudaSuccess ||
       ctas < 1)
     return;
   int pct = (ctas * per_cta * 100 + 227 * 1024 - 1) / (227 * 1024);
   if (pct > 100) pct = 100;
-  cudaFuncSetAttribute(tyr::skinny_gemm_kernel<TILES, GATED>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+  cudaFuncSetAttribute(tyr::skinny_gemm_kernel<TILES, GATED, false>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
 }
 static void skinny_prefer_l1() {
   static bool done[64] = {};
@@ -308,13 +382,15 @@ static int skinny_splits(int row_ctas, int M, int K) {
   return splits < 1 ? 1 : splits;
 }
 
-template <int TILES, bool GATED>
+template <int TILES, bool GATED, bool NORM = false>
 static cudaError_t skinny_start(dim3 grid, cudaStream_t stream, const tyr::SkinnyArgs& a, const tyr::SkinnySegments& seg) {
   using namespace tyr;
-  if (grid.y == 1) return launch_dependent(skinny_gemm_kernel<TILES, GATED>, grid, dim3(kSkWarps * 32), 0, stream, a, seg);
+  const size_t smem = NORM ? static_cast<size_t>(a.M) * (a.K + 8) * 2 : 0;
+  if (grid.y == 1) return launch_dependent(skinny_gemm_kernel<TILES, GATED, NORM>, grid, dim3(kSkWarps * 32), smem, stream, a, seg);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kSkWarps * 32);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -322,7 +398,7 @@ static cudaError_t skinny_start(dim3 grid, cudaStream_t stream, const tyr::Skinn
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   cfg.attrs = at; cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, skinny_gemm_kernel<TILES, GATED>, a, seg);
+  return cudaLaunchKernelEx(&cfg, skinny_gemm_kernel<TILES, GATED, NORM>, a, seg);
 }
 
 static int skinny_launch(const tyr::SkinnyArgs& a, const tyr::SkinnySegments& seg, int row_ctas, int splits, void* stream) {
@@ -339,6 +415,7 @@ static int skinny_launch(const tyr::SkinnyArgs& a, const tyr::SkinnySegments& se
   const dim3 grid(row_ctas, splits > 0 ? splits : skinny_splits(row_ctas, a.M, a.K));
   const cudaStream_t st = (cudaStream_t)stream;
   skinny_prefer_l1();
+  if (a.norm_w != nullptr) return (int)skinny_start<1, false, true>(grid, st, a, seg);
   return (int)(a.M <= 8 ? skinny_start<1, false>(grid, st, a, seg) : a.M <= 16 ? skinny_start<2, false>(grid, st, a, seg) : skinny_start<4, false>(grid, st, a, seg));
 }
 
@@ -352,9 +429,8 @@ static int skinny_single(const void* x, const void* w, const void* bias, void* y
   return skinny_launch(a, seg, (N + 15) / 16, 0, stream);
 }
 
-// Up to four matrices W[i] [N[i], K] that read the same x: y[i] = x W[i]^T in one launch.  `splits`: CTAs that share a contraction (0: by size).
-extern "C" TYR_EXPORT int tyr_skinny_many_bf16(const void* x, long long ldx, int n, const void* const* w, void* const* y, const long long* ldw,
-                                               const long long* ldy, const int* N, int M, int K, int splits, void* stream) {
+static int skinny_many(tyr::SkinnyArgs a, int n, const void* const* w, void* const* y, const long long* ldw, const long long* ldy, const int* N, int splits,
+                       void* stream) {
   using namespace tyr;
   if (n < 1 || n > kSkSegments) return -5;
   SkinnySegments seg{};
@@ -370,8 +446,60 @@ extern "C" TYR_EXPORT int tyr_skinny_many_bf16(const void* x, long long ldx, int
     tiles += (N[i] + 15LL) / 16;
     if (tiles > 0x7fffffff) return -1;
   }
-  const SkinnyArgs a{(const __nv_bfloat16*)x, seg.w[0], nullptr, nullptr, seg.y[0], ldx, ldw[0], ldy[0], M, N[0], K};
+  a.w = seg.w[0];
+  a.y = seg.y[0];
+  a.ldw = ldw[0];
+  a.ldy = ldy[0];
+  a.N = N[0];
   return skinny_launch(a, seg, (int)tiles, splits, stream);
+}
+
+// Up to four matrices W[i] [N[i], K] that read the same x: y[i] = x W[i]^T in one launch.  `splits`: CTAs that share a contraction (0: by size).
+extern "C" TYR_EXPORT int tyr_skinny_many_bf16(const void* x, long long ldx, int n, const void* const* w, void* const* y, const long long* ldw,
+                                               const long long* ldy, const int* N, int M, int K, int splits, void* stream) {
+  tyr::SkinnyArgs a{};
+  a.x = (const __nv_bfloat16*)x; a.ldx = ldx; a.M = M; a.K = K;
+  return skinny_many(a, n, w, y, ldw, ldy, N, splits, stream);
+}
+
+// The operand of the NORM forms: at most kSkNormNumbers of a batch's M <= 8 rows in a CTA's shared memory.
+constexpr int kSkNormNumbers = 16384;
+static int skinny_norm_args(tyr::SkinnyArgs& a, const void* x, const void* resid, const void* norm_w, void* resid_out, long long ldx, long long ldr, int M, int K,
+                            float eps, int one_plus_w) {
+  if (M < 1 || M > 8 || K < 32 || (K & 31) || M * (K + 8LL) > kSkNormNumbers || norm_w == nullptr) return -1;
+  if ((ldx | ldr) & 7) return -2;
+  for (const void* p : {x, resid, norm_w, (const void*)resid_out})
+    if (reinterpret_cast<uintptr_t>(p) & 15) return -3;
+  a.x = (const __nv_bfloat16*)x; a.resid = (const __nv_bfloat16*)resid; a.norm_w = (const __nv_bfloat16*)norm_w; a.resid_out = (__nv_bfloat16*)resid_out;
+  a.ldx = ldx; a.ldr = ldr; a.M = M; a.K = K; a.eps = eps; a.one_plus_w = one_plus_w;
+  return 0;
+}
+
+// The same of the RMS norm of x + resid (resid nullable; the sum goes to resid_out [M, K], nullable) with gain norm_w or 1 + norm_w.
+extern "C" TYR_EXPORT int tyr_skinny_norm_many_bf16(const void* x, const void* resid, const void* norm_w, void* resid_out, long long ldx, long long ldr, int n,
+                                                    const void* const* w, void* const* y, const long long* ldw, const long long* ldy, const int* N, int M,
+                                                    int K, float eps, int one_plus_w, void* stream) {
+  tyr::SkinnyArgs a{};
+  const int rc = skinny_norm_args(a, x, resid, norm_w, resid_out, ldx, ldr, M, K, eps, one_plus_w);
+  return rc ? rc : skinny_many(a, n, w, y, ldw, ldy, N, 0, stream);
+}
+
+// y [M, N] = silu(h wg^T) * (h wu^T) of the same norm h (both matrices with row stride ldw).
+extern "C" TYR_EXPORT int tyr_skinny_norm_swiglu_bf16(const void* x, const void* resid, const void* norm_w, void* resid_out, long long ldx, long long ldr,
+                                                      const void* wg, const void* wu, void* y, long long ldw, int M, int N, int K, float eps,
+                                                      int one_plus_w, void* stream) {
+  using namespace tyr;
+  SkinnyArgs a{};
+  const int rc = skinny_norm_args(a, x, resid, norm_w, resid_out, ldx, ldr, M, K, eps, one_plus_w);
+  if (rc) return rc;
+  if (N < 1) return -1;
+  if (ldw & 7) return -2;
+  if ((reinterpret_cast<uintptr_t>(wg) | reinterpret_cast<uintptr_t>(wu)) & 15) return -3;
+  a.w = (const __nv_bfloat16*)wg; a.w2 = (const __nv_bfloat16*)wu; a.y = (__nv_bfloat16*)y;
+  a.ldw = ldw; a.ldy = N; a.N = N;
+  SkinnySegments seg{};
+  seg.n = 1;
+  return (int)skinny_start<1, true, true>(dim3((N + 15) / 16, 1), (cudaStream_t)stream, a, seg);
 }
 
 extern "C" TYR_EXPORT int tyr_skinny_gemm_bf16(const void* x, const void* w, const void* bias, void* y, long long ldx,

@@ -774,3 +774,55 @@ def test_gemm_with_gated_addend(rows, bn, sets, per, N, K):
     acc = a.double() @ b.double().T
     ref = aux.double() + gate.double().repeat_interleave(per, 0) * acc
     assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * acc.abs().max() * gate.abs().max().double()).all()
+
+
+@pytest.mark.parametrize("M,Ns,K,resid", [(1, (40, 16, 7), 1024, True), (3, (1024,), 3584, True), (8, (48, 130), 2016, True), (5, (64,), 32, False), (2, (2048, 16), 8000, True)])
+def test_skinny_products_of_a_norm(M, Ns, K, resid):
+    """The norm taken by every CTA of the products against fp64 on the bf16 sum.  h is rounded to bf16 (2^-9 of each number, 2^-9 of a product's root sum of squares
+    with random signs, times 4 for the largest of a few hundred) and so is the result."""
+    from tyr_b200.ops.skinny import norm_supported, skinny_norm_many, skinny_norm_swiglu
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, res, nw = r(M, K + 8)[:, 8:], r(M, K) if resid else None, r(K) * 0.1
+    ws = [(r(N, K).float() * K ** -0.5).bfloat16() for N in Ns]
+    assert norm_supported(x, nw, ws)
+    ys, s = skinny_norm_many(x, res, nw, 1e-6, ws, one_plus_w=True)
+    want = x if res is None else (x.float() + res.float()).bfloat16()
+    assert torch.equal(s, want)
+    h = want.double() * torch.rsqrt(want.double().pow(2).mean(-1, keepdim=True) + 1e-6) * (1 + nw.double())
+    tol = lambda ref: 2.0 ** -8 * ref.abs() + 2.0 ** -7 * (h.norm(dim=-1, keepdim=True) * K ** -0.5)
+    for y, w in zip(ys, ws):
+        ref = h @ w.double().T
+        assert ((y.double() - ref).abs() <= tol(ref)).all()
+    up = (r(Ns[0], K).float() * K ** -0.5).bfloat16()
+    y, s2 = skinny_norm_swiglu(x, res, nw, 1e-6, ws[0], up, one_plus_w=True)
+    a, b = h @ ws[0].double().T, h @ up.double().T
+    ref = torch.nn.functional.silu(a) * b
+    assert torch.equal(s2, want) and ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -7 * (1 + a.abs() + b.abs())).all()
+
+
+def test_rope_norm_of_queries_and_keys_in_one_launch():
+    from tyr_b200.ops.rope import rope_norm, rope_norm_qk
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    for B, H, G, D, half in ((1, 8, 2, 256, 32), (5, 3, 3, 64, 32)):
+        q, k, qw, kw = r(B, H, 2 * D)[..., :D], r(B, G, D), r(D), r(D)
+        ang = torch.rand(40, half, device="cuda", generator=g) * 6
+        pos = torch.randint(0, 40, (B,), device="cuda", generator=g).int()
+        got = rope_norm_qk(q, k, ang.cos(), ang.sin(), q_weight=qw, k_weight=kw, positions=pos, one_plus_w=True)
+        for y, t, w in zip(got, (q, k), (qw, kw)):
+            assert torch.equal(y, rope_norm(t.contiguous(), ang.cos(), ang.sin(), weight=w, positions=pos, rot=2 * half, one_plus_w=True))
+
+
+@pytest.mark.parametrize("splits", [1, 2, 5, 32])
+@pytest.mark.parametrize("B,H,G,D", [(1, 8, 1, 256), (2, 16, 1, 64), (3, 6, 2, 128)])
+def test_decode_attention_merges_any_number_of_slices(splits, B, H, G, D):
+    """Also slices without keys.  Scores and sums in fp32, P rounded to bf16 (2^-9 of a mean of unit values) and the result too."""
+    from tyr_b200.ops.decode_attention import decode_attention
+    g = torch.Generator().manual_seed(splits + D)
+    r = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    cap, pos = 300, torch.tensor([257], dtype=torch.int32)
+    q, k, v, kc, vc = r(B, H, D), r(B, G, D), r(B, G, D), r(B, G, cap, D), r(B, G, cap, D)
+    want = decode_attention(q.float(), k.float(), v.float(), kc.clone().float(), vc.clone().float(), pos)
+    got = decode_attention(*(t.cuda() for t in (q, k, v, kc, vc, pos)), splits=splits)
+    assert (got.float().cpu() - want).abs().max() <= 2.0 ** -7

@@ -19,9 +19,10 @@ from ..io import safetensors as st
 from ..ops import delta_rule as dr
 from ..ops import moe as moe_ops
 from ..ops import prompt_mix
+from ..ops import skinny
 from ..ops.attention import attention
 from ..ops.decode_attention import decode_attention, geometry_supported
-from ..ops.rope import rope_norm
+from ..ops.rope import rope_norm_qk
 from .common import KVCache, LinearState, apply_rotary_partial, cached_attention, cos_sin_tables, gated_mlp, head_norm, lin, lin_many, norm_w, plain_inv_freq, swiglu_mlp
 from .generation import SamplingStrategy, generate_cached
 from .laguna import name_candidates
@@ -281,9 +282,8 @@ def attention_core_decode(cfg: Qwen35Config, q_norm, k_norm, qg, k, v, cos_table
     H, Hkv, D = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
     qg = qg.reshape(B, H, 2 * D)
     positions = pos_t.expand(B)
-    rot = 2 * cos_table.shape[1]
-    q = rope_norm(qg[..., :D], cos_table, sin_table, weight=q_norm, positions=positions, rot=rot, eps=cfg.rms_norm_eps, one_plus_w=True)
-    kn = rope_norm(k.reshape(B, Hkv, D), cos_table, sin_table, weight=k_norm, positions=positions, rot=rot, eps=cfg.rms_norm_eps, one_plus_w=True)
+    q, kn = rope_norm_qk(qg[..., :D], k.reshape(B, Hkv, D), cos_table, sin_table, q_weight=q_norm, k_weight=k_norm, positions=positions,
+                         eps=cfg.rms_norm_eps, one_plus_w=True)
     # the element-wise sigmoid gate is applied inside the attention kernel's final write
     o = decode_attention(q, kn, v.reshape(B, Hkv, D), cache.k, cache.v, pos_t, elem_gate=qg[..., D:])
     return o.reshape(B, 1, H * D)
@@ -410,6 +410,16 @@ def forward(m: Qwen35ForCausalLM, input_ids=None, attn_mask=None, inputs_embeds=
     return lin(forward_hidden(m, input_ids, attn_mask, inputs_embeds), m.lm_head)
 
 
+def _norm_products(f, x, norm, eps, ws):
+    """([h w^T for w in ws], the stream ``x + f``) with h the norm of the stream; rows [B, h], ``x`` None before the first layer."""
+    if skinny.norm_supported(f, norm, ws):
+        return skinny.skinny_norm_many(f, x, norm, eps, ws, one_plus_w=True)
+    if x is None:
+        return lin_many(rms(f, norm, eps), ws), f
+    h1, x = norm_w(f, norm, eps, one_plus_w=True, residual=x, return_residual=True)
+    return lin_many(h1, ws), x
+
+
 class HybridCache(HybridSession):
     """KV caches for full layers, conv + recurrent states for linear layers (Model.lean:784-860)."""
     name = "Qwen3.5"
@@ -464,24 +474,29 @@ class HybridCache(HybridSession):
         m, cfg = self.m, self.m.cfg
         eps = cfg.rms_norm_eps
         x = F.embedding(tok.reshape(-1, 1), m.embed_tokens)
-        n_layers = len(m.layers)
-        h1 = rms(x, m.layers[0].input_layernorm, eps)
+        B = x.shape[0]
+        f, x = x.reshape(B, -1), None                  # what is yet to be added to the stream, and the stream
         for i, l in enumerate(m.layers):
-            if cfg.is_full(i):
-                a = l.mixer
-                o = attention_core_decode(cfg, a.q_norm, a.k_norm, *lin_many(h1, (a.q_proj, a.k_proj, a.v_proj)), self.cos, self.sin, self.pos_t,
-                                          self.kv[i])
-                mixed = lin(o, a.o_proj)
+            full, a = cfg.is_full(i), l.mixer
+            ws = (a.q_proj, a.k_proj, a.v_proj) if full else (a.in_proj_qkv, a.in_proj_z, a.in_proj_b, a.in_proj_a)
+            parts, x = _norm_products(f, x, l.input_layernorm, eps, ws)
+            parts = [t.unsqueeze(1) for t in parts]
+            if full:
+                o = attention_core_decode(cfg, a.q_norm, a.k_norm, *parts, self.cos, self.sin, self.pos_t, self.kv[i])
+                mixed = lin(o, a.o_proj).reshape(B, -1)
             else:
-                mixed = gated_delta_net_forward(cfg, l.mixer, h1, self.lin[i])
+                mixed = lin(gated_delta_net_core(cfg, a, *parts, self.lin[i]), a.out_proj).reshape(B, -1)
+            if isinstance(l.ffn, MLP) and skinny.norm_supported(mixed, l.post_attention_layernorm, (l.ffn.gate_proj, l.ffn.up_proj)) \
+                    and skinny.swiglu_supported(mixed, l.ffn.gate_proj, l.ffn.up_proj):
+                act, x = skinny.skinny_norm_swiglu(mixed, x, l.post_attention_layernorm, eps, l.ffn.gate_proj, l.ffn.up_proj, one_plus_w=True)
+                f = lin(act, l.ffn.down_proj)
+                continue
             # residual add and the next norm in one kernel: (normed, new residual stream)
-            h3, h2 = norm_w(mixed, l.post_attention_layernorm, eps, one_plus_w=True, residual=x, return_residual=True)
-            f = swiglu_mlp(h3, l.ffn.gate_proj, l.ffn.up_proj, l.ffn.down_proj) if isinstance(l.ffn, MLP) else \
-                moe_forward(cfg, l.ffn, h3.reshape(-1, cfg.hidden_size)).reshape(h3.shape)
-            next_w = m.layers[i + 1].input_layernorm if i + 1 < n_layers else m.norm
-            h1, x = norm_w(f, next_w, eps, one_plus_w=True, residual=h2, return_residual=True)
+            h3, x = norm_w(mixed, l.post_attention_layernorm, eps, one_plus_w=True, residual=x, return_residual=True)
+            f = swiglu_mlp(h3, l.ffn.gate_proj, l.ffn.up_proj, l.ffn.down_proj) if isinstance(l.ffn, MLP) else moe_forward(cfg, l.ffn, h3)
+        h1, _ = norm_w(f, m.norm, eps, one_plus_w=True, residual=x, return_residual=True)
         self.pos_t += 1
-        return lin(h1[:, -1], m.lm_head)
+        return lin(h1, m.lm_head)
 
 
 def generate(m: Qwen35ForCausalLM, input_ids, max_new_tokens=64, strategy=SamplingStrategy(), eos_token_ids=None, on_step=None):

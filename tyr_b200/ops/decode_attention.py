@@ -36,9 +36,11 @@ def _sigs(lib_):
 
 
 def pick_splits(B: int, Hkv: int, keys: int) -> int:
-    """Enough CTAs to fill 148 SMs a few times over, but at least 256 keys per split."""
-    want = -(-592 // max(1, B * Hkv))
-    return max(1, min(want, 32, -(-keys // 256)))
+    """Enough CTAs to fill 148 SMs about twice, with at least 64 keys a split and 32 splits at most.  Us at 1 / 2 / 3 / 9 / 16 splits: one row of 2 K/V heads of
+    256 over 564 keys 21.1 / 18.1 / 15.8 / 13.4 / 14.0, over 4096 keys 167 / 92 / 67 / 33 / 23; 32 rows of 4 K/V heads of 256 over 576 keys
+    41.8 / 38.2 / 49.6 / 68.0 / 88.6; 16 rows of 2 over 2048 keys 93.5 / 54.5 / 43.9 / 30.3 / 36.5."""
+    want = 296 // max(1, B * Hkv)
+    return max(1, min(want, 32, -(-keys // 64)))
 
 
 def geometry_supported(Hq: int, Hkv: int, D: int) -> bool:

@@ -7,6 +7,7 @@ and the value-embedding blend ``v = (1-m) v + m ve`` (Examples/NanoChat/ModdedGP
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional
 
 import torch
@@ -126,3 +127,22 @@ def rope_norm(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, *, weight=N
     x1, x2 = xf[..., :hr], xf[..., hr:rot]
     out = torch.cat([x1 * c - x2 * s, x1 * s + x2 * c, xf[..., rot:]], dim=-1)
     return out.to(x.dtype)
+
+
+def rope_norm_qk(q: torch.Tensor, k: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, *, q_weight: torch.Tensor, k_weight: torch.Tensor,
+                 positions: torch.Tensor, eps: float = EPS, one_plus_w: bool = False):
+    """:func:`rope_norm` of queries [rows, H, D] and keys [rows, G, D] in one launch; rows and heads may be strided."""
+    rot = 2 * cos.shape[1]
+    low = lambda t: t.dtype == torch.bfloat16 and t.is_contiguous()
+    if not (q.is_cuda and q.dtype == k.dtype == torch.bfloat16 and q.stride(2) == k.stride(2) == 1 and low(q_weight) and low(k_weight)
+            and cos.dtype == sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous() and positions.dtype == torch.int32):
+        kw = dict(positions=positions, rot=rot, eps=eps, one_plus_w=one_plus_w)
+        return rope_norm(q, cos, sin, weight=q_weight, **kw), rope_norm(k, cos, sin, weight=k_weight, **kw)
+    rows, H, D = q.shape
+    G, dev = k.shape[1], q.device
+    qo, ko = torch.empty((rows, H, D), dtype=q.dtype, device=dev), torch.empty((rows, G, D), dtype=q.dtype, device=dev)
+    strides = (ctypes.c_longlong * 4)(q.stride(0), q.stride(1), k.stride(0), k.stride(1))
+    pos = positions.contiguous()
+    check(lib().tyr_rope_norm_qk(ptr(q), ptr(k), ptr(qo), ptr(ko), ptr(q_weight), ptr(k_weight), ptr(cos), ptr(sin), ptr(pos), strides, rows, cos.shape[0], H, G, D,
+                                 rot, eps, 1 if one_plus_w else 0, cur_stream(dev)), "rope_norm_qk")
+    return qo, ko

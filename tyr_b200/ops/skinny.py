@@ -25,7 +25,9 @@ def _sigs(lib_):
     for name, args in (("tyr_skinny_gemm_act_bf16", [P, P, P, P, L, L, L, I, I, I, I, F, F, P]),
                        ("tyr_skinny_heads_bf16", [P, P, P, L, L, L, L, L, L, I, I, I, I, P]),
                        ("tyr_skinny_gelu_mul_bf16", [P, P, P, P, L, L, L, L, I, I, I, P]),
-                       ("tyr_skinny_many_bf16", [P, L, I, P, P, P, P, P, I, I, I, P])):
+                       ("tyr_skinny_many_bf16", [P, L, I, P, P, P, P, P, I, I, I, P]),
+                       ("tyr_skinny_norm_many_bf16", [P, P, P, P, L, L, I, P, P, P, P, P, I, I, F, I, P]),
+                       ("tyr_skinny_norm_swiglu_bf16", [P, P, P, P, L, L, P, P, P, L, I, I, I, F, I, P])):
         fn = getattr(lib_, name, None)
         if fn is not None:
             fn.argtypes, fn.restype = args, I
@@ -79,6 +81,47 @@ def skinny_many(x2: torch.Tensor, ws: Sequence[torch.Tensor], splits: int = 0) -
     check(lib().tyr_skinny_many_bf16(ptr(x2), x2.stride(0), n, P(*[w.data_ptr() for w in ws]), P(*[y.data_ptr() for y in ys]), L(*[w.stride(0) for w in ws]),
                                      L(*[y.stride(0) for y in ys]), I(*[w.shape[0] for w in ws]), M, K, splits, cur_stream(x2.device)), "skinny_many")
     return ys
+
+
+NORM_NUMBERS = 16384       # of the normalised rows that a CTA of the forms below keeps
+
+
+def norm_supported(x2: torch.Tensor, norm_w: torch.Tensor, ws: Sequence[torch.Tensor]) -> bool:
+    """Up to 8 rows whose norm every CTA of the products takes again."""
+    M, K = x2.shape
+    return (len(ws) <= MAX_MATRICES and M <= 8 and M * (K + 8) <= NORM_NUMBERS and all(supported(x2, w) and w.shape[1] == K for w in ws)
+            and norm_w.dtype == torch.bfloat16 and norm_w.is_contiguous() and norm_w.data_ptr() % 16 == 0 and norm_w.numel() == K)
+
+
+def _norm_operands(x2, resid):
+    M, K = x2.shape
+    r = None if resid is None else resid if resid.stride(1) == 1 and resid.stride(0) % 8 == 0 and resid.data_ptr() % 16 == 0 else resid.contiguous()
+    return r, None if r is None else torch.empty((M, K), dtype=x2.dtype, device=x2.device), 0 if r is None else r.stride(0)
+
+
+def skinny_norm_many(x2: torch.Tensor, resid: Optional[torch.Tensor], norm_w: torch.Tensor, eps: float, ws: Sequence[torch.Tensor], one_plus_w: bool = False):
+    """``([h w^T for w in ws], s)`` with ``s = x2 + resid`` (bf16; x2 itself without ``resid``) and h its RMS norm times the gain, in one launch."""
+    M, K = x2.shape
+    r, out, ldr = _norm_operands(x2, resid)
+    n = len(ws)
+    ys = [torch.empty((M, w.shape[0]), dtype=torch.bfloat16, device=x2.device) for w in ws]
+    P, L, I = ctypes.c_void_p * n, ctypes.c_longlong * n, ctypes.c_int * n
+    check(lib().tyr_skinny_norm_many_bf16(ptr(x2), ptr(r), ptr(norm_w), ptr(out), x2.stride(0), ldr, n, P(*[w.data_ptr() for w in ws]),
+                                          P(*[y.data_ptr() for y in ys]), L(*[w.stride(0) for w in ws]), L(*[y.stride(0) for y in ys]),
+                                          I(*[w.shape[0] for w in ws]), M, K, eps, 1 if one_plus_w else 0, cur_stream(x2.device)), "skinny_norm_many")
+    return ys, x2 if out is None else out
+
+
+def skinny_norm_swiglu(x2: torch.Tensor, resid: Optional[torch.Tensor], norm_w: torch.Tensor, eps: float, gate_w: torch.Tensor, up_w: torch.Tensor,
+                       one_plus_w: bool = False):
+    """``(silu(h gate_w^T) * (h up_w^T), s)`` with h and s as in :func:`skinny_norm_many`."""
+    M, K = x2.shape
+    N = gate_w.shape[0]
+    r, out, ldr = _norm_operands(x2, resid)
+    y = torch.empty((M, N), dtype=torch.bfloat16, device=x2.device)
+    check(lib().tyr_skinny_norm_swiglu_bf16(ptr(x2), ptr(r), ptr(norm_w), ptr(out), x2.stride(0), ldr, ptr(gate_w), ptr(up_w), ptr(y), gate_w.stride(0), M, N, K,
+                                            eps, 1 if one_plus_w else 0, cur_stream(x2.device)), "skinny_norm_swiglu")
+    return y, x2 if out is None else out
 
 
 _SWIGLU = os.environ.get("TYR_SKINNY_SWIGLU", "1") != "0"
