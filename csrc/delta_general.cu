@@ -259,38 +259,54 @@ __global__ void __launch_bounds__(256) gated_norm_kernel(const float* __restrict
 }
 
 // The same with SiLU on a read-out that the chunk scan left in bf16, the gain in bf16: half a warp per (row, head) up to 128 channels, else a
-// warp, 16 bytes a lane.  Bound by memory traffic; as library calls it was seven passes in fp32.
+// warp, 16 bytes a lane, one block per row.  Bound by memory traffic: 8192 rows of 48 heads of 128 took 113 us with one head in flight and positions from
+// 64-bit divisions, 81 now; as library calls it was seven passes in fp32.
 __global__ void __launch_bounds__(256) gated_norm_rounded_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ z, long long ld_z,
-                                                                 const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, long long units,
-                                                                 int Hv, int dv, float eps) {
+                                                                 const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int Hv, int dv,
+                                                                 float eps) {
   pdl_entry();
   const int group = dv <= 128 ? 16 : 32, d = (threadIdx.x & (group - 1)) * 8;
   const bool live = d < dv;
-  const long long per_block = 256 / group;
-  for (long long u = blockIdx.x * per_block + threadIdx.x / group; u < (units + per_block - 1) / per_block * per_block; u += gridDim.x * per_block) {
-    const bool ok = live && u < units;
-    float x[8] = {}, g[8] = {}, wv[8] = {};
-    if (ok) {
-      const uint4 a = *reinterpret_cast<const uint4*>(o + u * dv + d), b = *reinterpret_cast<const uint4*>(z + u / Hv * ld_z + u % Hv * dv + d),
-                  c = *reinterpret_cast<const uint4*>(w + d);
-      const uint32_t ua[4] = {a.x, a.y, a.z, a.w}, ub[4] = {b.x, b.y, b.z, b.w}, uc[4] = {c.x, c.y, c.z, c.w};
+  const int at_once = 256 / group;
+  const __nv_bfloat16* o_row = o + static_cast<long long>(blockIdx.x) * Hv * dv;
+  const __nv_bfloat16* z_row = z + blockIdx.x * ld_z;
+  __nv_bfloat16* y_row = y + static_cast<long long>(blockIdx.x) * Hv * dv;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const uint4 uw = live ? *reinterpret_cast<const uint4*>(w + d) : zero;
+  constexpr int U = 3;                     // heads of a group whose loads are in flight together
+  for (int h0 = threadIdx.x / group; h0 < (Hv + at_once - 1) / at_once * at_once; h0 += U * at_once) {
+    uint4 uo[U], uz[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int h = h0 + u * at_once;
+      const bool ok = live && h < Hv;
+      uo[u] = ok ? *reinterpret_cast<const uint4*>(o_row + h * dv + d) : zero;
+      uz[u] = ok ? *reinterpret_cast<const uint4*>(z_row + h * dv + d) : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int h = h0 + u * at_once;
+      const uint32_t ua[4] = {uo[u].x, uo[u].y, uo[u].z, uo[u].w}, ub[4] = {uz[u].x, uz[u].y, uz[u].z, uz[u].w}, uc[4] = {uw.x, uw.y, uw.z, uw.w};
+      float x[8], ss = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float2 fa = unpack_bf16x2(ua[j]), fb = unpack_bf16x2(ub[j]), fc = unpack_bf16x2(uc[j]);
-        x[2 * j] = fa.x; x[2 * j + 1] = fa.y;
-        g[2 * j] = fb.x; g[2 * j + 1] = fb.y;
-        wv[2 * j] = fc.x; wv[2 * j + 1] = fc.y;
+        const float2 f = unpack_bf16x2(ua[j]);
+        x[2 * j] = f.x;
+        x[2 * j + 1] = f.y;
+        ss += f.x * f.x + f.y * f.y;
       }
+      for (int m = group >> 1; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+      const float rstd = rsqrtf(ss / dv + eps);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 g = unpack_bf16x2(ub[j]), c = unpack_bf16x2(uc[j]);
+        // the result is rounded to bf16: the approximate exponential and quotient, 1e-6 off, decide nothing (precise ones bound the kernel)
+        x[2 * j] = x[2 * j] * rstd * c.x * __fdividef(g.x, 1.f + __expf(-g.x));
+        x[2 * j + 1] = x[2 * j + 1] * rstd * c.y * __fdividef(g.y, 1.f + __expf(-g.y));
+      }
+      if (live && h < Hv)
+        *reinterpret_cast<uint4*>(y_row + h * dv + d) = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
     }
-    float ss = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) ss += x[j] * x[j];
-    for (int m = group >> 1; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
-    const float rstd = 1.f / sqrtf(ss / dv + eps);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = x[j] * rstd * wv[j] * dg_gate(g[j], 0);
-    if (ok)
-      *reinterpret_cast<uint4*>(y + u * dv + d) = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
   }
 }
 
@@ -459,9 +475,8 @@ extern "C" TYR_EXPORT int tyr_gated_norm(const float* o, const void* z, long lon
 // y = o / rms(o) * w * silu(z) per head, all bf16: o and y [rows, Hv, dv] contiguous, z rows of stride ld_z; dv a multiple of 8 up to 256.
 extern "C" TYR_EXPORT int tyr_gated_norm_rounded(const void* o, const void* z, long long ld_z, const void* w, void* y, long long rows, int Hv, int dv,
                                                  float eps, void* stream) {
-  if (rows <= 0 || Hv <= 0 || dv < 8 || dv > 256 || (dv & 7) || (ld_z & 7)) return -1;
+  if (rows <= 0 || rows > 0x7fffffff || Hv <= 0 || dv < 8 || dv > 256 || (dv & 7) || (ld_z & 7)) return -1;
   if ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) return -2;
-  const long long units = rows * Hv, per_block = dv <= 128 ? 16 : 8, want = (units + per_block - 1) / per_block;
-  return (int)launch_dependent(gated_norm_rounded_kernel, dim3(static_cast<unsigned>(want < 148LL * 16 ? want : 148LL * 16)), dim3(256), 0, (cudaStream_t)stream,
-                               (const __nv_bfloat16*)o, (const __nv_bfloat16*)z, ld_z, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, units, Hv, dv, eps);
+  return (int)launch_dependent(gated_norm_rounded_kernel, dim3(static_cast<unsigned>(rows)), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)o,
+                               (const __nv_bfloat16*)z, ld_z, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, Hv, dv, eps);
 }

@@ -1117,74 +1117,71 @@ __global__ void __launch_bounds__(256, 2) gdr_chunk_prepare_channel_kernel(GdrPr
 
 // Causal depthwise conv1d (kernel taps K <= 4, zero history) + bias + SiLU on channels-last activations:
 //   y[b, s, c] = silu(bias[c] + sum_j w[c, j] * x[b, s - (K - 1) + j, c]).
-// A thread owns 8 channels (16 bytes) of CONV_TOK tokens and issues the loads of all their rows and of the K - 1 before them first; the
-// window is read again from cache by the thread of the next tokens.  Bound by memory traffic.  A sliding window of 32 tokens whose
-// loads waited for one another took 21.8 us for 333 tokens of 6144 channels; this form 11.7 us, the wait for the product in front of it included.  The thread of the last tokens also leaves the last K inputs of its channels in `window` ([B, C, K], zeros
-// before the start), where a decoding step goes on.  The reference transposes to channels-first
+// A thread owns 4 channels (8 bytes) of CONV_TOK tokens and issues the loads of all their rows and of the K - 1 before them first; the
+// window is read again from cache by the thread of the next tokens.  Bound by the memory traffic that its registers let fly: with 8 channels a thread one block
+// stayed on an SM and 4 x 2048 tokens of 10240 channels took 173 us, 100 now.  A sliding window of 32 tokens whose
+// loads waited for one another took 21.8 us for 333 tokens of 6144 channels.  The thread of the last tokens also leaves the last K inputs of its channels in
+// `window` ([B, C, K], zeros before the start), where a decoding step goes on.  The reference transposes to channels-first
 // and calls the library's grouped convolution (Tyr/Model/Qwen35/Model.lean:642-700).
 namespace tyr {
-constexpr int CONV_TOK = 8;
+constexpr int CONV_TOK = 8, CONV_CH = 4;
+template <typename W>
+__device__ __forceinline__ void conv_load4(const W* p, float (&f)[CONV_CH]) {
+  if constexpr (sizeof(W) == 2) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y);
+    f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+  } else {
+    const float4 u = *reinterpret_cast<const float4*>(p);
+    f[0] = u.x; f[1] = u.y; f[2] = u.z; f[3] = u.w;
+  }
+}
 template <int K, typename W>
-__global__ void __launch_bounds__(256) causal_conv1d_silu_kernel(const __nv_bfloat16* __restrict__ x, const W* __restrict__ w,
-                                                                 const W* __restrict__ bias, __nv_bfloat16* __restrict__ y,
-                                                                 __nv_bfloat16* __restrict__ window, long long total, int S, int C,
-                                                                 long long x_sb, long long x_ss) {
+__global__ void __launch_bounds__(256, 4) causal_conv1d_silu_kernel(const __nv_bfloat16* __restrict__ x, const W* __restrict__ w,
+                                                                    const W* __restrict__ bias, __nv_bfloat16* __restrict__ y,
+                                                                    __nv_bfloat16* __restrict__ window, int groups, int S, int C,
+                                                                    long long x_sb, long long x_ss) {
   pdl_entry();
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int c8 = C >> 3;
-  const int c = static_cast<int>(i % c8) * 8;
-  const long long bt = i / c8;
-  const int nblk = (S + CONV_TOK - 1) / CONV_TOK;
-  const int s0 = static_cast<int>(bt % nblk) * CONV_TOK;
-  const long long b = bt / nblk;
+  const int gi = blockIdx.x * blockDim.x + threadIdx.x;          // group of channels
+  if (gi >= groups) return;
+  const int c = gi * CONV_CH, s0 = blockIdx.y * CONV_TOK;
+  const long long b = blockIdx.z;
   const __nv_bfloat16* xb = x + b * x_sb + c;
-  uint4 rows[CONV_TOK + K - 1];                      // inputs s0 - (K - 1) .. s0 + CONV_TOK - 1
+  uint2 rows[CONV_TOK + K - 1];                      // inputs s0 - (K - 1) .. s0 + CONV_TOK - 1
 #pragma unroll
   for (int r = 0; r < CONV_TOK + K - 1; ++r) {
     const int t = s0 - (K - 1) + r;
-    rows[r] = (t >= 0 && t < S) ? *reinterpret_cast<const uint4*>(xb + static_cast<long long>(t) * x_ss) : make_uint4(0u, 0u, 0u, 0u);
+    rows[r] = (t >= 0 && t < S) ? *reinterpret_cast<const uint2*>(xb + static_cast<long long>(t) * x_ss) : make_uint2(0u, 0u);
   }
-  float wt[8][K], bs[8];
+  float taps[K][CONV_CH], bs[CONV_CH] = {};          // the 4 K numbers at w + c K in their order: tap (channel, j) is number channel * K + j
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    bs[e] = bias ? static_cast<float>(bias[c + e]) : 0.f;
-#pragma unroll
-    for (int j = 0; j < K; ++j) wt[e][j] = static_cast<float>(w[(c + e) * K + j]);
-  }
+  for (int j = 0; j < K; ++j) conv_load4(w + static_cast<long long>(c) * K + j * CONV_CH, taps[j]);
+  if (bias != nullptr) conv_load4(bias + c, bs);
 #pragma unroll
   for (int s = 0; s < CONV_TOK; ++s) {
     if (s0 + s >= S) break;
-    float acc[8];
+    float acc[CONV_CH];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = bs[e];
+    for (int e = 0; e < CONV_CH; ++e) acc[e] = bs[e];
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      const uint32_t uu[4] = {rows[s + j].x, rows[s + j].y, rows[s + j].z, rows[s + j].w};
+      const float2 p0 = unpack_bf16x2(rows[s + j].x), p1 = unpack_bf16x2(rows[s + j].y);
+      const float f[CONV_CH] = {p0.x, p0.y, p1.x, p1.y};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = unpack_bf16x2(uu[e]);
-        acc[2 * e] += f.x * wt[2 * e][j];
-        acc[2 * e + 1] += f.y * wt[2 * e + 1][j];
-      }
+      for (int e = 0; e < CONV_CH; ++e) acc[e] += f[e] * taps[(e * K + j) / CONV_CH][(e * K + j) % CONV_CH];
     }
-    uint4 o;
-    uint32_t* oo = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float a0 = acc[2 * e], a1 = acc[2 * e + 1];
-      oo[e] = pack_bf16x2(a0 / (1.f + __expf(-a0)), a1 / (1.f + __expf(-a1)));
-    }
-    *reinterpret_cast<uint4*>(y + (b * S + s0 + s) * C + c) = o;
+    for (int e = 0; e < CONV_CH; ++e) acc[e] = acc[e] / (1.f + __expf(-acc[e]));
+    *reinterpret_cast<uint2*>(y + (b * S + s0 + s) * C + c) = make_uint2(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]));
   }
   if (window != nullptr && s0 + CONV_TOK >= S) {
 #pragma unroll
     for (int j = 0; j < K; ++j) {
       const int t = S - K + j;
-      const uint4 u = t >= 0 ? *reinterpret_cast<const uint4*>(xb + static_cast<long long>(t) * x_ss) : make_uint4(0u, 0u, 0u, 0u);
-      const uint32_t uu[4] = {u.x, u.y, u.z, u.w};
+      const uint2 u = t >= 0 ? *reinterpret_cast<const uint2*>(xb + static_cast<long long>(t) * x_ss) : make_uint2(0u, 0u);
+      const uint32_t uu[2] = {u.x, u.y};
 #pragma unroll
-      for (int e = 0; e < 8; ++e)
+      for (int e = 0; e < CONV_CH; ++e)
         window[(b * C + c + e) * K + j] = __ushort_as_bfloat16(static_cast<unsigned short>(uu[e >> 1] >> ((e & 1) * 16)));
     }
   }
@@ -1193,9 +1190,9 @@ __global__ void __launch_bounds__(256) causal_conv1d_silu_kernel(const __nv_bflo
 template <int K, typename W>
 static cudaError_t conv_launch(const void* x, const void* w, const void* bias, void* y, void* window, int B, int S, int C, long long x_sb,
                                long long x_ss, cudaStream_t st) {
-  const long long total = static_cast<long long>(B) * ((S + CONV_TOK - 1) / CONV_TOK) * (C >> 3);
-  return launch_dependent(causal_conv1d_silu_kernel<K, W>, dim3(static_cast<unsigned>((total + 255) / 256)), dim3(256), 0, st, (const __nv_bfloat16*)x,
-                          (const W*)w, (const W*)bias, (__nv_bfloat16*)y, (__nv_bfloat16*)window, total, S, C, x_sb, x_ss);
+  const int groups = C / CONV_CH;
+  return launch_dependent(causal_conv1d_silu_kernel<K, W>, dim3((groups + 255) / 256, (S + CONV_TOK - 1) / CONV_TOK, B), dim3(256), 0, st, (const __nv_bfloat16*)x,
+                          (const W*)w, (const W*)bias, (__nv_bfloat16*)y, (__nv_bfloat16*)window, groups, S, C, x_sb, x_ss);
 }
 }  // namespace tyr
 
@@ -1203,8 +1200,8 @@ static cudaError_t conv_launch(const void* x, const void* w, const void* bias, v
 extern "C" TYR_EXPORT int tyr_causal_conv1d_silu(const void* x, const void* w, const void* bias, void* y, void* window, int B, int S, int C,
                                                  int K, long long x_sb, long long x_ss, int w_bf16, void* stream) {
   using namespace tyr;
-  if (B <= 0 || S <= 0 || C <= 0 || (C & 7) || K <= 0 || K > 4 || (x_sb & 7) || (x_ss & 7)) return -1;
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) return -2;
+  if (B <= 0 || B > 65535 || S <= 0 || S > 65535 * CONV_TOK || C <= 0 || (C & 7) || K <= 0 || K > 4 || (x_sb & 7) || (x_ss & 7)) return -1;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(bias)) & 15) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 #define TYR_CONV(k) \
   case k: return (int)(w_bf16 ? conv_launch<k, __nv_bfloat16>(x, w, bias, y, window, B, S, C, x_sb, x_ss, st) : conv_launch<k, float>(x, w, bias, y, window, B, S, C, x_sb, x_ss, st))

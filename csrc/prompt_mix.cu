@@ -3,9 +3,11 @@
 //     store, where attention reads them;
 //   * attention_gate:     the attention output times sigmoid of the gate that the query projection carries beside each head.
 //
-// Both are bound by memory traffic: every operand passes through once, 16 bytes a lane, one warp per (token, head).  As library calls
+// Both are bound by memory traffic: every operand passes through once, 16 bytes a lane, one block per token (a warp takes several heads, whose
+// loads are in flight together; with one head a warp and positions from 64-bit divisions the gate took 96 us for 8192 tokens of 24
+// heads of 256, and takes 53).  As library calls
 // they were 27 passes over the same rows (contiguous copies, conversions, norms, concatenations, store writes).
-// Compiled without fast math.  A prompt of 333 tokens through Qwen3.5 0.8B took 1007 launches and 13.4 ms (6.3 ms of it on the GPU) and takes 414 and
+// A prompt of 333 tokens through Qwen3.5 0.8B took 1007 launches and 13.4 ms (6.3 ms of it on the GPU) and takes 414 and
 // 8.7 ms (4.6) with these and the fused passes of csrc/delta_rule.cu and csrc/delta_general.cu; 4 x 2048 tokens through 8 layers of the 27B widths 61.6 and 55.6 ms.
 #include "common.cuh"
 
@@ -37,44 +39,71 @@ struct OperandArgs {
 };
 
 // Lane l keeps channels 8 l .. 8 l + 7 of a head (D <= 256), and the channels that rotate with them are half / 8 lanes away.
-__global__ void __launch_bounds__(256) attention_operands_kernel(OperandArgs a) {
+__global__ void __launch_bounds__(256, 3) attention_operands_kernel(OperandArgs a) {
   pdl_entry();
   const int lane = threadIdx.x & 31, heads = a.H + 2 * a.G, d = lane * 8, shift = a.half >> 3;
-  const bool live = d < a.D;
-  const long long total = static_cast<long long>(a.B) * a.S * heads;
-  for (long long i = blockIdx.x * 8LL + (threadIdx.x >> 5); i < total; i += gridDim.x * 8LL) {
-    const int h = static_cast<int>(i % heads);
-    const long long row = i / heads;
-    const int b = static_cast<int>(row / a.S), s = static_cast<int>(row % a.S);
-    const bool is_q = h < a.H, is_v = h >= a.H + a.G;
-    const int g = is_q ? h : (is_v ? h - a.H - a.G : h - a.H);
-    const __nv_bfloat16* src = is_q ? a.q + row * a.q_row + g * a.q_head : (is_v ? a.v + row * a.v_row : a.k + row * a.k_row) + static_cast<long long>(g) * a.D;
-    __nv_bfloat16* dst = is_q ? a.q_out + (row * a.H + g) * a.D
-                              : (is_v ? a.v_store : a.k_store) + ((static_cast<long long>(b) * a.G + g) * a.cap + a.slot0 + s) * a.D;
-    if (is_v) {
-      if (live) *reinterpret_cast<uint4*>(dst + d) = *reinterpret_cast<const uint4*>(src + d);
-      continue;
-    }
-    float x[8] = {}, w[8] = {};
-    if (live) {
-      pm_load8(src + d, x);
-      pm_load8((is_q ? a.qw : a.kw) + d, w);
-    }
-    float ss = 0.f;
+  const int s = blockIdx.x, b = blockIdx.y;
+  const long long row = static_cast<long long>(b) * a.S + s;
+  const bool live = d < a.D, first = d < a.half, second = !first && d < 2 * a.half;
+  const int partner = first ? lane + shift : second ? lane - shift : lane;
+  float c[8] = {}, sn[8] = {};
+  uint4 qw = make_uint4(0u, 0u, 0u, 0u), kw = qw;
+  if (first || second) {
+    const long long at = static_cast<long long>(s) * a.half + (first ? d : d - a.half);      // half and d are multiples of 8
+    const float4 c0 = *reinterpret_cast<const float4*>(a.cosT + at), c1 = *reinterpret_cast<const float4*>(a.cosT + at + 4);
+    const float4 s0 = *reinterpret_cast<const float4*>(a.sinT + at), s1 = *reinterpret_cast<const float4*>(a.sinT + at + 4);
+    c[0] = c0.x; c[1] = c0.y; c[2] = c0.z; c[3] = c0.w; c[4] = c1.x; c[5] = c1.y; c[6] = c1.z; c[7] = c1.w;
+    sn[0] = s0.x; sn[1] = s0.y; sn[2] = s0.z; sn[3] = s0.w; sn[4] = s1.x; sn[5] = s1.y; sn[6] = s1.z; sn[7] = s1.w;
+  }
+  if (live) {
+    qw = *reinterpret_cast<const uint4*>(a.qw + d);
+    kw = *reinterpret_cast<const uint4*>(a.kw + d);
+  }
+  constexpr int U = 4;                     // heads of a warp whose loads are in flight together
+  for (int h0 = threadIdx.x >> 5; h0 < heads; h0 += 8 * U) {
+    uint4 in[U];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) ss += x[j] * x[j];
-    const float rstd = 1.f / sqrtf(warp_sum(ss) / a.D + a.eps);
-    const bool first = d < a.half, second = !first && d < 2 * a.half;
-    const int partner = first ? lane + shift : second ? lane - shift : lane;
-    const float* c = a.cosT + static_cast<long long>(s) * a.half + (first ? d : d - a.half);
-    const float* sn = a.sinT + static_cast<long long>(s) * a.half + (first ? d : d - a.half);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      x[j] = x[j] * rstd * (1.f + w[j]);
-      const float other = __shfl_sync(0xffffffffu, x[j], partner);
-      w[j] = first ? x[j] * c[j] - other * sn[j] : second ? x[j] * c[j] + other * sn[j] : x[j];
+    for (int u = 0; u < U; ++u) {
+      const int h = h0 + 8 * u;
+      const __nv_bfloat16* src = h < a.H ? a.q + row * a.q_row + h * a.q_head
+                                         : h < a.H + a.G ? a.k + row * a.k_row + static_cast<long long>(h - a.H) * a.D
+                                                         : a.v + row * a.v_row + static_cast<long long>(h - a.H - a.G) * a.D;
+      in[u] = live && h < heads ? *reinterpret_cast<const uint4*>(src + d) : make_uint4(0u, 0u, 0u, 0u);
     }
-    if (live) pm_store8(dst + d, w);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int h = h0 + 8 * u;
+      if (h >= heads) break;
+      const bool is_q = h < a.H, is_v = h >= a.H + a.G;
+      const int g = is_q ? h : (is_v ? h - a.H - a.G : h - a.H);
+      __nv_bfloat16* dst = is_q ? a.q_out + (row * a.H + g) * a.D
+                                : (is_v ? a.v_store : a.k_store) + ((static_cast<long long>(b) * a.G + g) * a.cap + a.slot0 + s) * a.D;
+      if (is_v) {
+        if (live) *reinterpret_cast<uint4*>(dst + d) = in[u];
+        continue;
+      }
+      const uint32_t words[4] = {in[u].x, in[u].y, in[u].z, in[u].w};
+      float x[8], y[8];
+      float ss = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = unpack_bf16x2(words[j]);
+        x[2 * j] = f.x;
+        x[2 * j + 1] = f.y;
+        ss += f.x * f.x + f.y * f.y;
+      }
+      const float rstd = rsqrtf(warp_sum(ss) / a.D + a.eps);
+      const uint4 gain = is_q ? qw : kw;
+      const uint32_t gains[4] = {gain.x, gain.y, gain.z, gain.w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float2 gj = unpack_bf16x2(gains[j >> 1]);
+        x[j] = x[j] * rstd * (1.f + (j & 1 ? gj.y : gj.x));
+        const float other = __shfl_sync(0xffffffffu, x[j], partner);
+        y[j] = first ? x[j] * c[j] - other * sn[j] : second ? x[j] * c[j] + other * sn[j] : x[j];
+      }
+      if (live) pm_store8(dst + d, y);
+    }
   }
 }
 
@@ -88,24 +117,21 @@ struct GateOutArgs {
 
 __global__ void __launch_bounds__(256) attention_gate_kernel(GateOutArgs a) {
   pdl_entry();
-  const int vecs = a.D >> 3;
-  const long long total = a.rows * a.H * vecs;
-  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
-    const int d = static_cast<int>(i % vecs) * 8;
-    const long long t = i / vecs, row = t / a.H;
-    const int h = static_cast<int>(t % a.H);
+  const int vecs = a.D >> 3, n = a.H * vecs;
+  const long long row = blockIdx.x;
+  const __nv_bfloat16* o_row = a.o + row / a.S * a.o_b + row % a.S * a.o_s;
+  const __nv_bfloat16* g_row = a.gate + row * a.gate_row;
+  __nv_bfloat16* y_row = a.y + row * a.H * a.D;
+#pragma unroll 3
+  for (int i = threadIdx.x; i < n; i += 256) {
+    const int h = i / vecs, d = i % vecs * 8;
     float o[8], g[8];
-    pm_load8(a.o + row / a.S * a.o_b + row % a.S * a.o_s + h * a.o_h + d, o);
-    pm_load8(a.gate + row * a.gate_row + h * a.gate_head + d, g);
+    pm_load8(o_row + h * a.o_h + d, o);
+    pm_load8(g_row + h * a.gate_head + d, g);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] *= 1.f / (1.f + expf(-g[j]));
-    pm_store8(a.y + t * a.D + d, o);
+    for (int j = 0; j < 8; ++j) o[j] = __fdividef(o[j], 1.f + __expf(-g[j]));     // a gate of -inf: 0, like the quotient
+    pm_store8(y_row + i * 8, o);
   }
-}
-
-inline unsigned pm_grid(long long units, int per_block) {
-  const long long want = (units + per_block - 1) / per_block;
-  return static_cast<unsigned>(want < 148LL * 16 ? want : 148LL * 16);
 }
 
 }  // namespace tyr
@@ -120,22 +146,22 @@ extern "C" TYR_EXPORT int tyr_attention_operands(const void* q, const void* k, c
   OperandArgs a{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, strides[0], strides[1], strides[2], strides[3],
                 (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, cosT, sinT, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_store, (__nv_bfloat16*)v_store,
                 dims[0], dims[1], dims[2], dims[3], dims[4], dims[5], dims[6], dims[7], eps};
-  if (a.B < 1 || a.S < 1 || a.H < 1 || a.G < 1 || a.D < 8 || a.D > 256 || (a.D & 7) || a.half < 8 || (a.half & 7) || 2 * a.half > a.D) return -1;
+  if (a.B < 1 || a.B > 65535 || a.S < 1 || a.H < 1 || a.G < 1 || a.D < 8 || a.D > 256 || (a.D & 7) || a.half < 8 || (a.half & 7) || 2 * a.half > a.D) return -1;
   if (a.slot0 < 0 || a.slot0 + static_cast<long long>(a.S) > a.cap) return -2;
   if ((a.q_row | a.k_row | a.v_row | a.q_head) & 7) return -3;
-  for (const void* p : {q, k, v, qw, kw, (const void*)q_out, (const void*)k_store, (const void*)v_store})
+  for (const void* p : {q, k, v, qw, kw, (const void*)cosT, (const void*)sinT, (const void*)q_out, (const void*)k_store, (const void*)v_store})
     if (p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15)) return -4;
-  return (int)launch_dependent(attention_operands_kernel, dim3(pm_grid(1LL * a.B * a.S * (a.H + 2 * a.G), 8)), dim3(256), 0, (cudaStream_t)stream, a);
+  return (int)launch_dependent(attention_operands_kernel, dim3(a.S, a.B), dim3(256), 0, (cudaStream_t)stream, a);
 }
 
 // y [rows, H * D] = o * sigmoid(gate); o [rows / S, S, H, D] by (batch, token, head) strides, gate [rows, H, D] by (row, head) strides.
 extern "C" TYR_EXPORT int tyr_attention_gate(const void* o, const void* gate, const long long* strides, void* y, long long rows, int S, int H, int D,
                                              void* stream) {
-  if (rows < 1 || S < 1 || rows % S || H < 1 || D < 8 || (D & 7)) return -1;
+  if (rows < 1 || rows > 0x7fffffff || S < 1 || rows % S || H < 1 || D < 8 || (D & 7)) return -1;
   for (int i = 0; i < 5; ++i)
     if (strides[i] & 7) return -3;
   for (const void* p : {o, gate, (const void*)y})
     if (p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15)) return -4;
   const GateOutArgs a{(const __nv_bfloat16*)o, (const __nv_bfloat16*)gate, strides[0], strides[1], strides[2], strides[3], strides[4], (__nv_bfloat16*)y, rows, S, H, D};
-  return (int)launch_dependent(attention_gate_kernel, dim3(pm_grid(rows * H * (D / 8), 256)), dim3(256), 0, (cudaStream_t)stream, a);
+  return (int)launch_dependent(attention_gate_kernel, dim3(static_cast<unsigned>(rows)), dim3(256), 0, (cudaStream_t)stream, a);
 }

@@ -124,7 +124,8 @@ def chunk_gated_delta_rule_fused(q, k, v, g, beta, state: Optional[torch.Tensor]
     Hv, dv = v.shape[2], v.shape[3]
     n, BH, dev = (S + 63) // 64, B * Hv, q.device
     f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)
-    u, w, qg, kd, intra, glast = f32(BH, n, 64, -(-dv // 64) * 64), f32(BH, n, 64, 128), f32(BH, n, 64, 128), f32(BH, n, 64, 128), f32(BH, n, 64, 64), f32(BH, n)
+    rows = BH * n * 64                                                       # one scratch block: u, w, qg, kd, intra, glast
+    u, w, qg, kd, intra, glast = f32(rows * (-(-dv // 64) * 64 + 3 * 128 + 64) + BH * n).split((rows * (-(-dv // 64) * 64), rows * 128, rows * 128, rows * 128, rows * 64, BH * n))
     strides = (ctypes.c_longlong * 9)(*[t.stride(i) for t in (q, k, v) for i in range(3)])
     gc, bc = g.float().contiguous(), beta.float().contiguous()
     st = cur_stream(dev)
@@ -140,7 +141,7 @@ def chunk_gated_delta_rule_fused(q, k, v, g, beta, state: Optional[torch.Tensor]
 
 def _conv_kernel_ok(x: torch.Tensor, K: int) -> bool:
     return (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[2] % 8 == 0 and K <= 4 and x.stride(2) == 1 and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0
-            and x.data_ptr() % 16 == 0 and hasattr(lib(), "tyr_causal_conv1d_silu"))
+            and x.data_ptr() % 16 == 0 and x.shape[0] <= 65535 and x.shape[1] <= 8 * 65535 and hasattr(lib(), "tyr_causal_conv1d_silu"))
 
 
 def _conv_kernel(x, weight, bias, window):
@@ -150,6 +151,7 @@ def _conv_kernel(x, weight, bias, window):
     low = weight.dtype == torch.bfloat16 and (bias is None or bias.dtype == torch.bfloat16)      # taps in the activations' type are read as they are
     w = (weight.reshape(C, K) if low else weight.reshape(C, K).float()).contiguous()
     b = None if bias is None else (bias if low else bias.float()).contiguous()
+    w, b = (t if t is None or t.data_ptr() % 16 == 0 else t.clone() for t in (w, b))
     check(lib().tyr_causal_conv1d_silu(ptr(x), ptr(w), ptr(b), ptr(y), ptr(window), B, S, C, K, x.stride(0), x.stride(1), 1 if low else 0, cur_stream(x.device)),
           "causal_conv1d_silu")
     return y

@@ -29,7 +29,7 @@ def _rows(t: torch.Tensor) -> bool:
 def operands_supported(q, k, v, store, q_norm, k_norm, cos, D: int) -> bool:
     """q, k, v: projections [B, S, C]; ``store``: a plain ``KVCache`` of bf16 rows of D; cos: [S, half] fp32."""
     return (q.is_cuda and q.dtype == k.dtype == v.dtype == torch.bfloat16 and D % 8 == 0 and D <= 256 and cos.dim() == 2 and cos.dtype == torch.float32
-            and cos.is_contiguous() and cos.shape[1] % 8 == 0 and 0 < 2 * cos.shape[1] <= D and _rows(q) and _rows(k) and _rows(v)
+            and cos.is_contiguous() and cos.data_ptr() % 16 == 0 and cos.shape[1] % 8 == 0 and 0 < 2 * cos.shape[1] <= D and _rows(q) and _rows(k) and _rows(v)
             and store is not None and not store.ring and store.k.dtype == store.v.dtype == torch.bfloat16 and store.k.is_contiguous() and store.v.is_contiguous()
             and store.k.shape[0] == q.shape[0] and store.k.shape[3] == store.v.shape[3] == D and store.k.data_ptr() % 16 == 0 and store.v.data_ptr() % 16 == 0
             and q_norm.dtype == k_norm.dtype == torch.bfloat16 and q_norm.is_contiguous() and k_norm.is_contiguous()
