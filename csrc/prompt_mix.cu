@@ -4,8 +4,8 @@
 //   * attention_gate:     the attention output times sigmoid of the gate that the query projection carries beside each head.
 //
 // Both are bound by memory traffic: every operand passes through once, 16 bytes a lane, one block per token (a warp takes several heads, whose
-// loads are in flight together; with one head a warp and positions from 64-bit divisions the gate took 96 us for 8192 tokens of 24
-// heads of 256, and takes 53).  As library calls
+// loads are in flight together; with one head a warp and positions from 64-bit divisions the two took 174 and 96 us for 8192 tokens of 24
+// heads of 256, and take 100 and 53).  As library calls
 // they were 27 passes over the same rows (contiguous copies, conversions, norms, concatenations, store writes).
 // A prompt of 333 tokens through Qwen3.5 0.8B took 1007 launches and 13.4 ms (6.3 ms of it on the GPU) and takes 414 and
 // 8.7 ms (4.6) with these and the fused passes of csrc/delta_rule.cu and csrc/delta_general.cu; 4 x 2048 tokens through 8 layers of the 27B widths 61.6 and 55.6 ms.
@@ -41,69 +41,76 @@ struct OperandArgs {
 // Lane l keeps channels 8 l .. 8 l + 7 of a head (D <= 256), and the channels that rotate with them are half / 8 lanes away.
 __global__ void __launch_bounds__(256, 3) attention_operands_kernel(OperandArgs a) {
   pdl_entry();
-  const int lane = threadIdx.x & 31, heads = a.H + 2 * a.G, d = lane * 8, shift = a.half >> 3;
+  const int lane = threadIdx.x & 31, d = lane * 8, shift = a.half >> 3;
   const int s = blockIdx.x, b = blockIdx.y;
   const long long row = static_cast<long long>(b) * a.S + s;
   const bool live = d < a.D, first = d < a.half, second = !first && d < 2 * a.half;
   const int partner = first ? lane + shift : second ? lane - shift : lane;
-  float c[8] = {}, sn[8] = {};
-  uint4 qw = make_uint4(0u, 0u, 0u, 0u), kw = qw;
+  const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+  float c[8], sn[8];                       // cosine, and the sine with its partner's sign; channels that don't rotate: 1 and 0
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    c[j] = 1.f;
+    sn[j] = 0.f;
+  }
   if (first || second) {
     const long long at = static_cast<long long>(s) * a.half + (first ? d : d - a.half);      // half and d are multiples of 8
     const float4 c0 = *reinterpret_cast<const float4*>(a.cosT + at), c1 = *reinterpret_cast<const float4*>(a.cosT + at + 4);
     const float4 s0 = *reinterpret_cast<const float4*>(a.sinT + at), s1 = *reinterpret_cast<const float4*>(a.sinT + at + 4);
+    const float sign = first ? -1.f : 1.f;
     c[0] = c0.x; c[1] = c0.y; c[2] = c0.z; c[3] = c0.w; c[4] = c1.x; c[5] = c1.y; c[6] = c1.z; c[7] = c1.w;
-    sn[0] = s0.x; sn[1] = s0.y; sn[2] = s0.z; sn[3] = s0.w; sn[4] = s1.x; sn[5] = s1.y; sn[6] = s1.z; sn[7] = s1.w;
+    sn[0] = sign * s0.x; sn[1] = sign * s0.y; sn[2] = sign * s0.z; sn[3] = sign * s0.w;
+    sn[4] = sign * s1.x; sn[5] = sign * s1.y; sn[6] = sign * s1.z; sn[7] = sign * s1.w;
   }
-  if (live) {
-    qw = *reinterpret_cast<const uint4*>(a.qw + d);
-    kw = *reinterpret_cast<const uint4*>(a.kw + d);
-  }
-  constexpr int U = 4;                     // heads of a warp whose loads are in flight together
-  for (int h0 = threadIdx.x >> 5; h0 < heads; h0 += 8 * U) {
+  const float inv_d = 1.f / a.D;
+  auto turned = [&](uint4 in, const float (&gain)[8]) {
+    const uint32_t words[4] = {in.x, in.y, in.z, in.w};
+    float x[8], ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = unpack_bf16x2(words[j]);
+      x[2 * j] = f.x;
+      x[2 * j + 1] = f.y;
+      ss += f.x * f.x + f.y * f.y;
+    }
+    const float rstd = rsqrtf(warp_sum(ss) * inv_d + a.eps);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      x[j] *= rstd * gain[j];
+      const float other = __shfl_sync(0xffffffffu, x[j], partner);
+      x[j] = x[j] * c[j] + other * sn[j];
+    }
+    return make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+  };
+  float gain[8];
+  auto load_gain = [&](const __nv_bfloat16* w) {
+    pm_load8(w + (live ? d : 0), gain);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) gain[j] += 1.f;
+  };
+  const int warp = threadIdx.x >> 5;
+  constexpr int U = 3;                     // heads of a warp whose loads are in flight together
+  const __nv_bfloat16* q_row = a.q + row * a.q_row + d;
+  __nv_bfloat16* q_to = a.q_out + row * a.H * a.D + d;
+  load_gain(a.qw);
+  for (int h0 = warp; h0 < a.H; h0 += 8 * U) {
     uint4 in[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int h = h0 + 8 * u;
-      const __nv_bfloat16* src = h < a.H ? a.q + row * a.q_row + h * a.q_head
-                                         : h < a.H + a.G ? a.k + row * a.k_row + static_cast<long long>(h - a.H) * a.D
-                                                         : a.v + row * a.v_row + static_cast<long long>(h - a.H - a.G) * a.D;
-      in[u] = live && h < heads ? *reinterpret_cast<const uint4*>(src + d) : make_uint4(0u, 0u, 0u, 0u);
-    }
+    for (int u = 0; u < U; ++u) in[u] = live && h0 + 8 * u < a.H ? *reinterpret_cast<const uint4*>(q_row + (h0 + 8 * u) * a.q_head) : none;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int h = h0 + 8 * u;
-      if (h >= heads) break;
-      const bool is_q = h < a.H, is_v = h >= a.H + a.G;
-      const int g = is_q ? h : (is_v ? h - a.H - a.G : h - a.H);
-      __nv_bfloat16* dst = is_q ? a.q_out + (row * a.H + g) * a.D
-                                : (is_v ? a.v_store : a.k_store) + ((static_cast<long long>(b) * a.G + g) * a.cap + a.slot0 + s) * a.D;
-      if (is_v) {
-        if (live) *reinterpret_cast<uint4*>(dst + d) = in[u];
-        continue;
-      }
-      const uint32_t words[4] = {in[u].x, in[u].y, in[u].z, in[u].w};
-      float x[8], y[8];
-      float ss = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = unpack_bf16x2(words[j]);
-        x[2 * j] = f.x;
-        x[2 * j + 1] = f.y;
-        ss += f.x * f.x + f.y * f.y;
-      }
-      const float rstd = rsqrtf(warp_sum(ss) / a.D + a.eps);
-      const uint4 gain = is_q ? qw : kw;
-      const uint32_t gains[4] = {gain.x, gain.y, gain.z, gain.w};
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float2 gj = unpack_bf16x2(gains[j >> 1]);
-        x[j] = x[j] * rstd * (1.f + (j & 1 ? gj.y : gj.x));
-        const float other = __shfl_sync(0xffffffffu, x[j], partner);
-        y[j] = first ? x[j] * c[j] - other * sn[j] : second ? x[j] * c[j] + other * sn[j] : x[j];
-      }
-      if (live) pm_store8(dst + d, y);
+      const uint4 out = turned(in[u], gain);
+      if (live && h0 + 8 * u < a.H) *reinterpret_cast<uint4*>(q_to + (h0 + 8 * u) * a.D) = out;
     }
+  }
+  const long long slot = static_cast<long long>(b) * a.G * a.cap + a.slot0 + s;
+  load_gain(a.kw);
+  for (int h = warp; h < 2 * a.G; h += 8) {
+    const bool is_v = h >= a.G;
+    const int g = is_v ? h - a.G : h;
+    const uint4 in = live ? *reinterpret_cast<const uint4*>((is_v ? a.v + row * a.v_row : a.k + row * a.k_row) + static_cast<long long>(g) * a.D + d) : none;
+    const uint4 out = is_v ? in : turned(in, gain);
+    if (live) *reinterpret_cast<uint4*>((is_v ? a.v_store : a.k_store) + (slot + static_cast<long long>(g) * a.cap) * a.D + d) = out;
   }
 }
 
