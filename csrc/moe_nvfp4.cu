@@ -135,13 +135,23 @@ __device__ __forceinline__ void route_token_n(const RouteArgs& a, const float* r
 #pragma unroll
   for (int j = 0; j < kMaxPer; ++j) {
     const int e = lane + 32 * j;
-    float l = (j < per && e < a.E) ? __ldcg(row + e) : -INFINITY;
-    if (a.low != nullptr && j < per && e < a.E) {
-      const float* lo = a.low + static_cast<long long>(tok) * 2 * a.E + e;
-      float s = __ldcg(lo) + __ldcg(lo + a.E);
-      for (int p = 1; p < a.parts; ++p) s += __ldcg(row + p * a.part_stride + e);
-      l += s;
-    }
+    score[j] = (j < per && e < a.E) ? __ldcg(row + e) : -INFINITY;
+  }
+  if (a.low != nullptr) {
+    const float* lo = a.low + static_cast<long long>(tok) * 2 * a.E + lane;
+#pragma unroll
+    for (int j = 0; j < kMaxPer; ++j) sel[j] = (j < per && lane + 32 * j < a.E) ? __ldcg(lo + 32 * j) + __ldcg(lo + a.E + 32 * j) : 0.f;
+#pragma unroll 2
+    for (int p = 1; p < a.parts; ++p)              // a part's experts at a time: their loads are in flight together
+#pragma unroll
+      for (int j = 0; j < kMaxPer; ++j)
+        if (j < per && lane + 32 * j < a.E) sel[j] += __ldcg(row + p * a.part_stride + lane + 32 * j);
+#pragma unroll
+    for (int j = 0; j < kMaxPer; ++j) score[j] += sel[j];
+  }
+#pragma unroll
+  for (int j = 0; j < kMaxPer; ++j) {
+    float l = score[j];
     if (a.softcap > 0.f && l != -INFINITY) l = a.softcap * tanhf(l / a.softcap);
     score[j] = l;
     mx = fmaxf(mx, l);
@@ -189,29 +199,33 @@ __device__ __forceinline__ void route_token_n(const RouteArgs& a, const float* r
       if (e < a.E && !((kept >> (e / size)) & 1u)) sel[j] = -INFINITY;
     }
   }
+  // Scores as integers of the same order (-0 as 0, NaN and what is taken or does not exist below all): two warp reductions find the best and, of
+  // equal ones, the lowest expert, like a stable top-k.  Ten shuffles a choice were a quarter of the routing of a decode step.
+  uint32_t key[kMaxPer];
+#pragma unroll
+  for (int j = 0; j < kMaxPer; ++j) {
+    const uint32_t u = __float_as_uint(sel[j] + 0.f);
+    key[j] = j < per && lane + 32 * j < a.E && sel[j] == sel[j] ? (u & 0x80000000u ? ~u : u | 0x80000000u) : 0u;
+  }
   float wsum = 0.f;
   float my_w = 0.f;
   int my_id = 0;
   for (int s = 0; s < a.k; ++s) {
-    // warp argmax (ties -> lowest expert index, like a stable top-k)
-    float best = -INFINITY;
-    int best_e = 0x7fffffff;
-    for (int j = 0; j < kMaxPer; ++j) {
-      const int e = lane + 32 * j;
-      if (sel[j] > best || (sel[j] == best && e < best_e)) { best = sel[j]; best_e = e; }
-    }
+    uint32_t best = 0u;
+    int best_j = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-      if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
-    }
+    for (int j = 0; j < kMaxPer; ++j)
+      if (key[j] > best) { best = key[j]; best_j = j; }
+    const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+    const uint32_t mine = best == top && lane + 32 * best_j < a.E ? lane + 32u * best_j : 0x7fffffffu;
+    int best_e = static_cast<int>(__reduce_min_sync(0xffffffffu, mine));
     // owner lane fetches the unbiased score and retires the entry
     float sc = 0.f;
     if ((best_e & 31) == lane) {
       const int j = best_e >> 5;
+#pragma unroll
       for (int q = 0; q < kMaxPer; ++q)
-        if (q == j) { sc = score[q]; sel[q] = -INFINITY; }
+        if (q == j) { sc = score[q]; key[q] = 0u; }
     }
     sc = __shfl_sync(0xffffffffu, sc, best_e & 31);
     wsum += sc;
@@ -295,8 +309,8 @@ __global__ void __launch_bounds__(256) moe_route_fused_kernel(RouteArgs a, const
     const float4* w4 = reinterpret_cast<const float4*>(wr + static_cast<long long>(e) * h);
     const int q4 = h >> 2;                            // float4 groups per row; this warp takes [half * q4 / 2, ...)
     const int lo = half * (q4 >> 1), hi = half ? q4 : (q4 >> 1);
-#pragma unroll 4
-    for (int i = lo + lane; i < hi; i += 32) {        // four weight loads in flight per lane
+#pragma unroll 8
+    for (int i = lo + lane; i < hi; i += 32) {        // eight weight loads in flight per lane
       const float4 w = __ldg(w4 + i);
 #pragma unroll
       for (int t = 0; t < kRouteTok; ++t) {
