@@ -74,6 +74,7 @@ struct __align__(1024) Fp4Smem {
   uint8_t b[F4_STAGES][F4_BN * F4_BKB];
   uint8_t sfa[F4_STAGES][F4_SF_STAGE];
   uint8_t sfb[F4_STAGES][F4_SF_STAGE];
+  uint8_t out[8][32 * 128];            // 32 rows of 64 bf16 results per epilogue warp
   uint64_t full[F4_STAGES];
   uint64_t empty[F4_STAGES];
   uint64_t acc_full[2];
@@ -138,6 +139,25 @@ __device__ __forceinline__ uint8_t ue4m3_encode(float s) {
 __device__ __forceinline__ float ue4m3_decode(uint8_t b) {
   const __half_raw h = __nv_cvt_fp8_to_halfraw(b, __NV_E4M3);
   return __half2float(*reinterpret_cast<const __half*>(&h));
+}
+// Eight codes by the conversion of the hardware, first number in the low nibble: the same rounding and saturation; NaN becomes zero as above, and only
+// the sign of a zero may differ.  By comparisons the SwiGLU epilogue spent a third of its instructions here.
+__device__ __forceinline__ uint32_t e2m1_codes(const float (&q)[8]) {
+  float v[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = q[j] == q[j] ? q[j] : 0.f;
+  uint32_t w;
+  asm("{\n\t"
+      ".reg .b8 b0, b1, b2, b3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+      "mov.b32 %0, {b0, b1, b2, b3};\n\t"
+      "}\n"
+      : "=r"(w)
+      : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]));
+  return w;
 }
 // offset of (row, 16-element block kb) in the tensor-core scale order, ktiles = K / 64
 __device__ __forceinline__ long long sf_offset(int row, int kb, int ktiles) {
@@ -473,16 +493,20 @@ fp4_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, Fp4Params p) {
       int e, mt, nt, lt;
       decode(tile, e, mt, nt, lt);
       const uint32_t buf = seg & 1;
+      const int prow = mt * F4_BM + quarter * 32 + lane;                       // padded row
+      // read before the accumulator is waited for: behind it these loads were part of every tile's chain
+      const float sa = p.a_row_scale ? p.a_row_scale[prow] : 1.f;
+      const float wg = p.w_global[e], wg2 = p.mode != 0 ? p.w_global2[e] : 1.f;
       if (!mbar_wait(&s.acc_full[buf], (seg >> 1) & 1, p.err, 1400 + buf)) { ok = false; break; }
       tc_fence_after();
-      const int prow = mt * F4_BM + quarter * 32 + lane;                       // padded row
       const int local = lt * F4_BM + quarter * 32 + lane;                      // row inside the expert
       const bool row_ok = local < s.gr[e + 1] - s.gr[e];
       const uint32_t t_row = tmem_base + buf * F4_BN + (static_cast<uint32_t>(quarter * 32) << 16);
-      const float sa = p.a_row_scale ? p.a_row_scale[prow] : 1.f;
       if (p.mode == 0) {
-        const float f = sa / p.w_global[e];
-        __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<long long>(prow) * p.N + nt * F4_BN + half * 64;
+        const float f = sa / wg;
+        // Through shared memory, so that a store writes whole 128-byte rows: row by row from the accumulator's lanes every store touched 32 lines, and
+        // a 4000-token prompt of 256 experts took 432 us in its two products (452 with codes by comparison and the factors read behind the accumulator), now 402.
+        uint8_t* st = s.out[warp - 2];
 #pragma unroll 1
         for (int c = 0; c < 2; ++c) {
           uint32_t r[32];
@@ -493,7 +517,6 @@ fp4_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, Fp4Params p) {
             __syncwarp();
             if (lane == 0) mbar_arrive(&s.acc_empty[buf]);
           }
-          if (!row_ok) continue;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             uint4 u;
@@ -501,9 +524,19 @@ fp4_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, Fp4Params p) {
             u.y = pack_bf16x2(__uint_as_float(r[q * 8 + 2]) * f, __uint_as_float(r[q * 8 + 3]) * f);
             u.z = pack_bf16x2(__uint_as_float(r[q * 8 + 4]) * f, __uint_as_float(r[q * 8 + 5]) * f);
             u.w = pack_bf16x2(__uint_as_float(r[q * 8 + 6]) * f, __uint_as_float(r[q * 8 + 7]) * f);
-            *reinterpret_cast<uint4*>(out + c * 32 + q * 8) = u;
+            *reinterpret_cast<uint4*>(st + lane * 128 + (((c * 4 + q) ^ (lane & 7)) << 4)) = u;
           }
         }
+        __syncwarp();
+        const int valid = s.gr[e + 1] - s.gr[e] - lt * F4_BM - quarter * 32;       // rows of the expert among these 32
+        uint8_t* out = reinterpret_cast<uint8_t*>(reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<long long>(prow - lane) * p.N + nt * F4_BN + half * 64);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = i * 4 + (lane >> 3), ch = lane & 7;
+          if (r < valid)
+            *reinterpret_cast<uint4*>(out + static_cast<long long>(r) * p.N * 2 + ch * 16) = *reinterpret_cast<const uint4*>(st + r * 128 + ((ch ^ (r & 7)) << 4));
+        }
+        __syncwarp();
       } else {
         // gate columns [32 half, +32) and the matching up columns at +64: h = silu(gate) * up, then NVFP4 with a global of 1
         uint32_t rg[32], ru[32];
@@ -513,7 +546,7 @@ fp4_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, Fp4Params p) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&s.acc_empty[buf]);
-        const float fg = sa / p.w_global[e], fu = sa / p.w_global2[e];
+        const float fg = sa / wg, fu = sa / wg2;
         float hv[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
@@ -533,10 +566,10 @@ fp4_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, Fp4Params p) {
           const float inv_s = sdec > 0.f ? 1.f / sdec : 0.f;
 #pragma unroll
           for (int w = 0; w < 2; ++w) {
-            uint32_t acc = 0;
+            float q[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc |= e2m1_code(hv[b * 16 + w * 8 + j] * inv_s) << (4 * j);
-            words[b * 2 + w] = acc;
+            for (int j = 0; j < 8; ++j) q[j] = hv[b * 16 + w * 8 + j] * inv_s;
+            words[b * 2 + w] = e2m1_codes(q);
           }
         }
         const int col = nt * 64 + half * 32;                 // first of my 32 result columns
