@@ -116,11 +116,6 @@ struct RouteArgs {
   float softcap, scale;
   int groups, keep;      // groups > 1: E / groups neighbouring experts form a group; only the `keep` groups with the best expert compete
   int ld;                // columns of a row of logits: E, or more where other projections of the token follow the router's
-  // Products with the terms of a split router matrix: a logit is the sum of `parts` numbers part_stride apart and, with `low`, of two columns of
-  // low [T, 2 E] that are E apart.
-  int parts;
-  long long part_stride;
-  const float* low;
 };
 
 // One warp routes one token from its row of logits.  The row may have been written by other CTAs of the same launch, so it is
@@ -136,18 +131,6 @@ __device__ __forceinline__ void route_token_n(const RouteArgs& a, const float* r
   for (int j = 0; j < kMaxPer; ++j) {
     const int e = lane + 32 * j;
     score[j] = (j < per && e < a.E) ? __ldcg(row + e) : -INFINITY;
-  }
-  if (a.low != nullptr) {
-    const float* lo = a.low + static_cast<long long>(tok) * 2 * a.E + lane;
-#pragma unroll
-    for (int j = 0; j < kMaxPer; ++j) sel[j] = (j < per && lane + 32 * j < a.E) ? __ldcg(lo + 32 * j) + __ldcg(lo + a.E + 32 * j) : 0.f;
-#pragma unroll 2
-    for (int p = 1; p < a.parts; ++p)              // a part's experts at a time: their loads are in flight together
-#pragma unroll
-      for (int j = 0; j < kMaxPer; ++j)
-        if (j < per && lane + 32 * j < a.E) sel[j] += __ldcg(row + p * a.part_stride + lane + 32 * j);
-#pragma unroll
-    for (int j = 0; j < kMaxPer; ++j) score[j] += sel[j];
   }
 #pragma unroll
   for (int j = 0; j < kMaxPer; ++j) {
@@ -245,27 +228,6 @@ __device__ __forceinline__ void route_token(const RouteArgs& a, const float* row
   else if (a.E <= 128) route_token_n<4>(a, row, tok, lane);
   else if (a.E <= 256) route_token_n<8>(a, row, tok, lane);
   else route_token_n<16>(a, row, tok, lane);       // E <= 512
-}
-
-__global__ void __launch_bounds__(256) split_bf16x3_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ out, long long n) {
-  pdl_entry();
-  for (long long i = (blockIdx.x * 256LL + threadIdx.x) * 4; i < n; i += gridDim.x * 1024LL) {
-    const float4 v = *reinterpret_cast<const float4*>(w + i);
-    const float f[4] = {v.x, v.y, v.z, v.w};
-    float t[3][4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float hi = __bfloat162float(__float2bfloat16(f[j]));
-      const bool finite = fabsf(hi) < INFINITY;
-      const float r = finite ? f[j] - hi : 0.f, mid = __bfloat162float(__float2bfloat16(r));
-      t[0][j] = hi;
-      t[1][j] = mid;
-      t[2][j] = r - mid;
-    }
-#pragma unroll
-    for (int p = 0; p < 3; ++p)
-      *reinterpret_cast<uint2*>(out + p * n + i) = make_uint2(pack_bf16x2(t[p][0], t[p][1]), pack_bf16x2(t[p][2], t[p][3]));
-  }
 }
 
 __global__ void __launch_bounds__(256) moe_route_kernel(RouteArgs a) {
@@ -876,18 +838,12 @@ extern "C" TYR_EXPORT int tyr_nvfp4_dequant(const void* packed, const void* scal
 
 extern "C" TYR_EXPORT int tyr_moe_route(const float* logits, const float* bias, int* ids, float* weights, int* counts,
                                         int T, int E, int k, int softmax, int renorm, float softcap, float scale,
-                                        int groups, int keep, int ld, int parts, long long part_stride, const float* low, void* stream) {
-  if (ld < E || parts < 1 || (parts > 1 && low == nullptr)) return -5;
+                                        int groups, int keep, int ld, void* stream) {
+  if (ld < E) return -5;
   if (T <= 0 || E <= 0 || E > 512 || k <= 0 || k > 32 || k > E) return -1;
   if (groups > 1 && (groups > 32 || E % groups || keep <= 0 || keep > groups || k > keep * (E / groups))) return -4;
-  RouteArgs a{logits, bias, ids, weights, counts, T, E, k, softmax, renorm, softcap, scale, groups, keep, ld, parts, part_stride, low};
+  RouteArgs a{logits, bias, ids, weights, counts, T, E, k, softmax, renorm, softcap, scale, groups, keep, ld};
   return (int)launch_dependent(moe_route_kernel, dim3((T + 7) / 8), dim3(256), 0, (cudaStream_t)stream, a);
-}
-
-// w fp32 [n] -> bf16 [3][n], whose sum is w to 24 bits (the first term alone where it is not finite).
-extern "C" TYR_EXPORT int tyr_split_bf16x3(const float* w, void* out, long long n, void* stream) {
-  if (n <= 0 || (n & 3) || (reinterpret_cast<uintptr_t>(w) & 15) || (reinterpret_cast<uintptr_t>(out) & 7)) return -1;
-  return (int)launch_dependent(split_bf16x3_kernel, dim3(blocks_for(n / 4)), dim3(256), 0, (cudaStream_t)stream, w, (__nv_bfloat16*)out, n);
 }
 
 // Router GEMV + routing in one launch: x bf16 [T, h] (h a multiple of 8), router weight fp32 [ld, h] whose first E rows route (the
@@ -907,7 +863,7 @@ extern "C" TYR_EXPORT int tyr_moe_route_fused(const void* x, const float* router
     cudaFuncSetAttribute(moe_route_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     configured = smem;
   }
-  RouteArgs a{nullptr, bias, ids, weights, counts, T, E, k, softmax, renorm, softcap, scale, groups, keep, ld, 1, 0, nullptr};
+  RouteArgs a{nullptr, bias, ids, weights, counts, T, E, k, softmax, renorm, softcap, scale, groups, keep, ld};
   dim3 grid((T + kRouteTok - 1) / kRouteTok, (ld + kRouteExp - 1) / kRouteExp);
   return (int)launch_dependent(moe_route_fused_kernel, grid, dim3(256), smem, (cudaStream_t)stream, a, (const __nv_bfloat16*)x,
                                router_w, logits, tickets, h);

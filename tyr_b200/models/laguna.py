@@ -367,10 +367,10 @@ def route(cfg: LagunaConfig, r: Router, x2: torch.Tensor):
     if moe_ops.route_fused_supported(x2, r.weight):
         return moe_ops.route_fused(x2, r.weight, cfg.num_experts_per_tok, softmax=False, bias=r.e_score_correction_bias, renorm=cfg.norm_topk_prob,
                                    softcap=cfg.moe_router_logit_softcapping, scale=cfg.moe_routed_scaling_factor)
-    logits, low = moe_ops.split_logits(x2, r.weight) if moe_ops.split_logits_supported(x2, r.weight) else (F.linear(x2.float(), r.weight.float()), None)
+    logits = F.linear(x2.float(), r.weight.float())
     return moe_ops.route(logits, cfg.num_experts_per_tok, softmax=False, bias=r.e_score_correction_bias,
                          renorm=cfg.norm_topk_prob, softcap=cfg.moe_router_logit_softcapping,
-                         scale=cfg.moe_routed_scaling_factor, low=low)
+                         scale=cfg.moe_routed_scaling_factor)
 
 
 def moe_forward(cfg: LagunaConfig, m: SparseMoeBlock, x2: torch.Tensor, use_fused: bool = True, ep=None) -> torch.Tensor:

@@ -20,7 +20,7 @@ import torch
 
 from .._native import register_signatures
 from ._common import check, cur_stream, lib, ptr
-from .gemm import gemm, grouped_gemm
+from .gemm import grouped_gemm
 
 E2M1 = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0, -0.0, -0.5, -1.0, -1.5, -2.0, -3.0, -4.0, -6.0])
 
@@ -31,7 +31,7 @@ def _sigs(lib_):
     P, I, L, F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
     table = {
         "tyr_nvfp4_quantize": [P, P, P, P, L, L, P], "tyr_nvfp4_dequant": [P, P, P, P, L, L, P],
-        "tyr_moe_route": [P, P, P, P, P, I, I, I, I, I, F, F, I, I, I, I, L, P, P], "tyr_split_bf16x3": [P, P, L, P],
+        "tyr_moe_route": [P, P, P, P, P, I, I, I, I, I, F, F, I, I, I, P],
         "tyr_moe_layout_small": [P, P, P, P, P, P, I, I, P, L, P],
         "tyr_moe_route_fused": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, F, I, I, I, P],
         "tyr_moe_layout": [P, P, P, P, P, P, P, P, I, I, P], "tyr_moe_count": [P, P, I, I, P],
@@ -116,13 +116,13 @@ def nvfp4_dequant(packed: torch.Tensor, scales: torch.Tensor, global_scale: torc
 # ---- routing -------------------------------------------------------------------------------------------
 def route(logits: torch.Tensor, k: int, *, softmax: bool = False, bias: Optional[torch.Tensor] = None,
           renorm: bool = True, softcap: float = 0.0, scale: float = 1.0, want_counts: bool = True, groups: int = 1, keep: int = 1,
-          experts: Optional[int] = None, low: Optional[torch.Tensor] = None):
-    """logits fp32 [T, E] (with ``low`` [T, 2 E]: [parts, T, E], both from :func:`split_logits`; or more columns, of which the first ``experts`` count) -> (ids int32 [T, k], weights fp32 [T, k], counts int32 [E]).
+          experts: Optional[int] = None):
+    """logits fp32 [T, E] (or more columns, of which the first ``experts`` count) -> (ids int32 [T, k], weights fp32 [T, k], counts int32 [E]).
     Sigmoid (Laguna, Tyr/Model/Laguna/MoE.lean:71-90) or softmax (Qwen3.5) scores; the selection
     bias only influences WHICH experts are picked; ties go to the lower expert index.  With ``groups`` > 1 the experts form
     that many equal groups of neighbours, a group counts by its best selection score (bias included), and only experts of the
     ``keep`` best groups compete."""
-    T, E = logits.shape[-2], experts or logits.shape[-1]
+    T, E = logits.shape[0], experts or logits.shape[1]
     if logits.is_cuda:
         lg = logits.float().contiguous()
         ids = torch.empty((T, k), dtype=torch.int32, device=logits.device)
@@ -130,10 +130,9 @@ def route(logits: torch.Tensor, k: int, *, softmax: bool = False, bias: Optional
         counts = torch.zeros(E, dtype=torch.int32, device=logits.device)
         b = bias.float().contiguous() if bias is not None else None
         check(lib().tyr_moe_route(ptr(lg), ptr(b), ptr(ids), ptr(w), ptr(counts), T, E, k, 1 if softmax else 0,
-                                  1 if renorm else 0, softcap, scale, groups, keep, lg.shape[-1], lg.shape[0] if low is not None else 1, T * lg.shape[-1],
-                                  ptr(low), cur_stream(logits.device)), "moe_route")
+                                  1 if renorm else 0, softcap, scale, groups, keep, lg.shape[1], cur_stream(logits.device)), "moe_route")
         return ids, w, counts
-    l = logits[:, :E].float() if low is None else logits.sum(0) + low[:, :E] + low[:, E:]
+    l = logits[:, :E].float()
     if softcap > 0:
         l = softcap * torch.tanh(l / softcap)
     scores = torch.softmax(l, -1) if softmax else torch.sigmoid(l)
@@ -149,31 +148,6 @@ def route(logits: torch.Tensor, k: int, *, softmax: bool = False, bias: Optional
     ids = order.to(torch.int32)
     counts = torch.bincount(ids.reshape(-1).long(), minlength=E).to(torch.int32)
     return ids, w * scale, counts
-
-
-def _router_parts(h: int) -> int:
-    """Equal parts of at most 400 channels, multiples of 8 (0: none)."""
-    return next((p for p in range(1, h // 8 + 1) if h % (8 * p) == 0 and h // p <= 400), 0)
-
-
-def split_logits_supported(x: torch.Tensor, router_w: torch.Tensor) -> bool:
-    return (x.is_cuda and x.dtype == torch.bfloat16 and router_w.dtype == torch.float32 and x.dim() == 2 and x.shape[1] % 8 == 0 and x.stride(1) == 1
-            and _router_parts(x.shape[1]) > 0 and router_w.shape[0] % 4 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and router_w.is_contiguous() and router_w.data_ptr() % 16 == 0
-            and not torch.is_grad_enabled())
-
-
-def split_logits(x: torch.Tensor, router_w: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
-    """bf16 rows [T, h] times an fp32 router [E, h] -> fp32 (high [parts, T, E], low [T, 2 E]) whose sum over parts and the two halves of low are the logits.
-    The router's numbers are the sum of three bf16 numbers each, whose products the tensor cores take exactly.  Their sums lose more than fp32 sums
-    over thousands of channels (1e-6 against 2.5e-7 at 1000), so those of the leading terms end after 400 channels at most; the other terms'
-    are 2^-8 of them.  4000 x 256 x 3072: about 45 us with the split; the library's fp32 product took
-    129 us and the conversion of the rows 34."""
-    E, h = router_w.shape
-    T, parts = x.shape[0], _router_parts(h)
-    w3 = torch.empty((3 * E, h), dtype=torch.bfloat16, device=x.device)
-    check(lib().tyr_split_bf16x3(ptr(router_w), ptr(w3), E * h, cur_stream(x.device)), "split_bf16x3")
-    cut = lambda t, rows: t.as_strided((parts, rows, h // parts), (h // parts, t.stride(0), 1))
-    return gemm(cut(x, T), cut(w3, E), out_dtype=torch.float32), gemm(x, w3[E:], out_dtype=torch.float32)
 
 
 def count_experts(ids: torch.Tensor, E: int) -> torch.Tensor:
