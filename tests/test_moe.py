@@ -219,6 +219,15 @@ def test_gpu_layout_of_a_decode_batch_in_one_launch(T, k, E):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("T,h", [(1, 8), (1, 12), (257, 264), (4099, 3072)])
+def test_gpu_widen_equals_the_conversion(T, h):
+    x = torch.randn(T + 1, h, generator=torch.Generator().manual_seed(T)).mul_(1e-3).bfloat16().cuda()
+    x.view(-1)[h:h + 8] = torch.tensor([0.0, -0.0, float("inf"), float("-inf"), float("nan"), 1e-40, 3e38, -1.0], dtype=torch.bfloat16)
+    for y in (x, x[1:], x[:, 1:]):               # aligned, perhaps not aligned, not contiguous
+        assert torch.equal(moe.widen(y).view(torch.int32), y.float().view(torch.int32))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("T,k,E,h", [(1, 1, 3, 256), (130, 4, 9, 512), (300, 2, 40, 768)])
 def test_gpu_scatter_quantize_equals_gather_quantize(T, k, E, h):
     """Every routed row at its place: the same codes, scales and factors."""

@@ -367,7 +367,7 @@ def route(cfg: LagunaConfig, r: Router, x2: torch.Tensor):
     if moe_ops.route_fused_supported(x2, r.weight):
         return moe_ops.route_fused(x2, r.weight, cfg.num_experts_per_tok, softmax=False, bias=r.e_score_correction_bias, renorm=cfg.norm_topk_prob,
                                    softcap=cfg.moe_router_logit_softcapping, scale=cfg.moe_routed_scaling_factor)
-    logits = F.linear(x2.float(), r.weight.float())
+    logits = F.linear(moe_ops.widen(x2), r.weight.float())
     return moe_ops.route(logits, cfg.num_experts_per_tok, softmax=False, bias=r.e_score_correction_bias,
                          renorm=cfg.norm_topk_prob, softcap=cfg.moe_router_logit_softcapping,
                          scale=cfg.moe_routed_scaling_factor)

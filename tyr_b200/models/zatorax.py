@@ -430,7 +430,7 @@ def route(s: MoeSpec, m: Experts, x2: torch.Tensor):
     if x2.is_cuda and x2.dtype == torch.bfloat16 and x2.shape[0] >= TCGEN05_MIN_ROWS and s.experts % 8 == 0 and x2.shape[1] % 8 == 0:
         logits = gemm(x2, m.router_lp, out_dtype=torch.float32)       # bf16 operands are exact here: fp32 sums of fp32 products
     else:
-        logits = F.linear(x2.float(), m.router)
+        logits = F.linear(moe_ops.widen(x2), m.router)
     return moe_ops.route(logits, s.top, **kw)
 
 

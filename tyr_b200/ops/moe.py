@@ -31,7 +31,7 @@ def _sigs(lib_):
     P, I, L, F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
     table = {
         "tyr_nvfp4_quantize": [P, P, P, P, L, L, P], "tyr_nvfp4_dequant": [P, P, P, P, L, L, P],
-        "tyr_moe_route": [P, P, P, P, P, I, I, I, I, I, F, F, I, I, I, P],
+        "tyr_moe_route": [P, P, P, P, P, I, I, I, I, I, F, F, I, I, I, P], "tyr_widen_bf16": [P, P, L, P],
         "tyr_moe_layout_small": [P, P, P, P, P, P, I, I, P, L, P],
         "tyr_moe_route_fused": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, F, I, I, I, P],
         "tyr_moe_layout": [P, P, P, P, P, P, P, P, I, I, P], "tyr_moe_count": [P, P, I, I, P],
@@ -148,6 +148,16 @@ def route(logits: torch.Tensor, k: int, *, softmax: bool = False, bias: Optional
     ids = order.to(torch.int32)
     counts = torch.bincount(ids.reshape(-1).long(), minlength=E).to(torch.int32)
     return ids, w * scale, counts
+
+
+def widen(x: torch.Tensor) -> torch.Tensor:
+    """x in fp32; bf16 rows on the GPU by one of our kernels where no gradient flows."""
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and x.numel() > 0 and x.numel() % 8 == 0 and x.data_ptr() % 16 == 0
+            and not (torch.is_grad_enabled() and x.requires_grad)):
+        return x.float()
+    out = torch.empty(x.shape, dtype=torch.float32, device=x.device)
+    check(lib().tyr_widen_bf16(ptr(x), ptr(out), x.numel(), cur_stream(x.device)), "widen_bf16")
+    return out
 
 
 def count_experts(ids: torch.Tensor, E: int) -> torch.Tensor:
