@@ -27,6 +27,7 @@
 namespace tyr {
 
 constexpr int kDecWarps = 4;
+constexpr int kDecMaxSplits = 64;        // slices of a (row, K/V head): two per lane of the warp that merges a head
 
 struct DecodeAttnArgs {
   const __nv_bfloat16* q;        // [B, Hq, D], batch stride q_bs, head stride D
@@ -165,16 +166,27 @@ __device__ __forceinline__ void decode_combine(const DecodeAttnArgs& a, int b, i
   // The slices' weights first, a warp per head, then the sums with the loads of several channels and slices in flight.  One channel after the other,
   // each with its own passes over the slices, was most of the kernel where few CTAs merge much: one row of
   // 8 heads of 256 over 564 keys in 9 slices took 26.2 us and takes 13.4, 32 slices 67.6 and 16.6.
-  __shared__ float s_f[GM][32], s_M[GM], s_L[GM];                 // at most 32 slices
+  __shared__ float s_f[GM][kDecMaxSplits], s_M[GM], s_L[GM];
   const int warp = tid >> 5, lane = tid & 31;
   for (int g = warp; g < G; g += kDecWarps) {
-    const long long row = static_cast<long long>(b) * a.Hq + hq0 + g;
-    const bool in = lane < a.splits;
-    const float m = in ? __ldcg(&a.part_ml[(row * a.splits + lane) * 2]) : -INFINITY;
-    const float M = warp_max(m);
-    const float f = in && m > -INFINITY ? exp2f(m - M) : 0.f;
-    const float L = warp_sum(f != 0.f ? __ldcg(&a.part_ml[(row * a.splits + lane) * 2 + 1]) * f : 0.f);
-    s_f[g][lane] = f;
+    const float* ml = a.part_ml + (static_cast<long long>(b) * a.Hq + hq0 + g) * a.splits * 2;
+    constexpr int P = kDecMaxSplits / 32;        // slices of a lane
+    float m[P], M = -INFINITY, L = 0.f;
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const int sp = lane + 32 * i;
+      m[i] = sp < a.splits ? __ldcg(ml + sp * 2) : -INFINITY;
+      M = fmaxf(M, m[i]);
+    }
+    M = warp_max(M);
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const int sp = lane + 32 * i;
+      const float f = m[i] > -INFINITY ? exp2f(m[i] - M) : 0.f;
+      if (f != 0.f) L += __ldcg(ml + sp * 2 + 1) * f;
+      s_f[g][sp] = f;
+    }
+    L = warp_sum(L);
     if (lane == 0) {
       s_M[g] = M;
       s_L[g] = L;
@@ -569,7 +581,7 @@ static int decode_attention_launch(const void* q, const void* k_new, const void*
                                    long long out_bs = 0, float out_scale = 1.f, int keep = 0, const void* back = nullptr, int back_rows = 0) {
   using namespace tyr;
   if (gate_mode < 0 || gate_mode > 3 || (gate_mode != 0 && gate == nullptr)) return -5;
-  if (B <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0 || Hq / Hkv > 16 || cap <= 0 || splits < 1 || splits > 64) return -1;
+  if (B <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0 || Hq / Hkv > 16 || cap <= 0 || splits < 1 || splits > kDecMaxSplits) return -1;
   const bool wide = Hq / Hkv > 8;
   if ((q_bs | kn_bs | vn_bs) & 7) return -3;                       // 16-byte rows
   if ((r1 != nullptr) != (r2 != nullptr)) return -6;

@@ -826,3 +826,41 @@ def test_decode_attention_merges_any_number_of_slices(splits, B, H, G, D):
     want = decode_attention(q.float(), k.float(), v.float(), kc.clone().float(), vc.clone().float(), pos)
     got = decode_attention(*(t.cuda() for t in (q, k, v, kc, vc, pos)), splits=splits)
     assert (got.float().cpu() - want).abs().max() <= 2.0 ** -7
+
+
+@pytest.mark.parametrize("splits", [33, 48, 64])
+@pytest.mark.parametrize("form", ["plain", "gated", "kept", "sink", "biased"])
+def test_decode_attention_merges_more_slices_than_lanes(form, splits, monkeypatch):
+    """4001 keys in more slices than a warp has lanes, 9 heads a K/V head or one; the forms that choose their slices themselves are told the number.  P is
+    rounded to bf16 (2^-9 of a mean whose errors average out) and so is the result: 2^-7 of the largest covers both."""
+    from tyr_b200.models.common import KVCache
+    from tyr_b200.ops import biased_attention as ba, decode_attention as da, kept_attention as ka, sink_attention as sa
+    monkeypatch.setattr(da, "pick_splits", lambda *a: splits)
+    monkeypatch.setattr(sa, "pick_splits", lambda *a: splits)
+    g = torch.Generator().manual_seed(splits)
+    r = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    for H, G, D in ((9, 1, 128), (4, 4, 64)):
+        B, cap = 2, 4010
+        q, k, v, kc, vc = r(B, H, D), r(B, G, D), r(B, G, D), r(B, G, cap, D), r(B, G, cap, D)
+        gate, sink, turns = r(B, H), torch.randn(H, generator=g), torch.randn(cap, D // 2, generator=g) * 3
+        back = torch.stack([turns.cos(), turns.sin()], -1)
+        both = torch.tensor([4000, 3999], dtype=torch.int32)
+
+        def run(dev, typ):
+            t = lambda x: x.to(dev, typ)
+            store = KVCache(t(kc.clone()), t(vc.clone()))
+            if form in ("plain", "gated"):
+                return da.decode_attention(t(q), t(k), t(v), store.k, store.v, both[:1].to(dev), elem_gate=t(q.neg()) if form == "gated" else None,
+                                           splits=splits)
+            if form == "kept":
+                return ka.step_attention(t(q)[:, None], store, both.to(dev), D, D, scale=D ** -0.5, window=3900, keep=7, head_gate=t(gate)[:, None],
+                                         back=back.to(dev))
+            if form == "sink":
+                return sa.step_attention(t(q)[:, None], t(k)[:, None], t(v)[:, None], store, both.to(dev), D, scale=D ** -0.5, sink=sink.to(dev))
+            return ba.step_attention(t(q)[:, None], t(k)[:, None], t(v)[:, None], store, both.to(dev), sink.abs().to(dev), gate[0].float().abs().to(dev),
+                                     window=None, scale=D ** -0.5, append=True)
+        want, got = run("cpu", torch.float32), run("cuda", torch.bfloat16).float().cpu()
+        assert (got - want).abs().max() <= 2.0 ** -7 * want.abs().max(), (form, H)
+    if form == "plain":
+        with pytest.raises(RuntimeError):
+            da.decode_attention(*(t.cuda() for t in (q, k, v, kc, vc, both)), splits=65)

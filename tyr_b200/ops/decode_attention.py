@@ -66,7 +66,7 @@ def decode_attention(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, 
     for a ring store) when ``append`` and returns the attention of the new query over the retained keys (all of a ring
     store; the last ``window`` positions of a plain one), ``[B, Hq, D]``.  ``head_gate`` ([B, Hq]) multiplies each head's
     output by ``softplus(gate)``, ``elem_gate`` ([B, Hq, D]) each element by ``sigmoid(gate)``; on the GPU the gate is
-    applied inside the kernel's final write."""
+    applied inside the kernel's final write.  ``splits``: slices of the keys, 1 to 64 (None: by size)."""
     B, Hq, D = q.shape
     Hkv, cap = k_cache.shape[1], k_cache.shape[2]
     sc = scale if scale is not None else 1.0 / math.sqrt(D)
