@@ -3,6 +3,7 @@ refuse what the kernels do not take (the kernels themselves are tested on a GPU 
 test_qwen35.py)."""
 import torch
 
+from tyr_b200.ops import decode_attention as DA
 from tyr_b200.ops import decode_gemm as DG
 from tyr_b200.ops import delta_rule as DR
 from tyr_b200.ops import fp4
@@ -45,3 +46,14 @@ def test_gdr_tile_predicate_needs_aligned_rows(monkeypatch):
         assert not DR._tile_ok(128, v, z, 32)                    # row stride not a multiple of 4 elements
         monkeypatch.setattr(DR, "_GDR_TILE_MIN_TILES", 64)
         assert not DR._tile_ok(128, v, None, 32)                 # fewer tiles than the threshold
+
+
+def test_slices_fill_the_chip_without_a_thin_last_wave():
+    """The fastest (or next to it) of the measured numbers of slices, for few and many pairs, short and long stores."""
+    for (B, G, keys, heads, D), good in {(1, 2, 564, 4, 256): {9}, (32, 4, 576, 4, 256): {2}, (40, 4, 2048, 4, 256): {3}, (72, 4, 8192, 4, 256): {1},
+                                         (32, 4, 2048, 4, 128): {3}, (38, 4, 8192, 4, 128): {2, 5, 6}, (48, 4, 8192, 4, 128): {2}, (64, 4, 2048, 4, 128): {3},
+                                         (40, 4, 2048, 8, 64): {4}, (38, 4, 8192, 8, 64): {4}, (75, 4, 8192, 8, 64): {2}}.items():
+        assert DA.pick_splits(B, G, keys, heads, D, D) in good, (B, G, keys, D)
+    for keys in (1, 64, 65, 300, 100000):
+        for B in (1, 7, 150, 100000):
+            assert 1 <= DA.pick_splits(B, 2, keys) <= min(32, -(-keys // 64))

@@ -131,7 +131,7 @@ def step_attention(q, k_new, v_new, store, pos: torch.Tensor, r1, r2, *, window:
     dvp = store.v.shape[3]
     if step_fused(q, G, store):
         keys = min(cap, window) if window else cap
-        splits = da.pick_splits(B, G, keys)
+        splits = da.pick_splits(B, G, keys, H // G, dkp, dvp)
         key = (q.device.index, B, H, G, dvp, splits)
         ws = da._workspaces.get(key)
         if ws is None:

@@ -5,6 +5,7 @@ The CPU path states the same contract in plain PyTorch and is the oracle of the 
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 from typing import Dict, Optional, Tuple
 
@@ -35,12 +36,25 @@ def _sigs(lib_):
         lib_.tyr_decode_attention_workspace_bytes.restype = L
 
 
-def pick_splits(B: int, Hkv: int, keys: int) -> int:
-    """Enough CTAs to fill 148 SMs about twice, with at least 64 keys a split and 32 splits at most.  Us at 1 / 2 / 3 / 9 / 16 splits: one row of 2 K/V heads of
-    256 over 564 keys 21.1 / 18.1 / 15.8 / 13.4 / 14.0, over 4096 keys 167 / 92 / 67 / 33 / 23; 32 rows of 4 K/V heads of 256 over 576 keys
-    41.8 / 38.2 / 49.6 / 68.0 / 88.6; 16 rows of 2 over 2048 keys 93.5 / 54.5 / 43.9 / 30.3 / 36.5."""
-    want = 296 // max(1, B * Hkv)
-    return max(1, min(want, 32, -(-keys // 64)))
+@functools.lru_cache(maxsize=4096)
+def pick_splits(B: int, Hkv: int, keys: int, heads: int = 1, DK: int = 128, DV: int = 128) -> int:
+    """Slices of the keys for each of B * Hkv (row, K/V head) pairs of ``heads`` query heads: the number with the least modelled time, in keys that a CTA
+    reads.  A CTA waits for its own loads, whatever shares its SM, so a launch takes as many waves of CTAs as it fills: 2, 3, 4 or 5 of them fit an SM by
+    registers, and of the smallest ones a wave holds 690 (704 took 1.19 times as long as 640).  A wave costs its keys (whole steps of 64) and 256 more, the merge
+    16384 / DV and 512 / DV a slice, four times that with more than 8 heads.
+
+    Us at 1 / 2 / 3 / 4 / 6 slices, heads of 256: 128 pairs of 576 keys 35.6 / 28.1 / 37.2 / 36.0 / 40.7, 160 of 2048 114 / 122 / 92 / 102 / 96, 288 of 8192
+    451 / 463 / 472 / 475 / 495; of 128: 128 of 2048 79 / 48 / 37 / 52 / 44, 192 of 8192 307 / 171 / 221 / 176 / 182; of 64: 160 of 8192 205 / 120 / 88 / 72 / 93.
+    Over 1 to 640 pairs of 300 to 32768 keys, plain, kept and biased, the choice takes 1.01 times the best on average and 1.25 at most; filling the SMs twice
+    takes 1.04 to 1.34 and 3.3, four times with 256 keys a slice 1.10 to 1.19 and 2.1."""
+    pairs = max(1, B * Hkv)
+    at_once = 296 if max(DK, DV) > 128 else 444 if DV > 64 else 592 if DK > 64 else 690
+    merge = (4 if heads > 8 else 1) * 512 / DV
+
+    def cost(s):
+        chunk = -(-keys // (64 * s)) * 64
+        return -(-pairs * s // at_once) * (chunk + 256) + (merge * (32 + s) if s > 1 else 0)
+    return min(range(1, max(1, min(32, -(-keys // 64))) + 1), key=cost)
 
 
 def geometry_supported(Hq: int, Hkv: int, D: int) -> bool:
@@ -99,7 +113,7 @@ def decode_attention(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, 
     q, k_new, v_new = (t if _rows_ok(t, D) else t.contiguous() for t in (q, k_new, v_new))
     keys = cap if ring or not window else min(cap, window)
     if splits is None:
-        splits = pick_splits(B, Hkv, keys)
+        splits = pick_splits(B, Hkv, keys, Hq // Hkv, D, D)
     key = (q.device.index, B, Hq, Hkv, D, splits)
     ws = _workspaces.get(key)
     if ws is None:

@@ -161,7 +161,7 @@ def step_attention(q, store, pos: torch.Tensor, dk: int, dv: int, *, scale: floa
     assert not store.ring or store.keep == keep
     if step_fused(q, G, store):
         keys = min(cap, window + keep) if window else cap
-        splits = da.pick_splits(B, G, keys)
+        splits = da.pick_splits(B, G, keys, H // G, dkp, dvp)
         key = (q.device.index, B, H, G, dvp, splits)
         ws = da._workspaces.get(key)
         if ws is None:
