@@ -1,12 +1,15 @@
 """Host-side logic of the decode-sized kernels' wrappers: CPU fallbacks equal the plain formulas and the path predicates
 refuse what the kernels do not take (the kernels themselves are tested on a GPU in test_gpu_kernels.py / test_moe.py /
 test_qwen35.py)."""
+import pytest
 import torch
 
+from tyr_b200.models.common import KVCache
 from tyr_b200.ops import decode_attention as DA
 from tyr_b200.ops import decode_gemm as DG
 from tyr_b200.ops import delta_rule as DR
 from tyr_b200.ops import fp4
+from tyr_b200.ops import prompt_mix as PM
 
 
 def test_decode_gemm_cpu_fallback_and_predicate():
@@ -57,3 +60,20 @@ def test_slices_fill_the_chip_without_a_thin_last_wave():
     for keys in (1, 64, 65, 300, 100000):
         for B in (1, 7, 150, 100000):
             assert 1 <= DA.pick_splits(B, 2, keys) <= min(32, -(-keys // 64))
+
+
+def test_prompt_operands_refuse_what_the_kernel_would_read_beyond():
+    B, S, H, G, D, half = 2, 5, 4, 2, 64, 16
+    bf = lambda *s: torch.zeros(s, dtype=torch.bfloat16)
+    q, k, v, w, tab = bf(B, S, H * 2 * D), bf(B, S, G * D), bf(B, S, G * D), bf(D), torch.zeros(S, half)
+    store = KVCache.allocate(B, G, S, D, "cpu", torch.bfloat16)
+    assert PM.operands_fit(q, k, v, store, w, w, tab, D, tab)
+    one = torch.zeros(1, half)                                     # a single position's turn broadcast over the prompt
+    for bad in ((q, k, v, store, w, w, one, D, one), (q, k, v, store, w, w, tab, D, one), (q, k, v, store, w[:1], w, tab, D, tab),
+                (q, k[..., :D], v, store, w, w, tab, D, tab), (q, k, v[..., :D], store, w, w, tab, D, tab), (q[..., :H * D + D], k, v, store, w, w, tab, D, tab),
+                (q, k, v, KVCache.allocate(B, G + 1, S, D, "cpu", torch.bfloat16), w, w, tab, D, tab), (q, k[:1], v, store, w, w, tab, D, tab)):
+        assert not PM.operands_fit(*bad)
+    for heads, tables in (((H + 1, G), tab), ((H, G + 1), tab), ((H, G), one)):
+        with pytest.raises(ValueError, match="heads of"):
+            PM.attention_operands(q, 2 * D, k, v, w, w, tables, tables, 1e-6, *heads, D, store)
+    assert store.length == 0

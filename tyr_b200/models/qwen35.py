@@ -255,7 +255,7 @@ def attention_core(cfg: Qwen35Config, q_norm, k_norm, qg, k, v, cos, sin, cache:
     B, S, _ = qg.shape
     H, Hkv, D = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
     if (attn_mask is None and cache is not None and cache.length == 0 and not torch.is_grad_enabled()
-            and prompt_mix.operands_supported(qg, k, v, cache, q_norm, k_norm, cos, D)):
+            and prompt_mix.operands_supported(qg, k, v, cache, q_norm, k_norm, cos, D, sin)):
         # a fresh prompt: one pass makes the queries and the store's rows, which attention reads, and one gates its output
         q = prompt_mix.attention_operands(qg, 2 * D, k, v, q_norm, k_norm, cos, sin, cfg.rms_norm_eps, H, Hkv, D, cache)
         o = attention(q.transpose(1, 2), *cache.view(), causal=True)

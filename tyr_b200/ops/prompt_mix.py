@@ -26,14 +26,23 @@ def _rows(t: torch.Tensor) -> bool:
             and (t.shape[0] == 1 or t.shape[1] == 1 or t.stride(0) == t.shape[1] * t.stride(1)))
 
 
-def operands_supported(q, k, v, store, q_norm, k_norm, cos, D: int) -> bool:
-    """q, k, v: projections [B, S, C]; ``store``: a plain ``KVCache`` of bf16 rows of D; cos: [S, half] fp32."""
-    return (q.is_cuda and q.dtype == k.dtype == v.dtype == torch.bfloat16 and D % 8 == 0 and D <= 256 and cos.dim() == 2 and cos.dtype == torch.float32
-            and cos.is_contiguous() and cos.data_ptr() % 16 == 0 and cos.shape[1] % 8 == 0 and 0 < 2 * cos.shape[1] <= D and _rows(q) and _rows(k) and _rows(v)
+def operands_fit(q, k, v, store, q_norm, k_norm, cos, D: int, sin=None) -> bool:
+    """The part of :func:`operands_supported` that does not ask where the tensors lie.  The kernel reads one row of the tables for each token, so tables
+    that broadcast over the tokens are not for it."""
+    tables = (cos,) if sin is None else (cos, sin)
+    return (q.dtype == k.dtype == v.dtype == torch.bfloat16 and D % 8 == 0 and D <= 256
+            and all(t.shape == cos.shape and t.dim() == 2 and t.shape[0] == q.shape[1] and t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0
+                    for t in tables)
+            and cos.shape[1] % 8 == 0 and 0 < 2 * cos.shape[1] <= D and q.shape[:2] == k.shape[:2] == v.shape[:2] and _rows(q) and _rows(k) and _rows(v)
             and store is not None and not store.ring and store.k.dtype == store.v.dtype == torch.bfloat16 and store.k.is_contiguous() and store.v.is_contiguous()
-            and store.k.shape[0] == q.shape[0] and store.k.shape[3] == store.v.shape[3] == D and store.k.data_ptr() % 16 == 0 and store.v.data_ptr() % 16 == 0
-            and q_norm.dtype == k_norm.dtype == torch.bfloat16 and q_norm.is_contiguous() and k_norm.is_contiguous()
-            and q_norm.data_ptr() % 16 == 0 and k_norm.data_ptr() % 16 == 0)
+            and store.k.shape == store.v.shape and store.k.shape[0] == q.shape[0] and store.k.shape[3] == D
+            and q.shape[2] % (2 * D) == 0 and k.shape[2] == v.shape[2] == store.k.shape[1] * D and store.k.data_ptr() % 16 == 0 and store.v.data_ptr() % 16 == 0
+            and all(w.dtype == torch.bfloat16 and w.shape == (D,) and w.is_contiguous() and w.data_ptr() % 16 == 0 for w in (q_norm, k_norm)))
+
+
+def operands_supported(q, k, v, store, q_norm, k_norm, cos, D: int, sin=None) -> bool:
+    """q, k, v: projections [B, S, C]; ``store``: a plain ``KVCache`` of bf16 rows of D; cos, sin: [S, half] fp32."""
+    return q.is_cuda and operands_fit(q, k, v, store, q_norm, k_norm, cos, D, sin)
 
 
 def attention_operands(q: torch.Tensor, q_head: int, k: torch.Tensor, v: torch.Tensor, q_norm: torch.Tensor, k_norm: torch.Tensor, cos: torch.Tensor,
@@ -41,6 +50,9 @@ def attention_operands(q: torch.Tensor, q_head: int, k: torch.Tensor, v: torch.T
     """Queries [B, S, H, D] (head h of ``q`` starts at column ``h * q_head``) after norm and rotation; keys and values go to the slots of
     ``store`` behind its length, which is advanced."""
     B, S = q.shape[:2]
+    if q.shape[2] != H * q_head or k.shape[2] != G * D or store.k.shape[1] != G or cos.shape[0] != S:
+        raise ValueError(f"{H} and {G} heads of {D} over {S} tokens do not fit projections {tuple(q.shape)}, {tuple(k.shape)}, a store "
+                         f"{tuple(store.k.shape)} and tables {tuple(cos.shape)}")
     if store.length + S > store.cap:
         raise ValueError(f"KV cache overflow: {store.length}+{S} > {store.cap}")
     out = torch.empty((B, S, H, D), dtype=q.dtype, device=q.device)
