@@ -77,3 +77,14 @@ def test_prompt_operands_refuse_what_the_kernel_would_read_beyond():
         with pytest.raises(ValueError, match="heads of"):
             PM.attention_operands(q, 2 * D, k, v, w, w, tables, tables, 1e-6, *heads, D, store)
     assert store.length == 0
+
+
+def test_delta_gates_leave_other_types_and_strides_to_the_plain_operations():
+    wide, p = torch.zeros(2, 7, 24, dtype=torch.bfloat16), torch.zeros(8)
+    b, a = wide[..., :8], wide[..., 8:16]
+    assert DR.gates_fit(b, a, p, p) and DR.gates_fit(b.float(), a.float(), p, p) and DR.gates_fit(b[:, :1], a[:, :1], p, p)
+    for t in (torch.float16, torch.float64):
+        assert not DR.gates_fit(b.to(t), a.to(t), p, p)
+    assert not DR.gates_fit(b, a.float(), p, p) and not DR.gates_fit(b, a, p.half(), p) and not DR.gates_fit(b, a, p, torch.zeros(16)[::2])
+    assert not DR.gates_fit(b[:, :5], a[:, :5], p, p) and not DR.gates_fit(b.mT.contiguous().mT, a.mT.contiguous().mT, p, p)
+    assert not DR.gates_fit(b, a, p[:1], p) and not DR.gates_fit(b, a, p, p.reshape(1, 8))

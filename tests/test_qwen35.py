@@ -262,3 +262,19 @@ def test_gated_norm_of_a_rounded_readout(B, S, Hv, dv):
     od = o.double()
     ref = (od * torch.rsqrt(od.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()).flatten(2) * torch.nn.functional.silu(z.double())
     assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-6).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32, torch.float64])
+def test_gpu_other_types_take_the_plain_operations(dtype):
+    """A prompt and two steps of types that the fused passes do not take, against the CPU in fp32.  The stream and the weights of
+    a few layers rounded to fp16, 2^-11 each time: 2 % of the largest logit is far above it and far below a wrong gate."""
+    cfg = tiny()
+    ids = torch.randint(0, cfg.vocab_size, (2, 11), generator=torch.Generator().manual_seed(1))
+    logits = []
+    for dev, t in (("cpu", torch.float32), ("cuda", dtype)):
+        m = Q.init(cfg, device=dev, dtype=t)
+        with torch.no_grad():
+            c, tok = Q.HybridCache(m, 2, 16), ids.to(dev)
+            logits.append(torch.stack([c.prefill(tok[:, :9]), c.step(tok[:, 9]), c.step(tok[:, 10])]).double().cpu())
+    assert (logits[1] - logits[0]).abs().max() <= 0.02 * logits[0].abs().max()

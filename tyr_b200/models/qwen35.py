@@ -331,7 +331,7 @@ def gated_delta_net_core(cfg: Qwen35Config, m, mixed, z, b, a, state: Optional[L
     q = conv_out[..., :kd].reshape(B, S, Hk, dk)
     k = conv_out[..., kd:2 * kd].reshape(B, S, Hk, dk)
     v = conv_out[..., 2 * kd:].reshape(B, S, Hv, dv)
-    if b.is_cuda and not torch.is_grad_enabled() and b.dtype == a.dtype and m.dt_bias.dtype == m.a_log.dtype == torch.float32:
+    if b.is_cuda and not torch.is_grad_enabled() and dr.gates_fit(b, a, m.dt_bias, m.a_log):
         g, beta = dr.delta_gates(b, a, m.dt_bias, m.a_log)
     else:
         beta = torch.sigmoid(b.float())

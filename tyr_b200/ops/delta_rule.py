@@ -312,6 +312,13 @@ def gdn_decode_fused(mixed, z, b, a, conv_state, conv_w, conv_b, dt_bias, a_log,
 
 
 # ---- any head size, bf16 or fp32, rows of unequal length (csrc/delta_general.cu; plain PyTorch off the GPU) ---------------------
+def gates_fit(b: torch.Tensor, a: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor) -> bool:
+    """What :func:`delta_gates` takes on the GPU: bf16 or fp32 rows, evenly spaced, and one fp32 number a head; callers keep the plain operations for others."""
+    even = lambda t: t.stride(2) == 1 and (t.shape[0] == 1 or t.shape[1] == 1 or t.stride(0) == t.shape[1] * t.stride(1))
+    return (b.dtype == a.dtype and b.dtype in (torch.bfloat16, torch.float32) and b.dim() == 3 and b.shape == a.shape and even(b) and even(a)
+            and all(t.dtype == torch.float32 and t.shape == b.shape[2:] and t.is_contiguous() for t in (dt_bias, a_log)))
+
+
 def delta_gates(b: torch.Tensor, a: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor):
     """b, a: [B, S, Hv] projections (rows may be strided) -> fp32 (g, beta): log decay ``-exp(a_log) softplus(a + dt_bias)`` and
     write strength ``sigmoid(b)``."""
@@ -380,7 +387,7 @@ def gated_norm(o: torch.Tensor, z: torch.Tensor, w: torch.Tensor, eps: float, ac
 def gated_norm_rounded(o: torch.Tensor, z: torch.Tensor, w: torch.Tensor, eps: float) -> Optional[torch.Tensor]:
     """:func:`gated_norm` (SiLU) of a bf16 read-out with a bf16 gain; None for what its kernel does not take."""
     B, S, Hv, dv = o.shape
-    if not (o.is_cuda and o.dtype == z.dtype == w.dtype == torch.bfloat16 and o.is_contiguous() and w.is_contiguous() and dv % 8 == 0 and dv <= 256
+    if not (o.is_cuda and o.dtype == z.dtype == w.dtype == torch.bfloat16 and o.is_contiguous() and w.is_contiguous() and w.shape == (dv,) and dv % 8 == 0 and dv <= 256
             and z.stride(2) == 1 and z.stride(1) % 8 == 0 and (B == 1 or S == 1 or z.stride(0) == S * z.stride(1)) and not torch.is_grad_enabled()
             and all(t.data_ptr() % 16 == 0 for t in (o, z, w))):
         return None
