@@ -243,3 +243,28 @@ def test_gpu_scatter_quantize_equals_gather_quantize(T, k, E, h):
     assert torch.equal(rows, b[3].long())
     sf = lambda t: fp4.unswizzle_scales(t, padded, h // 16)[rows]
     assert torch.equal(a[0][rows], b[0][rows]) and torch.equal(sf(a[1]), sf(b[1])) and torch.equal(a[2][rows], b[2][rows])
+
+
+def test_expert_layouts_follow_their_bank():
+    """A layout belongs to one bank and its present weights: not to a bank that lies where another lay, nor to weights written or replaced since."""
+    from tyr_b200.ops import fp4
+    g = torch.Generator().manual_seed(2)
+    bank = lambda: moe.PackedExperts.quantize(*(torch.randn(*s, generator=g) for s in ((2, 256, 256),) * 3))
+    same = lambda a, b: all(torch.equal(x, y) if isinstance(x, torch.Tensor) else x == y for x, y in zip(vars(a).values(), vars(b).values()))
+    a, b = bank(), bank()
+    first = fp4.prepared(a)
+    assert fp4.prepared(a) is first and same(first, fp4.Fp4Experts.prepare(a))
+    for name, t in vars(a).items():                      # the same storage under another bank, weights, scales and factors alike
+        t.copy_(getattr(b, name))
+    c = moe.PackedExperts(**vars(a))
+    assert same(fp4.prepared(c), fp4.Fp4Experts.prepare(b))
+    assert fp4.prepared(a) is first and same(first, fp4.Fp4Experts.prepare(b))        # written in place: where captured steps read
+    for name in ("up_scale", "down_global", "gate_packed"):
+        d = bank()
+        old = getattr(a, name).clone()
+        kept, now = getattr(a, name), getattr(d, name)
+        setattr(a, name, now)
+        assert fp4.prepared(a) is first and same(first, fp4.Fp4Experts.prepare(a)) and torch.equal(kept, old)
+    held = len(fp4._prepared)
+    del a, c
+    assert len(fp4._prepared) == held - 2

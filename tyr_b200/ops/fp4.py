@@ -14,8 +14,9 @@ from __future__ import annotations
 
 import ctypes
 import os
+import weakref
 from dataclasses import dataclass
-from typing import Optional, Tuple
+from typing import Dict, Optional, Tuple
 
 import torch
 
@@ -168,26 +169,54 @@ class Fp4Experts:
             return torch.stack([g.reshape(E, mi // 64, 64, c), u.reshape(E, mi // 64, 64, c)], dim=2).reshape(E, 2 * mi, c)
 
         u8 = lambda t: t.view(torch.uint8) if t.dtype != torch.uint8 else t
+        own = lambda t: t.float().clone(memory_format=torch.contiguous_format)
         gu_packed = tile_weights(inter(ex.gate_packed, ex.up_packed).contiguous())
         gu_sf = swizzle_scales(inter(u8(ex.gate_scale), u8(ex.up_scale)))
-        return Fp4Experts(gu_packed, gu_sf.contiguous(), ex.gate_global.float().contiguous(), ex.up_global.float().contiguous(),
-                          tile_weights(ex.down_packed.contiguous()), swizzle_scales(u8(ex.down_scale)).contiguous(),
-                          ex.down_global.float().contiguous(), h, mi)
+        return Fp4Experts(gu_packed, gu_sf.contiguous(), own(ex.gate_global), own(ex.up_global), tile_weights(ex.down_packed.contiguous()),
+                          swizzle_scales(u8(ex.down_scale)).contiguous(), own(ex.down_global), h, mi)
 
 
-_prepared = {}
+# id of a bank -> (the bank, its tensors as they were laid out, the layout).  A layout lives as long as its bank.
+_prepared: Dict[int, Tuple[weakref.ref, Tuple, Fp4Experts]] = {}
+
+
+def _tensors(ex) -> Tuple[torch.Tensor, ...]:
+    return (ex.gate_packed, ex.gate_scale, ex.gate_global, ex.up_packed, ex.up_scale, ex.up_global, ex.down_packed, ex.down_scale, ex.down_global)
+
+
+def _version(t: torch.Tensor) -> int:
+    return 0 if t.is_inference() else t._version             # inference tensors keep no count
 
 
 def prepared(ex) -> Fp4Experts:
-    """Cached per bank (keyed by the storage addresses of its packed tensors)."""
-    key = (ex.gate_packed.data_ptr(), ex.up_packed.data_ptr(), ex.down_packed.data_ptr(), ex.gate_packed.numel())
+    """The layout of a bank, made once.  Weights that were replaced or written since are laid out again, into the same storage where
+    it fits, so that steps captured before read the new ones."""
+    key, tensors = id(ex), _tensors(ex)
     hit = _prepared.get(key)
-    if hit is None:
-        hit = Fp4Experts.prepare(ex)
-        if len(_prepared) > 512:
-            _prepared.clear()
-        _prepared[key] = hit
-    return hit
+    if hit is not None and hit[0]() is not ex:               # an address alone may belong to another bank by now
+        hit = None
+    if hit is not None and all(r() is t and v == _version(t) for (r, v), t in zip(hit[1], tensors)):
+        return hit[2]
+    dev = tensors[0].device
+    # on the default stream like the weights: what a side stream allocates could be handed out there again while another stream's kernels still read it
+    home = torch.cuda.default_stream(dev) if dev.type == "cuda" and not torch.cuda.is_current_stream_capturing() else None
+    if home is not None:
+        cur = torch.cuda.current_stream(dev)
+        home.wait_stream(cur)
+    with torch.cuda.stream(home):
+        layout = Fp4Experts.prepare(ex)
+        if hit is not None:
+            old, new = vars(hit[2]), vars(layout)
+            if all(not isinstance(t, torch.Tensor) and t == old[n] or isinstance(t, torch.Tensor) and t.shape == old[n].shape and t.device == old[n].device
+                   for n, t in new.items()):
+                for n, t in new.items():
+                    if isinstance(t, torch.Tensor):
+                        old[n].copy_(t)
+                layout = hit[2]
+    if home is not None:
+        cur.wait_stream(home)
+    _prepared[key] = (weakref.ref(ex, lambda _: _prepared.pop(key, None)), tuple((weakref.ref(t), _version(t)) for t in tensors), layout)
+    return layout
 
 
 # ---- device ops --------------------------------------------------------------------------------------------------
