@@ -38,6 +38,8 @@ def test_fixed_slot_predicate():
     assert not fp4.fixed_slots_supported(129, 2048)            # an expert could receive more rows than a slot tile holds
     assert not fp4.fixed_slots_supported(64, 2048 + 64)        # hidden size must be a multiple of 256
     assert fp4.FIXED_SLOT_MAX_TOKENS == 128
+    assert fp4.scatter_fits(256) and fp4.scatter_fits(21760) and not fp4.scatter_fits(22016)      # four rows of codes and scales in 48 KB
+    assert not fp4.fixed_slots_supported(64, 22016)
 
 
 def test_gdr_tile_predicate_needs_aligned_rows(monkeypatch):

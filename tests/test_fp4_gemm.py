@@ -141,3 +141,24 @@ def test_fp4_moe_tensor_core_path(T, E, k, h, mi, skew):
     w4a16 = M.moe_eager(x, ids.long(), w, gd, ud, dd).float() + add.float()
     nrmse = ((out.float() - w4a16).pow(2).mean().sqrt() / (w4a16.pow(2).mean().sqrt() + 1e-12)).item()
     assert nrmse <= 0.35, nrmse
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("path", ["gemm", "gemm_sorted"])
+@pytest.mark.parametrize("T,E,k,h,mi", [(130, 8, 2, 512, 256), (5, 3, 2, 21760, 256), (5, 3, 2, 22016, 256)])
+def test_fp4_layer_of_any_width(path, T, E, k, h, mi):
+    """The whole layer as it is called, with pairs that have no expert, at the widest rows of the scatter and past them.  The bounds are those of
+    ``test_fp4_moe_tensor_core_path``; a sum over 22016 channels has sqrt(22016 / 1024) times the spread of that test's."""
+    dev = torch.device("cuda:0")
+    ex = _experts(E, mi, h, dev, 3)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(T, h, device=dev, generator=g).bfloat16()
+    ids = torch.stack([torch.randperm(E, device=dev, generator=g)[:k] for _ in range(T)]).to(torch.int32)
+    ids[1, 0] = E
+    w = torch.rand(T, k, device=dev, generator=g) + 0.1
+    out = M.moe_fp4_forward(x, ids, w, ex, force_path=path)
+    routed = torch.where(ids < E, w, torch.zeros_like(w))
+    ref = fp4.moe_fp4_tc_reference(x, ids.long() % E, routed, ex)
+    d = (out.float() - ref.float()).abs()
+    assert (d > 0.5 * (h / 1024) ** 0.5 + 0.02 * ref.float().abs()).float().mean().item() < 2e-3
+    assert _rel(out, ref) < 3e-2, _rel(out, ref)

@@ -229,7 +229,7 @@ def gather_quantize(x: torch.Tensor, order: Optional[torch.Tensor], ids: Optiona
     packed = torch.empty((padded_rows, h // 2), dtype=torch.uint8, device=dev)
     sf = torch.empty(padded_rows * (h // 16), dtype=torch.uint8, device=dev)
     rs = torch.empty(padded_rows, dtype=torch.float32, device=dev)
-    ppos = torch.zeros(n, dtype=torch.int32, device=dev) if order is not None else None
+    ppos = torch.full((n,), -1, dtype=torch.int32, device=dev) if order is not None else None        # -1: a pair without an expert
     E = (offsets.numel() - 1) if offsets is not None else 1
     check(lib().tyr_fp4_gather_quantize(ptr(x.contiguous()), ptr(order), ptr(ids), ptr(offsets), ptr(tiles), ptr(packed), ptr(sf),
                                         ptr(rs), ptr(ppos), n, k, h, E, cur_stream(dev)), "fp4_gather_quantize")
@@ -263,6 +263,11 @@ def grouped_gemm_fp4(a_packed, a_sf, a_row_scale, w_packed, w_sf, w_global, tile
     return out if mode == 0 else (out, out_sf)
 
 
+def scatter_fits(h: int) -> bool:
+    """The rows of the four tokens of a scatter CTA, codes and block scales, fit its 48 KB of shared memory (h <= 21760)."""
+    return 4 * (-(-(h // 2 + h // 16) // 16) * 16) <= 48 * 1024
+
+
 def scatter_quantize(x: torch.Tensor, ids: torch.Tensor, pos: torch.Tensor, offsets: torch.Tensor, tiles: torch.Tensor, padded_rows: int):
     """:func:`gather_quantize` of the sorted layout the other way round: every token is quantised once and its row written to each of its pairs'
     places.  ids int32 [T, k], ``pos`` their expert-major positions -> the same four results."""
@@ -279,7 +284,8 @@ def scatter_quantize(x: torch.Tensor, ids: torch.Tensor, pos: torch.Tensor, offs
 
 def moe_fp4_tc_forward(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, ex, offsets, order, tiles,
                        add: Optional[torch.Tensor] = None, pos: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """x [T, h] bf16, ids int32 [T, k], weights fp32 [T, k]; ``offsets`` / ``order`` / ``tiles`` from ``ops.moe.layout``, and its ``pos`` where there is one.
+    """x [T, h] bf16, ids int32 [T, k], weights fp32 [T, k]; ``offsets`` / ``order`` / ``tiles`` from ``ops.moe.layout``, and its ``pos``: without it, and for
+    rows that do not fit the scatter's shared memory, every pair's row is quantised for itself.
     Everything stays on the device: the row count of the padded layout is bounded on the host by T * k + 127 * E."""
     from . import moe as M
     T, h = x.shape
@@ -290,7 +296,7 @@ def moe_fp4_tc_forward(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor
     padded = ((pairs + 127 * min(E, pairs) + 127) // 128) * 128
     st = cur_stream(x.device)
     ids32 = ids.to(torch.int32).contiguous()
-    xq, xsf, xrs, ppos = (gather_quantize(x, order, ids32.reshape(-1), offsets, tiles, k, padded, pairs) if pos is None else
+    xq, xsf, xrs, ppos = (gather_quantize(x, order, ids32.reshape(-1), offsets, tiles, k, padded, pairs) if pos is None or not scatter_fits(h) else
                           scatter_quantize(x, ids32, pos, offsets, tiles, padded))
     hq, hsf = grouped_gemm_fp4(xq, xsf, xrs, w4.gu_packed, w4.gu_sf, w4.gate_global, tiles, offsets,
                                2 * mi, h, mode=1, w_global2=w4.up_global)
@@ -308,7 +314,7 @@ _FIXED_SLOTS = os.environ.get("TYR_MOE_FIXED_SLOTS", "1") != "0"     # 0: always
 
 
 def fixed_slots_supported(T: int, h: int) -> bool:
-    return (_FIXED_SLOTS and T <= FIXED_SLOT_MAX_TOKENS and h % 256 == 0
+    return (_FIXED_SLOTS and T <= FIXED_SLOT_MAX_TOKENS and h % 256 == 0 and scatter_fits(h)
             and hasattr(lib(), "tyr_fp4_scatter_quantize_fixed"))
 
 
