@@ -10,6 +10,9 @@ from tyr_b200.ops import decode_gemm as DG
 from tyr_b200.ops import delta_rule as DR
 from tyr_b200.ops import fp4
 from tyr_b200.ops import prompt_mix as PM
+from tyr_b200.ops import rope as RO
+from tyr_b200.ops import skinny as SK
+from tyr_b200.ops.gemm import gemm, gemm_many
 
 
 def test_decode_gemm_cpu_fallback_and_predicate():
@@ -90,3 +93,43 @@ def test_delta_gates_leave_other_types_and_strides_to_the_plain_operations():
     assert not DR.gates_fit(b, a.float(), p, p) and not DR.gates_fit(b, a, p.half(), p) and not DR.gates_fit(b, a, p, torch.zeros(16)[::2])
     assert not DR.gates_fit(b[:, :5], a[:, :5], p, p) and not DR.gates_fit(b.mT.contiguous().mT, a.mT.contiguous().mT, p, p)
     assert not DR.gates_fit(b, a, p[:1], p) and not DR.gates_fit(b, a, p, p.reshape(1, 8))
+
+
+def test_product_forms_refuse_operands_of_other_types_and_devices():
+    bf = lambda *s: torch.ones(s, dtype=torch.bfloat16)
+    a, w, aux, gate = bf(6, 16), bf(8, 16), bf(6, 8), bf(2, 8)
+    assert gemm(a, w, up=w, act="swiglu").shape == gemm(a, w, act="gated_add", aux=aux, gate=gate).shape == (6, 8)
+    for t in (torch.float32, torch.int8, torch.float16):
+        with pytest.raises(TypeError, match="up"):
+            gemm(a, w, up=w.to(t), act="swiglu")
+    there = torch.device("meta")
+    for kw in (dict(up=w.to(there), act="swiglu"), dict(act="gated_add", aux=aux, gate=gate.to(there))):
+        with pytest.raises(ValueError, match="meta"):
+            gemm(a, w, **kw)
+    for short in (aux[:5], aux[:, :4], aux[None]):
+        with pytest.raises(ValueError, match="gated_add"):
+            gemm(a, w, act="gated_add", aux=short, gate=gate)
+    with pytest.raises(ValueError, match="meta"):
+        gemm_many(a, [w, w.to(there)])
+
+
+def test_norm_products_refuse_operands_that_do_not_go_together():
+    bf = lambda *s: torch.ones(s, dtype=torch.bfloat16)
+    x, n, w = bf(3, 64), bf(64), bf(16, 64)
+    assert SK.norm_fit(x, None, n, [w]) and SK.norm_fit(x, x, n, [w, w])
+    for bad in ((x, x.float(), n, [w]), (x, x[:2], n, [w]), (x, x, n.float(), [w]), (x, x, n[:32], [w]), (x, x, n, [w, w.float()]), (x, x, n, [w[:, :32]]),
+                (x, x, n, [w.to("meta")])):
+        assert not SK.norm_fit(*bad)
+    with pytest.raises(ValueError, match="bf16 operands"):
+        SK.skinny_norm_many(x, x.float(), n, 1e-6, [w])
+    with pytest.raises(ValueError, match="differ"):
+        SK.skinny_norm_swiglu(x, x, n, 1e-6, w, w[:8])
+
+
+def test_turned_queries_and_keys_go_together():
+    bf, tab, pos = lambda *s: torch.ones(s, dtype=torch.bfloat16), torch.ones(9, 8), torch.zeros(3, dtype=torch.int32)
+    q, k, w = bf(3, 4, 32), bf(3, 2, 32), bf(32)
+    assert RO.qk_fit(q, k, tab, tab, w, w, pos)
+    for bad in ((q, k[:2], tab, tab, w, w, pos), (q, bf(3, 2, 16), tab, tab, w, w, pos), (q, k, tab, tab[:4], w, w, pos), (q, k, tab, tab, w[:1], w, pos),
+                (q, k, tab, tab, w, w, pos[:1]), (q, k, tab, tab, w, w.float(), pos), (q, k, tab, tab, w, w, pos.to("meta"))):
+        assert not RO.qk_fit(*bad)

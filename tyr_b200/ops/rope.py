@@ -129,13 +129,19 @@ def rope_norm(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, *, weight=N
     return out.to(x.dtype)
 
 
+def qk_fit(q, k, cos, sin, q_weight, k_weight, positions) -> bool:
+    """Queries and keys of the same rows and head size, with gains, tables and positions as the one launch reads them."""
+    low = lambda t: t.dtype == torch.bfloat16 and t.is_contiguous() and t.shape == q.shape[2:]
+    return (q.dtype == k.dtype == torch.bfloat16 and q.shape[::2] == k.shape[::2] and q.stride(2) == k.stride(2) == 1 and low(q_weight) and low(k_weight)
+            and cos.dtype == sin.dtype == torch.float32 and cos.shape == sin.shape and cos.is_contiguous() and sin.is_contiguous()
+            and positions.dtype == torch.int32 and positions.shape == q.shape[:1] and all(t.device == q.device for t in (k, cos, sin, q_weight, k_weight, positions)))
+
+
 def rope_norm_qk(q: torch.Tensor, k: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, *, q_weight: torch.Tensor, k_weight: torch.Tensor,
                  positions: torch.Tensor, eps: float = EPS, one_plus_w: bool = False):
     """:func:`rope_norm` of queries [rows, H, D] and keys [rows, G, D] in one launch; rows and heads may be strided."""
     rot = 2 * cos.shape[1]
-    low = lambda t: t.dtype == torch.bfloat16 and t.is_contiguous()
-    if not (q.is_cuda and q.dtype == k.dtype == torch.bfloat16 and q.stride(2) == k.stride(2) == 1 and low(q_weight) and low(k_weight)
-            and cos.dtype == sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous() and positions.dtype == torch.int32):
+    if not (q.is_cuda and qk_fit(q, k, cos, sin, q_weight, k_weight, positions)):
         kw = dict(positions=positions, rot=rot, eps=eps, one_plus_w=one_plus_w)
         return rope_norm(q, cos, sin, weight=q_weight, **kw), rope_norm(k, cos, sin, weight=k_weight, **kw)
     rows, H, D = q.shape

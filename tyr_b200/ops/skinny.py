@@ -73,7 +73,7 @@ def skinny_many(x2: torch.Tensor, ws: Sequence[torch.Tensor], splits: int = 0) -
     M, K = x2.shape
     if not x2.is_cuda:
         return [(x2.float() @ w.float().T).to(x2.dtype) for w in ws]
-    if not (all(w.shape[1] == K and w.dtype == torch.bfloat16 and w.stride(1) == 1 for w in ws) and x2.dtype == torch.bfloat16 and x2.stride(1) == 1):
+    if not (all(w.shape[1] == K and w.dtype == torch.bfloat16 and w.stride(1) == 1 and w.device == x2.device for w in ws) and x2.dtype == torch.bfloat16 and x2.stride(1) == 1):
         raise ValueError("skinny_many takes bf16 rows and matrices over one contraction")
     n = len(ws)
     ys = [torch.empty((M, w.shape[0]), dtype=torch.bfloat16, device=x2.device) for w in ws]
@@ -93,7 +93,17 @@ def norm_supported(x2: torch.Tensor, norm_w: torch.Tensor, ws: Sequence[torch.Te
             and norm_w.dtype == torch.bfloat16 and norm_w.is_contiguous() and norm_w.data_ptr() % 16 == 0 and norm_w.numel() == K)
 
 
-def _norm_operands(x2, resid):
+def norm_fit(x2: torch.Tensor, resid: Optional[torch.Tensor], norm_w: torch.Tensor, ws: Sequence[torch.Tensor]) -> bool:
+    """Types, shapes and devices of the norm's operands and of the matrices behind it go together."""
+    M, K = x2.shape
+    return (all(t.dtype == torch.bfloat16 and t.device == x2.device for t in (x2, norm_w, *ws, *(() if resid is None else (resid,))))
+            and (resid is None or resid.shape == x2.shape) and norm_w.shape == (K,) and norm_w.is_contiguous()
+            and all(w.dim() == 2 and w.shape[1] == K and w.stride(1) == 1 for w in ws))
+
+
+def _norm_operands(x2, resid, norm_w, ws):
+    if not norm_fit(x2, resid, norm_w, ws):
+        raise ValueError(f"norm and products of rows {tuple(x2.shape)} ({x2.dtype}) take bf16 operands over the same channels, on one device")
     M, K = x2.shape
     r = None if resid is None else resid if resid.stride(1) == 1 and resid.stride(0) % 8 == 0 and resid.data_ptr() % 16 == 0 else resid.contiguous()
     return r, None if r is None else torch.empty((M, K), dtype=x2.dtype, device=x2.device), 0 if r is None else r.stride(0)
@@ -102,7 +112,7 @@ def _norm_operands(x2, resid):
 def skinny_norm_many(x2: torch.Tensor, resid: Optional[torch.Tensor], norm_w: torch.Tensor, eps: float, ws: Sequence[torch.Tensor], one_plus_w: bool = False):
     """``([h w^T for w in ws], s)`` with ``s = x2 + resid`` (bf16; x2 itself without ``resid``) and h its RMS norm times the gain, in one launch."""
     M, K = x2.shape
-    r, out, ldr = _norm_operands(x2, resid)
+    r, out, ldr = _norm_operands(x2, resid, norm_w, ws)
     n = len(ws)
     ys = [torch.empty((M, w.shape[0]), dtype=torch.bfloat16, device=x2.device) for w in ws]
     P, L, I = ctypes.c_void_p * n, ctypes.c_longlong * n, ctypes.c_int * n
@@ -117,7 +127,9 @@ def skinny_norm_swiglu(x2: torch.Tensor, resid: Optional[torch.Tensor], norm_w: 
     """``(silu(h gate_w^T) * (h up_w^T), s)`` with h and s as in :func:`skinny_norm_many`."""
     M, K = x2.shape
     N = gate_w.shape[0]
-    r, out, ldr = _norm_operands(x2, resid)
+    if up_w.shape != gate_w.shape or up_w.stride() != gate_w.stride():
+        raise ValueError(f"gate and up matrices {tuple(gate_w.shape)} and {tuple(up_w.shape)} differ in shape or strides")
+    r, out, ldr = _norm_operands(x2, resid, norm_w, (gate_w, up_w))
     y = torch.empty((M, N), dtype=torch.bfloat16, device=x2.device)
     check(lib().tyr_skinny_norm_swiglu_bf16(ptr(x2), ptr(r), ptr(norm_w), ptr(out), x2.stride(0), ldr, ptr(gate_w), ptr(up_w), ptr(y), gate_w.stride(0), M, N, K,
                                             eps, 1 if one_plus_w else 0, cur_stream(x2.device)), "skinny_norm_swiglu")
