@@ -124,7 +124,7 @@ __device__ __forceinline__ float apply_act(float v, int act) {
 //   ACT 3: v = alpha * acc * 2 * sqrt(aux)     (gradient of y = relu(z)^2 given aux = y)
 //   ACT 7: alpha * silu(acc) (+ ...)
 //   ACT 9: gelu(acc) * aux
-//   ACT 10: aux + gate * acc (`gt`: the chunk's gates)
+//   ACT 10: aux + gate * acc, in the epilogue itself (a gate per column)
 //   ACT 6: xIELU of acc: alpha z^2 + z / 2 above zero, beta (e^z - 1 - z) + z / 2 below (no aux)
 template <int ACT>
 __device__ __forceinline__ void epi_chunk(const uint32_t (&r)[32], const float (&ax)[32], bool use_aux, float alpha,
@@ -969,7 +969,8 @@ static int launch_gemm(const TyrGemmArgs& a, const CUtensorMap& tmA, const CUten
   }
   if (a.out_mode != 2 && tiles < grid) grid = static_cast<int>(tiles);
   p.raster_m = (a.group_offsets == nullptr && tp.tp_mode == 0 && a.M < (a.segs > 0 ? seg_cols : a.N) && g_raster_m) ? 1 : 0;
-  p.l2_prefetch = (a.group_offsets == nullptr && tp.tp_mode == 0) ? g_l2_prefetch : 0;
+  // the walk ahead knows one B and batch coordinates: not the products of several matrices, nor gate and up matrices apart
+  p.l2_prefetch = (a.group_offsets == nullptr && tp.tp_mode == 0 && a.segs == 0 && a.B2 == nullptr) ? g_l2_prefetch : 0;
   p.sk_slabs = 0;
   if (a.out_mode == 2) {
     const int num_kb = (a.K + BK - 1) / BK;
