@@ -864,3 +864,34 @@ def test_decode_attention_merges_more_slices_than_lanes(form, splits, monkeypatc
     if form == "plain":
         with pytest.raises(RuntimeError):
             da.decode_attention(*(t.cuda() for t in (q, k, v, kc, vc, both)), splits=65)
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,T", [(7, 10, 10, 2048), (9, 20, 10, 1536)])
+def test_flash_attention_heads_beyond_one_group(B, Hq, Hkv, T):
+    """Causal work is handed out by groups of heads that fit the L2 (64 heads of 2048 tokens).  More heads than one group, the last group short: every head's
+    result and gradients are those of its batch row alone, which is one group, bit for bit."""
+    from tyr_b200.ops import flash
+    g = torch.Generator(device="cuda").manual_seed(T)
+    r = lambda H: torch.randn(B, T, H, 128, device=_dev(), generator=g).bfloat16()
+    q, k, v, do = r(Hq), r(Hkv), r(Hkv), r(Hq)
+
+    def both(s):
+        o, lse = flash.flash_fwd_bthd(q[s], k[s], v[s], causal=True, window=None, scale=None)
+        return (o, lse, *flash.flash_bwd_bthd(do[s], q[s], k[s], v[s], o, lse, causal=True, window=None, scale=None)[:3])
+    whole = both(slice(0, B))
+    for b in range(B):
+        for x, y in zip(whole, both(slice(b, b + 1))):
+            assert torch.equal(x[b:b + 1], y), b
+
+
+@pytest.mark.parametrize("iters", [0, 1, 4, 5])
+@pytest.mark.parametrize("shape", [(3, 128, 128), (2, 64, 200), (2, 328, 72), (1, 8, 8)])
+def test_newton_schulz_moved_equals_the_copying_form(shape, iters):
+    """Wide, tall and square, odd and even: the result in x's storage or in the scratch is the one that the copying form returns."""
+    from tyr_b200.ops import polar
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    x = torch.randn(shape, device=_dev(), generator=g)
+    x = (x / x.norm(dim=(1, 2), keepdim=True)).bfloat16()
+    want = polar.newton_schulz_(x.clone(), iters)
+    got = polar.newton_schulz_moved(x.clone(), iters)
+    assert got.shape == x.shape and torch.equal(got, want) and (iters == 0 or not torch.equal(got, x))
