@@ -163,11 +163,6 @@ def init(cfg: FluxConfig, device="cpu", dtype=torch.float32, seed=0) -> FluxMode
                      mk(6 * h, h), mk(6 * h, h), mk(3 * h, h), mk(cfg.in_channels, h), mk(2 * h, h))
 
 
-def modulation(vec: torch.Tensor, w: torch.Tensor, n: int) -> torch.Tensor:
-    """silu(vec) @ w^T -> [B, n, hidden]."""
-    return lin(F.silu(vec), w).reshape(vec.shape[0], n, -1)
-
-
 def _qk(cfg, qkv, norm: QKNorm, pe):
     B, S, _ = qkv.shape
     H, D = cfg.num_heads, cfg.head_dim

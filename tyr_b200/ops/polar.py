@@ -68,16 +68,6 @@ def _tall_step(g: torch.Tensor, a: float, b: float, c: float) -> torch.Tensor:
 _scratch = {}
 
 
-def _chain_scratch(x, need: int) -> torch.Tensor:
-    key = (x.device.index, need)
-    buf = _scratch.get(key)
-    if buf is None:
-        buf = torch.empty(need, dtype=torch.uint8, device=x.device)
-        _scratch.clear()
-        _scratch[key] = buf
-    return buf
-
-
 def newton_schulz_moved(x: torch.Tensor, num_iters: int) -> torch.Tensor:
     """:func:`newton_schulz_` of a contiguous stacked batch whose storage the iterations may use: the result is x's storage or a fresh buffer, and x is not
     kept."""
@@ -101,7 +91,12 @@ def _native_chain(x: torch.Tensor, num_iters: int) -> torch.Tensor:
     B, R, C = xb.shape
     out = xb.contiguous().clone()
     need = lib().tyr_newton_schulz_scratch_bytes(B, R, C)
-    buf = _chain_scratch(x, need)
+    key = (x.device.index, need)
+    buf = _scratch.get(key)
+    if buf is None:
+        buf = torch.empty(need, dtype=torch.uint8, device=x.device)
+        _scratch.clear()
+        _scratch[key] = buf
     a, b, c = MUON_COEFFS
     check(lib().tyr_newton_schulz_bf16(ptr(out), ptr(buf), need, B, R, C, num_iters, a, b, c,
                                        ptr(err_word(x.device)), cur_stream(x.device)), "newton_schulz")
