@@ -491,8 +491,9 @@ __device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
 // ----------------------------------------------------------------------------------------
 // Order of the attention kernels' work: `tiles` tiles of each of `heads` (batch, head) pairs.  Causal tiles differ in work by their rank in the sequence, and a
 // hardware scheduler that gets them head by head ends on heavy ones: 80 heads of 2048 tokens are 39 key blocks an SM with tiles of 2 to 16, 48 heads of
-// 1000 tokens 6.5 with tiles of 2 to 8.  So the heaviest tiles of a group of heads come first, and a group's operands fit the L2.  Causal, forward / backward, us: 8 x 10 heads
-// of 2048 tokens 210 / 466 head by head and 166 / 366 now, 8 x 6 heads of 1000 tokens 60 / 101 and 49 / 92.
+// 1000 tokens 6.5 with tiles of 2 to 8.  So the heaviest tiles of a group of heads come first, and a group's operands fit the L2.  Causal, forward / backward, us, head by head
+// and in this order: 8 x 10 heads of 2048 tokens 210 / 466 and 166 / 366, 8 x 6 heads of 1000 tokens 60 / 101 and 49 / 92.  With masks as two bounds a row as well
+// (csrc/attention_fwd.cu) they take 129 / 368 and 30 / 85.
 // ----------------------------------------------------------------------------------------
 struct TileOrder { int tiles, heads, group; };
 constexpr long long kTileGroupBytes = 64LL << 20;

@@ -34,8 +34,8 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
     "--expt-relaxed-constexpr",
 ]
-# Units whose results are carried through thousands of steps or stand for the fp32 mode: correctly rounded division, square root
-# and library exponentials.  Every other unit is compiled with fast math.
+# Units whose results are carried through thousands of steps, stand for the fp32 mode or go to a store that later steps read: division, square root and
+# functions as they are written (a kernel that takes an approximation names it) and no flushing of denormals.  Every other unit is compiled with fast math.
 PRECISE_UNITS = ("delta_general", "attention_general", "depth_average", "flux_tables", "gates", "joint_attention", "latent", "lightning", "mix_conv", "prompt_mix", "rotary_store",
                  "selective_scan")
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-Wall", "-pthread"]
