@@ -314,9 +314,13 @@ def gdn_decode_fused(mixed, z, b, a, conv_state, conv_w, conv_b, dt_bias, a_log,
 # ---- any head size, bf16 or fp32, rows of unequal length (csrc/delta_general.cu; plain PyTorch off the GPU) ---------------------
 def gates_fit(b: torch.Tensor, a: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor) -> bool:
     """What :func:`delta_gates` takes on the GPU: bf16 or fp32 rows, evenly spaced, and one fp32 number a head; callers keep the plain operations for others."""
-    even = lambda t: t.stride(2) == 1 and (t.shape[0] == 1 or t.shape[1] == 1 or t.stride(0) == t.shape[1] * t.stride(1))
-    return (b.dtype == a.dtype and b.dtype in (torch.bfloat16, torch.float32) and b.dim() == 3 and b.shape == a.shape and even(b) and even(a)
-            and all(t.dtype == torch.float32 and t.shape == b.shape[2:] and t.is_contiguous() for t in (dt_bias, a_log)))
+    shape = b.shape
+    if b.dtype != a.dtype or b.dtype not in (torch.bfloat16, torch.float32) or len(shape) != 3 or a.shape != shape:
+        return False
+    for t in (b, a):
+        if not t.is_contiguous() and (t.stride(2) != 1 or (shape[0] > 1 and shape[1] > 1 and t.stride(0) != shape[1] * t.stride(1))):
+            return False
+    return (dt_bias.dtype == a_log.dtype == torch.float32 and dt_bias.shape == a_log.shape == shape[2:] and dt_bias.is_contiguous() and a_log.is_contiguous())
 
 
 def delta_gates(b: torch.Tensor, a: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor):

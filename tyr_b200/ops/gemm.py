@@ -103,11 +103,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_layout: str = "K", b_layout: str
             raise ValueError("gemm `up` goes with a gated activation and a K-major gate matrix of the same shape and strides")
         if up.dtype != b.dtype:
             raise TypeError(f"gemm `up` of {up.dtype} beside a gate matrix of {b.dtype}")
+        if up.device != a.device:
+            raise ValueError(f"gemm operands on {a.device} and {up.device}")
         N *= 2
     if K != K2:
         raise ValueError(f"gemm reduction mismatch: {tuple(a.shape)} ({a_layout}) vs {tuple(b.shape)} ({b_layout})")
-    if any(t is not None and t.device != a.device for t in (up, gate)):
-        raise ValueError(f"gemm operands on {a.device} and {[str(t.device) for t in (up, gate) if t is not None]}")
     batch = max(batch_a, batch_b)
     if batch_a not in (1, batch) or batch_b not in (1, batch):
         raise ValueError("gemm batch mismatch")
@@ -115,6 +115,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_layout: str = "K", b_layout: str
     if act == "gated_add" and (aux is None or gate is None or gate.dim() != 2 or gate.shape[1] != N or M % gate.shape[0] or gate.stride(1) != 1 or N % 8
                                or a.dim() != 2 or aux.shape != (M, N) or accumulate or out_dtype == torch.float32):
         raise ValueError("gated_add takes its addend as aux [M, N] and gates [sets, N] with N % 8 == 0 and M a multiple of the sets")
+    if act == "gated_add" and gate.device != a.device:
+        raise ValueError(f"gemm operands on {a.device} and {gate.device}")
     if act == "gelu_mul" and aux is None:
         raise ValueError("gelu_mul takes its factor as aux")
     if gated:
@@ -201,7 +203,8 @@ MAX_MATRICES = 4         # of one launch (gemm_many)
 def gemm_many(a: torch.Tensor, bs: Sequence[torch.Tensor], *, bn: int = 0, tile_rows: int = 0) -> List[torch.Tensor]:
     """``[a @ b^T for b in bs]`` in one launch: a [M, K] and two to four matrices [N_i, K] (rows may be strided), bf16."""
     M, K = a.shape
-    if any(b.device != a.device for b in bs):
+    dev = a.device
+    if any([b.device != dev for b in bs]):
         raise ValueError(f"gemm_many operands on {a.device} and {[str(b.device) for b in bs]}")
     if not a.is_cuda:
         return [_reference(a, b, "K", "K", None, 1.0, 0.0, None, a.dtype) for b in bs]

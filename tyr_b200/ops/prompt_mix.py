@@ -29,15 +29,18 @@ def _rows(t: torch.Tensor) -> bool:
 def operands_fit(q, k, v, store, q_norm, k_norm, cos, D: int, sin=None) -> bool:
     """The part of :func:`operands_supported` that does not ask where the tensors lie.  The kernel reads one row of the tables for each token, so tables
     that broadcast over the tokens are not for it."""
-    tables = (cos,) if sin is None else (cos, sin)
-    return (q.dtype == k.dtype == v.dtype == torch.bfloat16 and D % 8 == 0 and D <= 256
-            and all(t.shape == cos.shape and t.dim() == 2 and t.shape[0] == q.shape[1] and t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0
-                    for t in tables)
-            and cos.shape[1] % 8 == 0 and 0 < 2 * cos.shape[1] <= D and q.shape[:2] == k.shape[:2] == v.shape[:2] and _rows(q) and _rows(k) and _rows(v)
-            and store is not None and not store.ring and store.k.dtype == store.v.dtype == torch.bfloat16 and store.k.is_contiguous() and store.v.is_contiguous()
-            and store.k.shape == store.v.shape and store.k.shape[0] == q.shape[0] and store.k.shape[3] == D
-            and q.shape[2] % (2 * D) == 0 and k.shape[2] == v.shape[2] == store.k.shape[1] * D and store.k.data_ptr() % 16 == 0 and store.v.data_ptr() % 16 == 0
-            and all(w.dtype == torch.bfloat16 and w.shape == (D,) and w.is_contiguous() and w.data_ptr() % 16 == 0 for w in (q_norm, k_norm)))
+    bf16, f32 = torch.bfloat16, torch.float32
+    B, S, C = q.shape
+    sin = cos if sin is None else sin
+    if not (q.dtype == k.dtype == v.dtype == q_norm.dtype == k_norm.dtype == bf16 and cos.dtype == sin.dtype == f32 and D % 8 == 0 and D <= 256
+            and cos.dim() == 2 and store is not None and not store.ring):
+        return False
+    half, sk, sv = cos.shape[1], store.k, store.v
+    return (cos.shape == sin.shape == (S, half) and half % 8 == 0 and 0 < 2 * half <= D and cos.is_contiguous() and sin.is_contiguous()
+            and C % (2 * D) == 0 and k.shape == v.shape == (B, S, sk.shape[1] * D) and _rows(q) and _rows(k) and _rows(v)
+            and sk.dtype == sv.dtype == bf16 and sk.shape == sv.shape and sk.shape[0] == B and sk.shape[3] == D and sk.is_contiguous() and sv.is_contiguous()
+            and q_norm.shape == k_norm.shape == (D,) and q_norm.is_contiguous() and k_norm.is_contiguous()
+            and (cos.data_ptr() | sin.data_ptr() | sk.data_ptr() | sv.data_ptr() | q_norm.data_ptr() | k_norm.data_ptr()) % 16 == 0)
 
 
 def operands_supported(q, k, v, store, q_norm, k_norm, cos, D: int, sin=None) -> bool:
