@@ -699,7 +699,10 @@ extern "C" TYR_EXPORT int tyr_rmsnorm_weighted(const void* x, const void* w, con
   a.gate = (const __nv_bfloat16*)gate; a.resid = (const __nv_bfloat16*)resid;
   a.resid_out = (__nv_bfloat16*)resid_out; a.y = (__nv_bfloat16*)y;
   a.rows = rows; a.D = D; a.eps = eps; a.one_plus_w = one_plus_w;
-  if (D >= 1024 && (rows <= 2048 || D >= 2048) && D <= 256 * kRowVecs * 8)     // sum and norm, rows x D: 2049 x 4096 14.6 us by CTAs and 21.8 by warps, 8192 x 5120 80.0 and 82.8, 8192 x 1024 19.7 and 14.0
+  // A CTA per row has one load of each thread in flight and pays its start and its reduction each time: ahead while the rows are few for a warp per row, or so wide
+  // that a warp walks long.  Sum and norm, rows x D, us by CTAs / by warps: 2049 x 4096 11 / 18, 3000 x 2048 10 / 12, 3500 x 2048 10.7 / 10.1, 4096 x 4096 32 / 34,
+  // 6000 x 4096 46 / 42, 8192 x 2048 34 / 28, 8192 x 6144 87 / 99, 30000 x 2048 119 / 83, 32768 x 8192 432 / 433; the norm alone 8192 x 3072 31 / 21, 32768 x 2048 83 / 48.
+  if (D >= 1024 && (rows <= 2048 || D >= 6144 || (D >= 4096 && rows <= 4096) || (D >= 2048 && rows <= 3000)) && D <= 256 * kRowVecs * 8)
     return (int)launch_dependent(rmsnorm_weighted_row_kernel, dim3(rows), dim3(256), 0, (cudaStream_t)stream, a);
   return (int)launch_dependent(rmsnorm_weighted_kernel, dim3(grid_for_rows(rows, 8)), dim3(256), 0, (cudaStream_t)stream, a);
 }

@@ -895,3 +895,17 @@ def test_newton_schulz_moved_equals_the_copying_form(shape, iters):
     want = polar.newton_schulz_(x.clone(), iters)
     got = polar.newton_schulz_moved(x.clone(), iters)
     assert got.shape == x.shape and torch.equal(got, want) and (iters == 0 or not torch.equal(got, x))
+
+
+@pytest.mark.parametrize("rows,D", [(2048, 1024), (2049, 1024), (3000, 2048), (3001, 2048), (4096, 4096), (4097, 4096), (4097, 6144)])
+def test_weighted_norm_on_both_sides_of_its_rule(rows, D):
+    """A CTA or a warp a row: the sum is rounded to bf16 once, the result once (2^-8), its root and sum in fp32."""
+    from tyr_b200.ops.norm import rms_norm_weighted
+    g = torch.Generator(device="cuda").manual_seed(rows + D)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, res, w = r(rows, D), r(rows, D), r(D) * 0.1
+    y, s = rms_norm_weighted(x, w, 1e-6, one_plus_w=True, residual=res, return_residual=True)
+    assert torch.equal(s, (x.float() + res.float()).bfloat16())
+    ref = s.double() * torch.rsqrt(s.double().pow(2).mean(-1, keepdim=True) + 1e-6) * (1 + w.double())
+    assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-6).all()
+    assert torch.equal(rms_norm_weighted(s, w, 1e-6, one_plus_w=True), y)
