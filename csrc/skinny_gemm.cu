@@ -205,8 +205,10 @@ __global__ void __launch_bounds__(kSkWarps * 32) skinny_gemm_kernel(SkinnyArgs a
     }
 #pragma unroll
     for (int i = 0; i < TILES; ++i) {
+      // The plain load keeps the gated form of 9 to 16 tokens at 69.4 us for 2 x 17408 x 5120, with __ldg beside the other form it takes 74.4; of 17 to 32
+      // tokens 106 and 105.
       const uint4* xp = reinterpret_cast<const uint4*>(xr[i] + 32 * c);
-      const uint4 xv = live[i] ? (NORM ? *xp : __ldg(xp)) : make_uint4(0u, 0u, 0u, 0u);
+      const uint4 xv = live[i] ? (NORM || (GATED && TILES == 2) ? *xp : __ldg(xp)) : make_uint4(0u, 0u, 0u, 0u);
       mma_16816(acc[i], lo.x, hi.x, lo.y, hi.y, xv.x, xv.y);
       mma_16816(acc[i], lo.z, hi.z, lo.w, hi.w, xv.z, xv.w);
       if (GATED) {
@@ -370,13 +372,15 @@ static void skinny_prefer_l1() {
   skinny_set_carveout<4, true>();
 }
 
-// CTAs of a cluster that share the contraction of one 16-row tile: as many as stay resident at once beside the other tiles' (6, 4 or 3
-// on an SM for up to 8, 16 or 32 tokens), each with at least kSkSplitChannels channels.  One row, us at 1 / 2 / 3 / 4 / 8 CTAs: 1024 x 3584
-// 10.1 / 5.9 / 5.6 / 5.2 / 4.6, 4096 x 12288 36.8 / 23.4 / 20.3 / 26.4 / 25.5, 5120 x 17408 52.1 / 34.1 / 44.6 / 36.4 / 42.2 (past one wave of CTAs
-// it gets slower); 32 rows, two matrices of 1024 x 5120 27.2 / 15.9 / 13.5 / 20.9 / 28.2.
-constexpr int kSkSplitChannels = 512;
+// CTAs of a cluster that share the contraction of one 16-row tile: as many as stay resident at once beside the other tiles' (6 or 3 on an SM for up to 8 or 32
+// tokens, 4 for 9 to 16 of which clusters find nine tenths), each with at least kSkSplitChannels channels, and none of a contraction that one CTA walks in few steps.  Weights
+// from HBM, us at 1 / 2 / 3 / 4 / 8 CTAs: one row, 1024 x 3584 10.1 / 5.9 / 5.6 / 5.2 / 4.6, 3584 x 1024 3.7 / 4.5 / 4.7 / 6.9 / 11, 4096 x 12288 36.8 / 23.4 / 20.3 / 26.4 / 25.5,
+// 5120 x 17408 52.1 / 34.1 / 44.6 / 36.4 / 42.2 (past one wave of CTAs it gets slower); 16 rows, 3072 x 2048 7.1 / 6.4 / 10.6 / 10.4 / 16.5; 32 rows, two matrices of
+// 1024 x 5120 27.2 / 15.9 / 13.5 / 20.9 / 28.2.  Over 1 to 32 rows, 16 to 32000 columns and 512 to 17408 channels 0.8 % from the best on average, 25 % at most.
+constexpr int kSkSplitChannels = 512, kSkSplitFrom = 1536;
 static int skinny_splits(int row_ctas, int M, int K) {
-  int splits = 148 * (M <= 8 ? 6 : M <= 16 ? 4 : 3) / row_ctas;
+  int splits = (M <= 8 ? 148 * 6 : M <= 16 ? 532 : 148 * 3) / row_ctas;
+  if (M <= 16 && K < kSkSplitFrom) return 1;
   if (splits > K / kSkSplitChannels) splits = K / kSkSplitChannels;
   if (splits > tyr::kSkMaxSplits) splits = tyr::kSkMaxSplits;
   return splits < 1 ? 1 : splits;
