@@ -133,3 +133,11 @@ def test_turned_queries_and_keys_go_together():
     for bad in ((q, k[:2], tab, tab, w, w, pos), (q, bf(3, 2, 16), tab, tab, w, w, pos), (q, k, tab, tab[:4], w, w, pos), (q, k, tab, tab, w[:1], w, pos),
                 (q, k, tab, tab, w, w, pos[:1]), (q, k, tab, tab, w, w.float(), pos), (q, k, tab, tab, w, w, pos.to("meta"))):
         assert not RO.qk_fit(*bad)
+
+
+def test_matrices_share_a_launch_where_that_is_the_faster_way():
+    for M, K, widths, want in ((1, 5120, (12288, 1024, 1024), [1, 2]), (8, 4096, (1024, 12288, 1024), [0, 2]), (9, 5120, (12288, 1024, 1024), [0, 1, 2]),
+                               (1, 1024, (6144, 2048, 16, 16), [0, 1, 2, 3]), (4, 5120, (10240, 6144, 48, 48), [0, 1, 2, 3]), (1, 4096, (16384, 1024, 1024), [0, 1, 2]),
+                               (20, 5120, (4096,), []), (32, 4096, (2048, 2048), []), (20, 5120, (48, 48), [0, 1]), (32, 5120, (1024, 1024), [0, 1]),
+                               (20, 1024, (4096, 512, 512), [0, 1, 2]), (32, 8192, (3072, 64), [1]), (16, 64, (7,), [0]), (3, 64, (), [])):
+        assert SK.shared_launch(M, K, widths) == want, (M, K, widths)

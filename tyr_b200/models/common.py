@@ -60,8 +60,9 @@ def lin(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor] = None, act:
 
 def lin_many(x: torch.Tensor, ws: Sequence[torch.Tensor]) -> List[torch.Tensor]:
     """``[lin(x, w) for w in ws]``.  A decode-sized batch takes all products that the weight-streaming kernel serves in one launch: up to 16 rows
-    every one of them, up to 32 rows those whose matrices have too few 128-row tiles for the tensor-core kernel of that size.  There the library
-    took 16.5 us for two products of [48, 5120] and 19.3 us for two of [1024, 5120] at 32 rows; one launch takes 7.0 and 13.5 us."""
+    every one of them, up to 32 rows those whose matrices have too few 128-row tiles for the tensor-core kernel of that size, as far as one launch is
+    the faster way (see ``shared_launch``).  The library took 16.5 us for two products of [48, 5120] and 19.3 us for two of [1024, 5120] at 32 rows; one launch
+    takes 7.0 and 13.5 us."""
     rows = x.numel() // x.shape[-1]
     if rows >= TCGEN05_MIN_ROWS and x.is_cuda and x.dtype == torch.bfloat16 and not torch.is_grad_enabled():
         # prompts: all of them up to MANY_MAX_ROWS rows, else the narrow ones
@@ -77,6 +78,8 @@ def lin_many(x: torch.Tensor, ws: Sequence[torch.Tensor]) -> List[torch.Tensor]:
     x2 = x.reshape(rows, -1)
     few = [i for i, w in enumerate(ws) if _skinny.supported(x2, w) or
            (_skinny.supported(x2, w, _skinny.MAX_ROWS) and w.shape[0] < 128 * _decode_gemm.MIN_ROW_TILES)][:_skinny.MAX_MATRICES]
+    if few:
+        few = [few[i] for i in _skinny.shared_launch(rows, x2.shape[1], [ws[i].shape[0] for i in few])]
     out = [lin(x, w) if i not in few else None for i, w in enumerate(ws)]
     if few:
         for i, y in zip(few, _skinny.skinny_many(x2, [ws[i] for i in few])):

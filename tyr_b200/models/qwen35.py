@@ -412,7 +412,7 @@ def forward(m: Qwen35ForCausalLM, input_ids=None, attn_mask=None, inputs_embeds=
 
 def _norm_products(f, x, norm, eps, ws):
     """([h w^T for w in ws], the stream ``x + f``) with h the norm of the stream; rows [B, h], ``x`` None before the first layer."""
-    if skinny.norm_supported(f, norm, ws):
+    if skinny.norm_supported(f, norm, ws) and len(skinny.shared_launch(*f.shape, [w.shape[0] for w in ws])) == len(ws):
         return skinny.skinny_norm_many(f, x, norm, eps, ws, one_plus_w=True)
     if x is None:
         return lin_many(rms(f, norm, eps), ws), f

@@ -67,6 +67,24 @@ def skinny_linear(x2: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor
     return y
 
 
+def shared_launch(M: int, K: int, widths: Sequence[int]) -> List[int]:
+    """Which of the matrices [N_i, K] are best read by one launch over M rows; the others are left to the products of their own.
+
+    Up to 8 rows a launch holds 888 tiles of 16 columns at once, and a few tiles more are a wave of their own: 12288, 1024 and 1024 columns of 5120 take 35.2 us in
+    one launch, and 23.1 and 6.9 with the widest by itself.  Above 16 rows the tensor-core kernel does not take narrow matrices and the library stands against the
+    shared launch, at about 2.5 us and 1.5 a 1024 channels a matrix whatever its width, where the launch takes 4.5 us and one more a million numbers.
+    20 rows, library / shared: two of 1024 x 4096 17.2 / 10.7, two of 2048 x 4096 15.7 / 19.1, 4096 x 5120 10.6 / 24.2, two of 48 x 5120 16.1 / 6.1."""
+    idx = sorted(range(len(widths)), key=widths.__getitem__)
+    if M > LINEAR_MAX_ROWS:
+        while idx and 4.5 + 1e-6 * K * sum(widths[i] for i in idx) >= len(idx) * (2.5 + 1.5e-3 * K):
+            idx.pop()
+    elif M <= 8 and len(idx) > 1:
+        tiles = [-(-widths[i] // 16) for i in idx]
+        if tiles[-1] <= 888 < sum(tiles) <= 976:
+            idx.pop()
+    return sorted(idx)
+
+
 def skinny_many(x2: torch.Tensor, ws: Sequence[torch.Tensor], splits: int = 0) -> List[torch.Tensor]:
     """``[x2 w^T for w in ws]`` in one launch: x2 [M <= 32, K] bf16, up to four matrices [N_i, K] bf16 (rows may be strided).  ``splits``: CTAs
     of a cluster that share a contraction (0: by size)."""
