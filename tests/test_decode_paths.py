@@ -60,7 +60,8 @@ def test_slices_fill_the_chip_without_a_thin_last_wave():
     """The fastest (or next to it) of the measured numbers of slices, for few and many pairs, short and long stores."""
     for (B, G, keys, heads, D), good in {(1, 2, 564, 4, 256): {9}, (32, 4, 576, 4, 256): {2}, (40, 4, 2048, 4, 256): {3}, (72, 4, 8192, 4, 256): {1},
                                          (32, 4, 2048, 4, 128): {3}, (38, 4, 8192, 4, 128): {2, 5, 6}, (48, 4, 8192, 4, 128): {2}, (64, 4, 2048, 4, 128): {3},
-                                         (40, 4, 2048, 8, 64): {4}, (38, 4, 8192, 8, 64): {4}, (75, 4, 8192, 8, 64): {2}}.items():
+                                         (40, 4, 2048, 8, 64): {4}, (38, 4, 8192, 8, 64): {4}, (75, 4, 8192, 8, 64): {2},
+                                         (16, 4, 200, 8, 256): {1}, (8, 4, 129, 8, 256): {1}, (8, 4, 1000, 16, 64): {4, 5, 6, 8, 10}}.items():
         assert DA.pick_splits(B, G, keys, heads, D, D) in good, (B, G, keys, D)
     for keys in (1, 64, 65, 300, 100000):
         for B in (1, 7, 150, 100000):

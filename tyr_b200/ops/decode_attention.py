@@ -41,15 +41,18 @@ def pick_splits(B: int, Hkv: int, keys: int, heads: int = 1, DK: int = 128, DV: 
     """Slices of the keys for each of B * Hkv (row, K/V head) pairs of ``heads`` query heads: the number with the least modelled time, in keys that a CTA
     reads.  A CTA waits for its own loads, whatever shares its SM, so a launch takes as many waves of CTAs as it fills: 2, 3, 4 or 5 of them fit an SM by
     registers, and of the smallest ones a wave holds 690 (704 took 1.19 times as long as 640).  A wave costs its keys (whole steps of 64) and 256 more, the merge
-    16384 / DV and 512 / DV a slice, four times that with more than 8 heads.
+    16384 / DV and 512 / DV a slice, with more than 8 heads four times that (twice at DV 64).  Up to 256 keys of 4 heads or more one CTA is through before a merge
+    begins to pay.
 
     Us at 1 / 2 / 3 / 4 / 6 slices, heads of 256: 128 pairs of 576 keys 35.6 / 28.1 / 37.2 / 36.0 / 40.7, 160 of 2048 114 / 122 / 92 / 102 / 96, 288 of 8192
     451 / 463 / 472 / 475 / 495; of 128: 128 of 2048 79 / 48 / 37 / 52 / 44, 192 of 8192 307 / 171 / 221 / 176 / 182; of 64: 160 of 8192 205 / 120 / 88 / 72 / 93.
-    Over 1 to 640 pairs of 300 to 32768 keys, plain, kept and biased, the choice takes 1.01 times the best on average and 1.25 at most; filling the SMs twice
-    takes 1.04 to 1.34 and 3.3, four times with 256 keys a slice 1.10 to 1.19 and 2.1."""
+    Over 1 to 1024 pairs of 65 to 32768 keys of 1 to 16 heads, plain, kept and biased, the choice takes 1.01 times the best on average and 1.31 at most; filling
+    the SMs twice takes 1.04 to 1.34 and 3.3, four times with 256 keys a slice 1.06 to 1.42 and 2.3."""
+    if keys <= 256 and heads >= 4:
+        return 1
     pairs = max(1, B * Hkv)
     at_once = 296 if max(DK, DV) > 128 else 444 if DV > 64 else 592 if DK > 64 else 690
-    merge = (4 if heads > 8 else 1) * 512 / DV
+    merge = (1 if heads <= 8 else 4 if DV > 64 else 2) * 512 / DV
 
     def cost(s):
         chunk = -(-keys // (64 * s)) * 64
